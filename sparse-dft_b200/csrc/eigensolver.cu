@@ -1,10 +1,12 @@
 // Device eigensolver for the Davidson Rayleigh-Ritz step (lowest `wanted`
 // eigenpairs of an m x m Hermitian matrix, m up to ~1290).
 //
-// 1. tridiagonalize_kernel: one cooperative launch, one CTA per SM, columns
-//    distributed cyclically and held in shared memory. Step j of the
-//    Householder reduction (LAPACK zhetd2, lower, H_j = I - tau v v^H with
-//    v[j+1] = 1) needs one grid-wide barrier: after it every CTA forms
+// 1. Householder reduction (LAPACK zhetd2, lower, H_j = I - tau v v^H with
+//    v[j+1] = 1): tridiagonalize_cluster_kernel for orders up to 256 and for
+//    the last 256 rows of larger matrices, in one 16-CTA cluster;
+//    tridiagonalize_kernel for the steps before: one cooperative launch, one
+//    CTA per SM, columns distributed cyclically and held in shared memory.
+//    Its step j needs one grid-wide barrier: after it every CTA forms
 //    w = p - tau/2 (p^H v) v from the published p and shares of p^H v,
 //    recomputes the next reflector redundantly from the published next column
 //    (plus this rank-2 update), then in one pass over its own columns applies
@@ -111,8 +113,9 @@ __device__ bool grid_barrier(unsigned int* arrive, unsigned int* error, unsigned
 }
 
 struct TridiagArgs {
-  const Cx<double>* a;
+  Cx<double>* a;
   int m, grid, cpc;
+  int stop;  // reflectors formed here: m - 1 for the whole reduction, fewer when the cluster kernel takes the rest
   double* d;
   double* e;
   Cx<double>* tau;
@@ -294,7 +297,7 @@ __global__ void __launch_bounds__(kTridiagThreads, 1) tridiagonalize_kernel(Trid
   if (!grid_barrier(t.arrive, t.error, static_cast<unsigned int>(G), &ok)) return;
 
   for (int j = 0; j < m - 1; ++j) {
-    const bool last = j == m - 2;
+    const bool last = j == t.stop - 1;
     // All of this step's global reads first (one round of L2 latency): p on
     // own rows, column j+1, p at own columns and at row j+1, the CTA shares
     // of p^H v (every warp sums them in the same order).
@@ -384,7 +387,357 @@ __global__ void __launch_bounds__(kTridiagThreads, 1) tridiagonalize_kernel(Trid
     for (int k = 0; k < R; ++k) v[k] = vn[k];
   }
   __syncthreads();
-  if ((m - 1) % G == cta && tid == 0) t.d[m - 1] = cols[static_cast<long long>((m - 1) / G) * m + m - 1].re;
+  if (t.stop == m - 1) {
+    if ((m - 1) % G == cta && tid == 0) t.d[m - 1] = cols[static_cast<long long>((m - 1) / G) * m + m - 1].re;
+    return;
+  }
+  // The trailing matrix, every update applied, for the cluster kernel.
+  for (int s = 0; s < cpc; ++s) {
+    const int c = cta + s * G;
+    if (c >= t.stop && c < m)
+      for (int r = t.stop + tid; r < m; r += kTridiagThreads)
+        t.a[r + static_cast<long long>(c) * m] = cols[static_cast<long long>(s) * m + r];
+  }
+}
+
+// Householder reduction of a matrix of order m <= kClusterOrder by one
+// cluster of 16 CTAs: column c = rank + 16 q on CTA `rank`, held in registers
+// for the whole reduction, every exchange through distributed shared memory. The grid kernel above pays a global release, a
+// polled counter and L2 round trips per step: about 5 us whatever the order,
+// against 1.25 us at order 64, 1.3 at 128 and 1.8 at 256 here (0.5 -> 0.28 ms
+// for order 160, 4.07 -> 2.9 ms for the 640 whose last 256 rows end here). The
+// step is bound by its serial chain of instructions, not by a pipe or memory.
+// It reduces whole matrices up to kClusterOrder and the trailing kClusterOrder
+// rows of larger ones; a solve below kClusterOrder needs no cooperative
+// launch, so solves on other streams do not queue behind it.
+//
+// Reflector j has head row h = j + 1 and v = e_h + scale x, x the part of
+// column j below h. Step j starts with x, and A x and row h of the trailing
+// matrix (updates < j applied; by symmetry column h) complete in every CTA:
+//   vector phase  A v = A e_h + scale A x, w = tau A v + alpha v, column h with
+//                 update j applied, and from it the next x;
+//   pass          update j and the products A x of the next reflector. A warp's
+//                 lanes are 8 columns x 4 rows, a thread's tile RT rows (r = 32 i
+//                 + row group) x CT columns (q = 8 k + lane): each v, w, x read
+//                 from shared memory serves CT columns. (With the matrix in
+//                 shared memory and one column per lane the pass was bound by
+//                 shared-memory wavefronts, 20 per row.) Entries of finished
+//                 rows and columns meet zeros of v, w and x, and whole tile
+//                 rows and columns are skipped once finished;
+//   scalars       one more warp forms the next norm, tau and scale meanwhile:
+//                 nothing before the next vector phase needs them, so their
+//                 square root, reciprocals and sums stay off the step's chain;
+//   publish       A x and the head row to every CTA of the cluster (asynchronous
+//                 stores that complete an mbarrier there: no cluster barrier and
+//                 no flush of the reflector's global stores in a step), and from
+//                 one more warp the CTA's share of x^H A x (v^H A v = A_hh +
+//                 2 Re(scale (A x)_h) + |scale|^2 x^H A x gives the real
+//                 alpha = -|tau|^2 v^H A v / 2).
+constexpr int kClusterCtas = 16;    // non-portable cluster size
+constexpr int kClusterOrder = 256;  // the largest tile without spills (8 x 2); 10 x 3 for 320 ran at 3.3 us a step
+constexpr int kPassWarps = 8;
+constexpr int kColumnLanes = 8;     // lanes over columns; the other 4 over rows
+constexpr int kRowGroups = kPassWarps * (32 / kColumnLanes);
+constexpr int kScalarWarp = kPassWarps, kShareWarp = kPassWarps + 1;
+constexpr int kClusterThreads = 32 * (kPassWarps + 2);
+
+struct ClusterArgs {
+  const Cx<double>* a;  // m x m, leading dimension ld
+  long long ld;
+  int m;
+  double* d;
+  double* e;
+  Cx<double>* tau;
+  Cx<double>* reflectors;  // column j holds v_j in rows j+1.., leading dimension ld
+  unsigned int* error;     // set when an exchange does not complete in time
+};
+
+// Position of vector entry c: one pad per 16 entries, so that a CTA's own
+// columns (stride 16) fall into different banks.
+__host__ __device__ constexpr int padded(int c) { return c + (c >> 4); }
+
+template <int RT, int CT>
+constexpr std::size_t cluster_smem() {
+  return sizeof(Cx<double>) * (7 * static_cast<std::size_t>(padded(kRowGroups * RT)) +
+                               (kPassWarps + 1) * kColumnLanes * CT + 4 + kClusterCtas);
+}
+
+__device__ __forceinline__ unsigned cluster_address(const void* local, int rank) {
+  unsigned remote;
+  const unsigned own = static_cast<unsigned>(__cvta_generic_to_shared(local));
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(own), "r"(rank));
+  return remote;
+}
+// Asynchronous stores to a CTA of the cluster; their bytes count towards the
+// phase of the mbarrier at `barrier` in the same CTA.
+__device__ __forceinline__ void cluster_store(unsigned address, Cx<double> v, unsigned barrier) {
+  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.f64 [%0], {%1, %2}, [%3];" ::"r"(address),
+               "d"(v.re), "d"(v.im), "r"(barrier)
+               : "memory");
+}
+__device__ __forceinline__ void cluster_store(unsigned address, double v, unsigned barrier) {
+  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.f64 [%0], %1, [%2];" ::"r"(address), "d"(v),
+               "r"(barrier)
+               : "memory");
+}
+// Waits for the phase `parity` of a local mbarrier; false after the time limit.
+__device__ __forceinline__ bool exchange_wait(unsigned barrier, unsigned parity) {
+  unsigned long long start = 0;
+  for (int spins = 0;; ++spins) {
+    unsigned done;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(done)
+        : "r"(barrier), "r"(parity)
+        : "memory");
+    if (done) return true;
+    if ((spins & 255) == 255) {
+      const unsigned long long now = global_ns();
+      if (!start) start = now;
+      else if (now - start > kWaitNs) return false;
+    }
+  }
+}
+__device__ __forceinline__ void cluster_barrier() {
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+template <int RT, int CT>
+__global__ void __cluster_dims__(kClusterCtas, 1, 1) __launch_bounds__(kClusterThreads, 1)
+    tridiagonalize_cluster_kernel(ClusterArgs t) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  constexpr int C = kClusterCtas, CL = kColumnLanes;
+  constexpr int L = kRowGroups * RT, PL = padded(L), COLS = CL * CT;
+  static_assert(RT % 2 == 0 && kRowGroups % C == 0 && L <= C * COLS && L <= 32 * kPassWarps,
+                "every column has a slot, every row a thread of the pass's warps");
+  const int m = t.m, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  unsigned rank_;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank_));
+  const int rank = static_cast<int>(rank_);
+  Cx<double>* abuf = reinterpret_cast<Cx<double>*>(smem_raw);  // A x: [2][PL], by step parity
+  Cx<double>* hbuf = abuf + 2 * PL;                            // head row: [2][PL]
+  Cx<double>* vs = hbuf + 2 * PL;
+  Cx<double>* ws = vs + PL;
+  Cx<double>* xs = ws + PL;
+  Cx<double>* red = xs + PL;                  // [kPassWarps][COLS]
+  Cx<double>* heads = red + kPassWarps * COLS;  // head row at own columns
+  Cx<double>* pick = heads + COLS;            // entry below the head
+  Cx<double>* scalars = pick + 1;             // tau, scale
+  double* shares = reinterpret_cast<double*>(scalars + 2);  // x^H A x of each CTA's columns: [2][C]
+  unsigned long long* arrived = reinterpret_cast<unsigned long long*>(shares + 2 * C);  // mbarriers, by step parity
+
+  for (int i = tid; i < 7 * PL; i += kClusterThreads) abuf[i] = Cx<double>{0.0, 0.0};
+  const int cl = lane % CL, rg = warp * (32 / CL) + lane / CL;
+  Cx<double> y[RT][CT];
+#pragma unroll
+  for (int i = 0; i < RT; ++i)
+#pragma unroll
+    for (int k = 0; k < CT; ++k) {
+      const int r = i * kRowGroups + rg, c = rank + C * (cl + CL * k);
+      y[i][k] = warp < kPassWarps && r < m && c < m ? t.a[r + static_cast<long long>(c) * t.ld] : Cx<double>{0.0, 0.0};
+    }
+  // Publish: thread (column pq, part ps) sums partial ps, and stores the sum to CTAs ps and ps + 8.
+  const int pq = warp * (32 / kPassWarps) + lane / kPassWarps, ps = lane % kPassWarps;
+  const unsigned remote0 = cluster_address(smem_raw, ps), remote1 = cluster_address(smem_raw, ps + kPassWarps);
+  const unsigned remote_lane = cluster_address(smem_raw, lane % C);
+  auto offset = [&](const void* p) {
+    return static_cast<unsigned>(static_cast<const unsigned char*>(p) - smem_raw);
+  };
+  // A step's exchange is complete when its bytes, the arrival that announces them and the
+  // scalars' arrival are in.
+  if (tid == 0) {
+    for (int i = 0; i < 2; ++i)
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 2;" ::"r"(
+                       static_cast<unsigned>(__cvta_generic_to_shared(arrived + i)))
+                   : "memory");
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  const unsigned barriers = static_cast<unsigned>(__cvta_generic_to_shared(arrived));
+  const int padded_rg = padded(rg);
+  const int pairs_end = (m + 2 * kRowGroups - 1) / (2 * kRowGroups), cols_end = (m + C * CL - 1) / (C * CL);
+  bool alive = true;
+  // No CTA of the cluster writes into one that has not started.
+  cluster_barrier();
+
+  Cx<double> x{0.0, 0.0};  // row tid of the current column below its head
+  for (int j = -1; j < m - 1; ++j) {
+    const int par = j & 1, next = par ^ 1, h = j + 1;
+    const bool last = j == m - 2;
+    // The exchange of step j - 1 (the u-th use of this parity's barrier, from 0: phase u & 1).
+    if (j >= 0 && alive) {
+      alive = exchange_wait(barriers + 8 * par, (j >> 1) & 1);
+      if (!alive && lane == 0) atomicOr(t.error, 2u);
+    }
+    if (warp < kPassWarps && (warp + 1) * 32 > j) {  // a warp with live rows (or just finished ones)
+      Cx<double> tau{0.0, 0.0}, scale{0.0, 0.0}, head_w{0.0, 0.0};
+      double alpha = 0.0;
+      const Cx<double>* ab = abuf + par * PL;
+      const Cx<double>* hb = hbuf + par * PL;
+      if (j >= 0) {
+        tau = scalars[0];
+        scale = scalars[1];
+        double tree[C];
+#pragma unroll
+        for (int i = 0; i < C; ++i) tree[i] = shares[par * C + i];
+#pragma unroll
+        for (int o = C / 2; o > 0; o >>= 1)
+#pragma unroll
+          for (int i = 0; i < o; ++i) tree[i] += tree[i + o];
+        const Cx<double> ah = ab[padded(h)], hh = hb[padded(h)];
+        const double vav = fma(scale.re * scale.re + scale.im * scale.im, tree[0],
+                               fma(2.0, scale.re * ah.re - scale.im * ah.im, hh.re));
+        alpha = (-0.5 * (tau.re * tau.re + tau.im * tau.im)) * vav;
+        head_w = cmulz(tau, cadd(cconj(hh), cmulz(scale, ah)));
+        head_w.re += alpha;  // v[h] = 1
+        head_w.im = -head_w.im;
+      }
+      const int r = tid;
+      if (r < m) {
+        Cx<double> col{0.0, 0.0}, v{0.0, 0.0}, w{0.0, 0.0};
+        if (j < 0) {
+          col = t.a[r];
+        } else if (r >= h) {
+          const Cx<double> hr = cconj(hb[padded(r)]);
+          v = r == h ? Cx<double>{1.0, 0.0} : cmulz(x, scale);
+          w = cmulz(tau, cadd(hr, cmulz(scale, ab[padded(r)])));
+          w.re += alpha * v.re;
+          w.im += alpha * v.im;
+          col = csub(hr, cadd(cmulz(v, head_w), w));
+          if (rank == (j & (C - 1))) t.reflectors[r + static_cast<long long>(j) * t.ld] = v;
+        }
+        if (r == h && rank == 0) t.d[h] = col.re;
+        if (r == h + 1) pick[0] = col;
+        x = r > h + 1 ? col : Cx<double>{0.0, 0.0};
+        vs[padded(r)] = v;
+        ws[padded(r)] = w;
+        xs[padded(r)] = x;
+      }
+    }
+    if (last) break;
+    __syncthreads();
+
+    if (warp == kScalarWarp) {
+      double re2 = 0.0, im2 = 0.0;
+#pragma unroll 4
+      for (int r = lane; r < L; r += 32) {  // zeros outside the column
+        const Cx<double> xr = xs[padded(r)];
+        re2 += xr.re * xr.re;
+        im2 += xr.im * xr.im;
+      }
+      double xnorm2 = re2 + im2;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) xnorm2 += __shfl_xor_sync(0xffffffffu, xnorm2, o);
+      // make_reflector with its two reciprocals on two lanes at once.
+      const Cx<double> a = pick[0];
+      const bool trivial = xnorm2 == 0.0 && a.im == 0.0;
+      const double beta = -copysign(sqrt(a.re * a.re + a.im * a.im + xnorm2), a.re);
+      const double dr = a.re - beta;
+      const double inverse = 1.0 / ((lane & 1) ? dr * dr + a.im * a.im : beta);
+      const double inv_beta = __shfl_sync(0xffffffffu, inverse, 0), inv_den = __shfl_sync(0xffffffffu, inverse, 1);
+      if (lane == 0) {
+        const Cx<double> zero{0.0, 0.0};
+        const Cx<double> th = trivial ? zero : Cx<double>{-dr * inv_beta, -a.im * inv_beta};
+        scalars[0] = th;
+        scalars[1] = trivial ? zero : Cx<double>{dr * inv_den, -a.im * inv_den};
+        asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(barriers + 8 * next) : "memory");
+        if (rank == 0) {
+          t.e[h] = trivial ? a.re : beta;
+          t.tau[h] = th;
+        }
+      }
+    } else if (warp == kShareWarp) {
+      // 32 bytes of each live column and every CTA's share.
+      if (lane == 0)
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(barriers + 8 * next),
+                     "r"(32 * (m - 1 - h) + 8 * C)
+                     : "memory");
+      asm volatile("bar.sync 1, %0;" ::"n"(32 * (kPassWarps + 1)) : "memory");
+      double share = 0.0;
+      if (lane < COLS) {
+        Cx<double> sum[kPassWarps];
+#pragma unroll
+        for (int w = 0; w < kPassWarps; ++w) sum[w] = red[w * COLS + lane];
+        const int c = rank + C * lane;
+        const Cx<double> xc = c < L ? xs[padded(c)] : Cx<double>{0.0, 0.0};
+#pragma unroll
+        for (int o = kPassWarps / 2; o > 0; o >>= 1)
+#pragma unroll
+          for (int w = 0; w < o; ++w) sum[w] = cadd(sum[w], sum[w + o]);
+        share = sum[0].re * xc.re + sum[0].im * xc.im;
+      }
+#pragma unroll
+      for (int o = COLS > 16 ? 16 : COLS > 8 ? 8 : 4; o > 0; o >>= 1) share += __shfl_xor_sync(0xffffffffu, share, o);
+      if (COLS <= 16) share = __shfl_sync(0xffffffffu, share, 0);
+      if (lane < C) cluster_store(remote_lane + offset(shares + next * C + rank), share, remote_lane + offset(arrived + next));
+    } else {
+      // Live tile rows, two at a time (four independent chains of multiply-adds), and columns.
+      const int first_pair = (h + 1) / (2 * kRowGroups), first_col = (h + 1) / (C * CL);
+      const int head_pair = rg == (h + 1) % kRowGroups ? first_pair : -1;
+      const bool head_second = (h + 1) / kRowGroups & 1;
+#pragma unroll
+      for (int k = 0; k < CT; ++k) {
+        Cx<double> acc[2] = {};
+        if (k >= first_col && k < cols_end) {
+          const int c = rank + C * (cl + CL * k);
+          const Cx<double> none{0.0, 0.0};  // slots past the tile's order
+          const Cx<double> wc = c < L ? cconj(ws[padded(c)]) : none, vc = c < L ? cconj(vs[padded(c)]) : none;
+#pragma unroll
+          for (int i = 0; i < RT; i += 2) {
+            if (i / 2 < first_pair || i / 2 >= pairs_end) continue;
+            Cx<double> v[2], w[2], xr[2];
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+              const int at = padded((i + u) * kRowGroups) + padded_rg;
+              v[u] = vs[at];
+              w[u] = ws[at];
+              xr[u] = xs[at];
+            }
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+              Cx<double> z = y[i + u][k];
+              z.re = fma(-v[u].re, wc.re, fma(v[u].im, wc.im, fma(-w[u].re, vc.re, fma(w[u].im, vc.im, z.re))));
+              z.im = fma(-v[u].re, wc.im, fma(-v[u].im, wc.re, fma(-w[u].re, vc.im, fma(-w[u].im, vc.re, z.im))));
+              y[i + u][k] = z;
+              acc[u] = cadd(acc[u], cdot1(z, xr[u]));
+            }
+            if (i / 2 == head_pair) heads[cl + CL * k] = head_second ? y[i + 1][k] : y[i][k];
+          }
+        }
+        Cx<double> sum = cadd(acc[0], acc[1]);
+#pragma unroll
+        for (int o = CL; o < 32; o <<= 1) {
+          sum.re += __shfl_xor_sync(0xffffffffu, sum.re, o);
+          sum.im += __shfl_xor_sync(0xffffffffu, sum.im, o);
+        }
+        if (lane < CL) red[warp * COLS + lane + CL * k] = sum;
+      }
+      // The pass's and the share's warps: the scalars are not needed yet.
+      asm volatile("bar.sync 1, %0;" ::"n"(32 * (kPassWarps + 1)) : "memory");
+      if (warp * (32 / kPassWarps) < COLS) {
+        Cx<double> sum = red[ps * COLS + pq];
+#pragma unroll
+        for (int o = kPassWarps / 2; o > 0; o >>= 1) {
+          sum.re += __shfl_xor_sync(0xffffffffu, sum.re, o);
+          sum.im += __shfl_xor_sync(0xffffffffu, sum.im, o);
+        }
+        const int c = rank + C * pq;
+        if (c > h && c < m) {
+          const Cx<double> head = heads[pq];
+          const unsigned to_a = offset(abuf + next * PL + padded(c)), to_h = offset(hbuf + next * PL + padded(c));
+          const unsigned bar = offset(arrived + next);
+          cluster_store(remote0 + to_a, sum, remote0 + bar);
+          cluster_store(remote1 + to_a, sum, remote1 + bar);
+          cluster_store(remote0 + to_h, head, remote0 + bar);
+          cluster_store(remote1 + to_h, head, remote1 + bar);
+        }
+      }
+    }
+  }
+  // No CTA leaves while another may still read or write its shared memory.
+  cluster_barrier();
 }
 
 // Number of eigenvalues of the tridiagonal (d, e) below x: sign changes of
@@ -652,35 +1005,47 @@ __global__ void __launch_bounds__(kThreads) cluster_orthonormalize_kernel(const 
 // Compact WY factor of each block of kReflectorBlock reflectors:
 // H_j0 ... H_j0+nb-1 = I - V T V^H (LAPACK zlarft, forward, columnwise),
 // T upper triangular (column-major, leading dimension kReflectorBlock), from
-// the block's Gram matrix V^H V. One CTA per block.
+// the block's Gram matrix G = V^H V. One CTA per block. T grows by doubling:
+// two neighbouring blocks T1, T2 of order s join as
+//   [T1  -T1 (G12 T2)]
+//   [ 0        T2    ]
+// so the factor takes six rounds of two parallel triangular products instead
+// of 64 dependent columns.
 __global__ void __launch_bounds__(kThreads) reflector_blocks_kernel(const Cx<double>* __restrict__ grams,
                                                                     const Cx<double>* __restrict__ tau, int m,
                                                                     Cx<double>* __restrict__ tfac) {
-  // One CTA per block of NB reflectors: T of I - V T V^H (zlarft) from the
-  // block's Gram matrix G = V^H V (column-major NB x NB, computed by cuBLAS).
   constexpr int NB = kReflectorBlock, LD = NB + 1;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   Cx<double>* gram = reinterpret_cast<Cx<double>*>(smem_raw);  // NB x LD, gram[a * LD + b] = G(a, b)
   Cx<double>* tmat = gram + NB * LD;                            // NB x LD
+  Cx<double>* prod = tmat + NB * LD;                            // G12 T2 of every pair of a round
   const int j0 = blockIdx.x * NB;
   const int nb = min(NB, m - 1 - j0);
   const int tid = threadIdx.x;
   const Cx<double>* g = grams + static_cast<long long>(blockIdx.x) * NB * NB;
   for (int idx = tid; idx < NB * NB; idx += kThreads) {
     const int col = idx / NB, row = idx % NB;
-    gram[row * LD + col] = g[idx];
-    tmat[(idx / NB) * LD + idx % NB] = Cx<double>{0.0, 0.0};
+    gram[row * LD + col] = row < nb && col < nb ? g[idx] : Cx<double>{0.0, 0.0};
+    tmat[row * LD + col] = row == col && row < nb ? tau[j0 + row] : Cx<double>{0.0, 0.0};
   }
   __syncthreads();
-  // T(i,i) = tau_i; T(0:i, i) = -tau_i T(0:i, 0:i) G(0:i, i).
-  for (int i = 0; i < nb; ++i) {
-    const Cx<double> ti = tau[j0 + i];
-    if (tid < i) {
+  for (int s = 1; s < nb; s *= 2) {
+    const int items = NB / 2 * s;
+    for (int idx = tid; idx < items; idx += kThreads) {
+      const int pair = idx / (s * s), a = idx / s % s, b = idx % s, first = pair * 2 * s, second = first + s;
       Cx<double> sum{0.0, 0.0};
-      for (int c = tid; c < i; ++c) sum = cadd(sum, cmulz(tmat[tid * LD + c], gram[c * LD + i]));
-      tmat[tid * LD + i] = cmulz(Cx<double>{-ti.re, -ti.im}, sum);
+      for (int c = 0; c <= b; ++c)
+        sum = cadd(sum, cmulz(gram[(first + a) * LD + second + c], tmat[(second + c) * LD + second + b]));
+      prod[idx] = sum;
     }
-    if (tid == 0) tmat[i * LD + i] = ti;
+    __syncthreads();
+    for (int idx = tid; idx < items; idx += kThreads) {
+      const int pair = idx / (s * s), a = idx / s % s, b = idx % s, first = pair * 2 * s, second = first + s;
+      Cx<double> sum{0.0, 0.0};
+      for (int c = a; c < s; ++c)
+        sum = cadd(sum, cmulz(tmat[(first + a) * LD + first + c], prod[pair * s * s + c * s + b]));
+      tmat[(first + a) * LD + second + b] = Cx<double>{-sum.re, -sum.im};
+    }
     __syncthreads();
   }
   for (int idx = tid; idx < NB * NB; idx += kThreads) {
@@ -762,7 +1127,8 @@ constexpr std::size_t kSmemLimit = 227 * 1024;
 
 std::size_t invit_smem(int m) { return static_cast<std::size_t>(kInvitThreads) * (5 * sizeof(double) + 1) * m; }
 
-constexpr std::size_t kBlockSmem = sizeof(Cx<double>) * 2 * kReflectorBlock * (kReflectorBlock + 1);
+constexpr std::size_t kBlockSmem =
+    sizeof(Cx<double>) * (2 * kReflectorBlock * (kReflectorBlock + 1) + kReflectorBlock * kReflectorBlock / 4);
 
 }  // namespace
 
@@ -807,6 +1173,21 @@ void cooperative_launch(void* kernel, int grid, int threads, TridiagArgs& args, 
   }
   cudaEventDestroy(ready);  // released once the recorded work completes
   cudaEventDestroy(done);
+}
+template <int RT, int CT>
+void launch_cluster(const ClusterArgs& t, cudaStream_t stream) {
+  const auto kernel = tridiagonalize_cluster_kernel<RT, CT>;
+  constexpr std::size_t smem = cluster_smem<RT, CT>();
+  allow_dynamic_smem(kernel, smem);
+  SDFT_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  kernel<<<kClusterCtas, kClusterThreads, smem, stream>>>(t);
+  SDFT_LAUNCH("tridiagonalize_cluster_kernel");
+}
+
+// The smallest register tile that holds the order.
+void cluster_tridiagonalize(const ClusterArgs& t, cudaStream_t stream) {
+  if (t.m <= 4 * kRowGroups) launch_cluster<4, 1>(t, stream);
+  else launch_cluster<8, 2>(t, stream);
 }
 }  // namespace
 
@@ -862,8 +1243,15 @@ void hermitian_lowest(cublasHandle_t blas, Cx<double>* a, int m, int wanted, dou
     if (trace) SDFT_CUDA(cudaEventRecord(marks[i], stream));
   };
   mark(0);
-  TridiagArgs t{a, m, grid, cpc, d, e, tau, reflectors, colbuf, pbuf, dotbuf, arrive, error_word};
-  cooperative_launch(reinterpret_cast<void*>(tridiagonalize_kernel), grid, kTridiagThreads, t, smem, stream);
+  const int tail = std::min(m, kClusterOrder), stop = m - tail;  // the cluster kernel's order, the grid kernel's reflectors
+  if (stop > 0) {
+    TridiagArgs t{a, m, grid, cpc, stop, d, e, tau, reflectors, colbuf, pbuf, dotbuf, arrive, error_word};
+    cooperative_launch(reinterpret_cast<void*>(tridiagonalize_kernel), grid, kTridiagThreads, t, smem, stream);
+  }
+  const std::size_t corner = static_cast<std::size_t>(stop) * (mm + 1);
+  cluster_tridiagonalize(ClusterArgs{a + corner, m, tail, d + stop, e + stop, tau + stop, reflectors + corner,
+                                     error_word},
+                         stream);
   mark(1);
 
   const int warps_per_block = 4;
@@ -954,7 +1342,7 @@ void hermitian_lowest(cublasHandle_t blas, Cx<double>* a, int m, int wanted, dou
                  m, wanted, ms[0], ms[1], ms[2], ms[3], ms[4]);
     for (auto& ev : marks) cudaEventDestroy(ev);
   }
-  if (error) throw CudaError("tridiagonalization barrier wait limit exceeded");
+  if (error) throw CudaError("tridiagonalization wait limit exceeded");
 }
 
 double identity_deviation(Cx<double>* b, int m, EigenWorkspace& ws, cudaStream_t stream) {

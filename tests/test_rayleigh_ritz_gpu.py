@@ -89,3 +89,30 @@ def test_davidson_shaped_pencil(context):
     d = rng.standard_normal((n - k0, n - k0)) + 1j * rng.standard_normal((n - k0, n - k0))
     h[k0:, k0:] = 0.5 * (d + d.conj().T) + 5.0 * np.eye(n - k0)
     check(context, h, np.eye(n), 320)
+
+
+def spaced(n, rng):
+    """n ascending eigenvalues on [-2, 30] at least half a mean spacing (16 / n) apart: inverse iteration finds
+    the vectors one by one, orthogonal to eps ||T|| / gap (2.2e-16 x 30 x 400 / 16 = 2e-13 at n = 400), so a
+    random spectrum's smallest gap would set the orthogonality measured here, not the reduction."""
+    return -2.0 + 32.0 * (np.arange(n) + rng.uniform(0.25, 0.75, n)) / n
+
+
+@pytest.mark.parametrize("n", [2, 3, 16, 17, 64, 65, 127, 128, 129, 255, 256, 257, 258, 400])
+def test_tridiagonalisation_orders(context, n):
+    """Orders around the cluster kernel's tiles (128, 256: rows and columns of the tile that are
+    partly or just filled) and its hand-over from the grid kernel (257 and up)."""
+    rng = np.random.Generator(np.random.PCG64(100 + n))
+    h, s = pencil(n, rng, spectrum=spaced(n, rng))
+    check(context, h, s, 0)
+
+
+@pytest.mark.parametrize("n", [5, 130, 300])
+def test_tridiagonalisation_of_decoupled_blocks(context, n):
+    """Columns that are already reduced (trivial reflectors) and exact zeros among coupled blocks."""
+    rng = np.random.Generator(np.random.PCG64(200 + n))
+    half = n // 2
+    lam = rng.permutation(spaced(n, rng))
+    h = np.diag(lam).astype(complex)
+    h[half:, half:], _ = pencil(n - half, rng, spectrum=np.sort(lam[half:]))
+    check(context, h, np.eye(n), 0)
