@@ -620,15 +620,14 @@ sdft_b200_status sdft_b200_density_functionals(sdft_b200_context* context, const
     require(!core_count || (core_hkl && core), "null core arrays");
     const auto support = sdft_b200::functional_support(lattice, count, hkl, density, core_count, core_hkl, core,
                                                        quadrature_padding);
-    const std::size_t n = support.keys.size();
+    const std::size_t n = support.count;
     *support_count = n;
     if (!capacity) return;
     require(capacity >= n, "density functional output capacity below the support size");
     require(context && support_hkl && potential && xc_potential && result, "null density functional outputs");
-    for (std::size_t i = 0; i < n; ++i)
-      for (int a = 0; a < 3; ++a) support_hkl[3 * i + a] = support.keys[i][a];
     sdft_b200::FunctionalResult r;
-    sdft_b200::density_functionals(*context->impl, support, reinterpret_cast<sdft_b200::Cx<double>*>(potential),
+    sdft_b200::density_functionals(*context->impl, support, support_hkl,
+                                    reinterpret_cast<sdft_b200::Cx<double>*>(potential),
                                    reinterpret_cast<sdft_b200::Cx<double>*>(xc_potential), r);
     result->hartree_energy = r.hartree_energy;
     result->xc_energy = r.xc_energy;
@@ -660,20 +659,18 @@ sdft_b200_status sdft_b200_collinear_functionals(
     const double* const values[2] = {up, down};
     const auto support =
         sdft_b200::collinear_support(lattice, counts, keys, values, core_count, core_hkl, core, padding);
-    const std::size_t n = support.keys.size();
+    const std::size_t n = support.count;
     *support_count = n;
     if (!capacity) return;
     require(capacity >= n, "density functional output capacity below the support size");
     require(context && support_hkl && potential_up && potential_down && xc_potential_up && xc_potential_down &&
                 result,
             "null density functional outputs");
-    for (std::size_t i = 0; i < n; ++i)
-      for (int a = 0; a < 3; ++a) support_hkl[3 * i + a] = support.keys[i][a];
     using C = sdft_b200::Cx<double>;
     C* const potential[2] = {reinterpret_cast<C*>(potential_up), reinterpret_cast<C*>(potential_down)};
     C* const xc[2] = {reinterpret_cast<C*>(xc_potential_up), reinterpret_cast<C*>(xc_potential_down)};
     sdft_b200::FunctionalResult r[2];
-    sdft_b200::collinear_functionals(*context->impl, support, potential, xc, r);
+    sdft_b200::collinear_functionals(*context->impl, support, support_hkl, potential, xc, r);
     for (int c = 0; c < 2; ++c) {
       result[c].hartree_energy = r[c].hartree_energy;
       result[c].xc_energy = r[c].xc_energy;

@@ -5,9 +5,12 @@
 // ordered reductions, ordered Fourier accumulation).
 //
 // Pipeline (one context stream, every array device-resident):
-//   1. host: keys sorted into the reference's map order (lexicographic h, k,
-//      l), the union support of density and frozen core, wrapped grid
-//      indices of +G and -G, G vectors with the reference's arithmetic;
+//   1. host: one pass over the keys marks them in a bitmap of the box that
+//      holds them (repeated keys, the union's size; raster order of the box is
+//      the reference's map order, lexicographic h, k, l);
+//   1b. device: a key's union position is its rank in the bitmap (population
+//      counts with a prefix per word); values, flags, wrapped grid indices of
+//      +G and -G, and G with the reference's arithmetic go there;
 //   2. scatter: two complex grids per density field set, n + i g_z and
 //      g_x + i g_y (i q_a rho packed as the reference's real_components);
 //      with a core, valence and core fields go to separate grids and are
@@ -28,9 +31,9 @@
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
-#include <numeric>
+#include <limits>
+#include <map>
 #include <string>
-#include <unordered_map>
 
 #include "local_hamiltonian.cuh"
 #include "pbe.cuh"
@@ -328,26 +331,82 @@ __global__ void __launch_bounds__(kTileThreads) xc_merge_kernel(const double* re
 
 using Key = std::array<int, 3>;
 
-struct SortedField {
-  std::vector<Key> keys;
-  std::vector<Cx<double>> values;
-};
+// A Fourier field in the caller's arrays.
+KeyField key_field(std::size_t count, const int* hkl, const double* values) { return {count, hkl, values}; }
 
-// Keys in the reference's std::map order; duplicates are rejected.
-SortedField sorted_field(std::size_t count, const int* hkl, const double* values, const char* what) {
-  std::vector<std::size_t> order(count);
-  std::iota(order.begin(), order.end(), std::size_t(0));
-  auto key = [&](std::size_t i) { return Key{hkl[3 * i], hkl[3 * i + 1], hkl[3 * i + 2]}; };
-  std::sort(order.begin(), order.end(), [&](std::size_t a, std::size_t b) { return key(a) < key(b); });
-  SortedField out;
-  out.keys.reserve(count);
-  out.values.reserve(count);
-  for (std::size_t i : order) {
-    if (!out.keys.empty() && out.keys.back() == key(i)) throw InvalidArgument(std::string("duplicate ") + what + " Fourier key");
-    out.keys.push_back(key(i));
-    out.values.push_back(Cx<double>{values[2 * i], values[2 * i + 1]});
+// Widest box whose bitmap is kept: a key beyond it puts the XC grid above 512
+// points on that axis for every padding, and the call is refused.
+constexpr long long kMaxExtent = 255;
+
+long long cell_of(const Key& k, const int m[3]) {
+  return (static_cast<long long>(k[0] + m[0]) * (2 * m[1] + 1) + (k[1] + m[1])) * (2 * m[2] + 1) + (k[2] + m[2]);
+}
+
+// Extents of all fields, then the union's bitmap; repeated keys within a field
+// are refused, in field order, through `after(field)` once a field is marked
+// (the reference's order of checks).
+template <typename After>
+void mark_keys(FunctionalSupport& s, int fields, const char* const names[], After after) {
+  long long m[3] = {0, 0, 0};
+  for (int f = 0; f < fields; ++f)
+    for (std::size_t i = 0; i < s.field[f].count; ++i)
+      for (int a = 0; a < 3; ++a) m[a] = std::max(m[a], std::llabs(s.field[f].hkl[3 * i + a]));
+  const bool boxed = std::max({m[0], m[1], m[2]}) <= kMaxExtent;
+  for (int a = 0; a < 3; ++a) s.extent[a] = static_cast<int>(std::min<long long>(m[a], 1 << 20));
+  const std::size_t words =
+      boxed ? ceil_div(static_cast<std::size_t>(2 * m[0] + 1) * (2 * m[1] + 1) * (2 * m[2] + 1), 64) : 0;
+  s.bits.assign(words, 0);
+  std::vector<std::uint64_t> own;
+  for (int f = 0; f < fields; ++f) {
+    const KeyField& field = s.field[f];
+    bool repeated = false;
+    if (boxed) {
+      own.assign(words, 0);
+      for (std::size_t i = 0; i < field.count; ++i) {
+        const long long cell = cell_of(Key{field.hkl[3 * i], field.hkl[3 * i + 1], field.hkl[3 * i + 2]}, s.extent);
+        const std::uint64_t bit = std::uint64_t(1) << (cell & 63);
+        repeated |= (own[cell >> 6] & bit) != 0;
+        own[cell >> 6] |= bit;
+      }
+      for (std::size_t w = 0; w < words; ++w) s.bits[w] |= own[w];
+    } else {  // refused by the grid limit; only the order of the checks matters
+      std::vector<Key> keys(field.count);
+      for (std::size_t i = 0; i < field.count; ++i)
+        keys[i] = Key{field.hkl[3 * i], field.hkl[3 * i + 1], field.hkl[3 * i + 2]};
+      std::sort(keys.begin(), keys.end());
+      repeated = std::adjacent_find(keys.begin(), keys.end()) != keys.end();
+    }
+    if (repeated) throw InvalidArgument(std::string("duplicate ") + names[f] + " Fourier key");
+    after(f);
   }
-  return out;
+}
+
+// Largest |re| or |im| of a field's values; infinity when one is not finite.
+double largest(const KeyField& f) {
+  double most = 0.0;
+  for (std::size_t i = 0; i < 2 * f.count; ++i) {
+    const double a = std::fabs(f.values[i]);
+    most = a <= most ? most : a;
+    if (std::isnan(a)) return std::numeric_limits<double>::infinity();
+  }
+  return most;
+}
+
+// Whether every value of a and of b, and their sum where they share a key, is
+// finite. Sums are looked at one by one only where the largest could overflow.
+bool finite_sum(const KeyField& a, const KeyField& b) {
+  const double most_a = largest(a), most_b = largest(b);
+  if (!std::isfinite(most_a) || !std::isfinite(most_b)) return false;
+  if (std::isfinite(most_a + most_b)) return true;
+  std::map<Key, std::size_t> where;
+  for (std::size_t i = 0; i < a.count; ++i) where[Key{a.hkl[3 * i], a.hkl[3 * i + 1], a.hkl[3 * i + 2]}] = i;
+  for (std::size_t i = 0; i < b.count; ++i) {
+    const auto at = where.find(Key{b.hkl[3 * i], b.hkl[3 * i + 1], b.hkl[3 * i + 2]});
+    if (at != where.end())
+      for (int c = 0; c < 2; ++c)
+        if (!std::isfinite(a.values[2 * at->second + c] + b.values[2 * i + c])) return false;
+  }
+  return true;
 }
 
 int env_padding() {
@@ -375,48 +434,142 @@ struct V3 {
 };
 
 // The XC grid padding * max(3, 2 m_a + 1) per axis (rounded to a smooth
-// length under SDFT_FAST_DENSITY_GRID=1, the reference's cached_grid), the
-// wrapped grid indices of +G and -G, the union position of -G and the G
-// vectors of the support's keys.
+// length under SDFT_FAST_DENSITY_GRID=1, the reference's cached_grid), and the
+// union's size with the rank of each bitmap word.
 void finish_support(FunctionalSupport& s, const V3 b[3], int padding) {
-  int m[3] = {0, 0, 0};
-  for (const auto& k : s.keys)
-    for (int a = 0; a < 3; ++a) m[a] = std::max(m[a], std::abs(k[a]));
   const bool fast = env_fast_grid();
   for (int a = 0; a < 3; ++a) {
-    const long long n = static_cast<long long>(padding) * std::max(3, 2 * m[a] + 1);
+    const long long n = static_cast<long long>(padding) * std::max(3, 2 * s.extent[a] + 1);
     const long long length = fast ? fast_fft_length(static_cast<int>(std::min<long long>(n, 1 << 20))) : n;
     if (length > kMaxLine) throw InvalidArgument("XC grid axis above 512 points is not supported");
     s.shape[a] = static_cast<int>(length);
   }
   s.points = static_cast<long long>(s.shape[0]) * s.shape[1] * s.shape[2];
-  auto wrap = [](int p, int dim) {
-    const int value = p % dim;
-    return value < 0 ? value + dim : value;
-  };
-  auto index = [&](const Key& k) {
-    return (static_cast<long long>(wrap(k[0], s.shape[0])) * s.shape[1] + wrap(k[1], s.shape[1])) * s.shape[2] +
-           wrap(k[2], s.shape[2]);
-  };
-  std::unordered_map<long long, int> position;
-  position.reserve(s.keys.size() * 2);
-  for (std::size_t u = 0; u < s.keys.size(); ++u) position[index(s.keys[u])] = static_cast<int>(u);
-  s.index.resize(s.keys.size());
-  s.opposite.resize(s.keys.size());
-  s.opposite_key.resize(s.keys.size());
-  s.q.resize(3 * s.keys.size());
-  for (std::size_t u = 0; u < s.keys.size(); ++u) {
-    const Key& k = s.keys[u];
-    const Key o{-k[0], -k[1], -k[2]};
-    s.index[u] = index(k);
-    s.opposite[u] = index(o);
-    const auto found = position.find(s.opposite[u]);
-    s.opposite_key[u] = found == position.end() ? -1 : found->second;
-    // reciprocal_vector (src/density_functionals.cpp:34-39): h b0 + k b1 + l b2 per component.
-    s.q[3 * u] = k[0] * b[0].x + k[1] * b[1].x + k[2] * b[2].x;
-    s.q[3 * u + 1] = k[0] * b[0].y + k[1] * b[1].y + k[2] * b[2].y;
-    s.q[3 * u + 2] = k[0] * b[0].z + k[1] * b[1].z + k[2] * b[2].z;
+  for (int a = 0; a < 3; ++a) {
+    s.reciprocal[3 * a] = b[a].x;
+    s.reciprocal[3 * a + 1] = b[a].y;
+    s.reciprocal[3 * a + 2] = b[a].z;
   }
+  s.rank.resize(s.bits.size());
+  std::uint32_t total = 0;
+  for (std::size_t w = 0; w < s.bits.size(); ++w) {
+    s.rank[w] = total;
+    total += static_cast<std::uint32_t>(__builtin_popcountll(s.bits[w]));
+  }
+  s.count = total;
+}
+
+// The support on the device, in one block of ctx.staging_in.
+struct DeviceSupport {
+  KeyData keys;
+  const Cx<double>* down;  // collinear: the down channel's values
+};
+
+struct KeyMap {
+  const std::uint64_t* bits;
+  const std::uint32_t* rank;
+  int m[3];
+};
+
+__device__ __forceinline__ long long map_cell(const KeyMap& map, int h, int k, int l) {
+  return (static_cast<long long>(h + map.m[0]) * (2 * map.m[1] + 1) + (k + map.m[1])) * (2 * map.m[2] + 1) +
+         (l + map.m[2]);
+}
+
+// Union position of a key of the support (of a key in the box, -1 where absent).
+__device__ __forceinline__ int map_position(const KeyMap& map, int h, int k, int l) {
+  const long long cell = map_cell(map, h, k, l);
+  const std::uint64_t word = map.bits[cell >> 6], bit = std::uint64_t(1) << (cell & 63);
+  return word & bit ? static_cast<int>(map.rank[cell >> 6] + __popcll(word & (bit - 1))) : -1;
+}
+
+// One field's values and key data to its union positions. Fields that share a
+// key write the same key data; their flags are set by launches in stream order.
+__global__ void place_keys_kernel(const int* __restrict__ hkl, const Cx<double>* __restrict__ values,
+                                  std::size_t count, KeyMap map, int n0, int n1, int n2, V3 b0, V3 b1, V3 b2,
+                                  unsigned char flag, Cx<double>* __restrict__ field, unsigned char* __restrict__ flags,
+                                  long long* __restrict__ index, long long* __restrict__ opposite,
+                                  int* __restrict__ opposite_key, double* __restrict__ q) {
+  for (std::size_t i = blockIdx.x * static_cast<std::size_t>(blockDim.x) + threadIdx.x; i < count;
+       i += static_cast<std::size_t>(gridDim.x) * blockDim.x) {
+    const int h = hkl[3 * i], k = hkl[3 * i + 1], l = hkl[3 * i + 2];
+    const int u = map_position(map, h, k, l);
+    field[u] = values[i];
+    flags[u] |= flag;
+    // |h| <= m < n0 / 2 on every axis: one addition wraps.
+    const auto at = [&](int x, int y, int z) {
+      return (static_cast<long long>(x < 0 ? x + n0 : x) * n1 + (y < 0 ? y + n1 : y)) * n2 + (z < 0 ? z + n2 : z);
+    };
+    index[u] = at(h, k, l);
+    opposite[u] = at(-h, -k, -l);
+    opposite_key[u] = map_position(map, -h, -k, -l);
+    // reciprocal_vector (src/density_functionals.cpp:34-39): h b0 + k b1 + l b2 per component.
+    const auto dot = [&](double x, double y, double z) {
+      return __dadd_rn(__dadd_rn(__dmul_rn(h, x), __dmul_rn(k, y)), __dmul_rn(l, z));
+    };
+    q[3 * u] = dot(b0.x, b1.x, b2.x);
+    q[3 * u + 1] = dot(b0.y, b1.y, b2.y);
+    q[3 * u + 2] = dot(b0.z, b1.z, b2.z);
+  }
+}
+
+DeviceSupport upload_support(Context& ctx, const FunctionalSupport& s) {
+  const std::size_t n = s.count;
+  std::size_t offset = 0;
+  auto take = [&](std::size_t bytes) {
+    const std::size_t at = offset;
+    offset += (bytes + 255) / 256 * 256;
+    return at;
+  };
+  const std::size_t o_val = take(16 * n), o_core = take(16 * n), o_down = take(s.collinear ? 16 * n : 0),
+                    o_flags = take(n), zeroed = offset, o_index = take(8 * n), o_opp = take(8 * n),
+                    o_q = take(24 * n), o_okey = take(4 * n), o_bits = take(8 * s.bits.size()),
+                    o_rank = take(4 * s.rank.size());
+  std::size_t o_hkl[3], o_in[3];
+  for (int f = 0; f < s.fields; ++f) {
+    o_hkl[f] = take(12 * s.field[f].count);
+    o_in[f] = take(16 * s.field[f].count);
+  }
+  auto* base = static_cast<unsigned char*>(ctx.staging_in.reserve(offset));
+  auto upload = [&](std::size_t at, const void* from, std::size_t bytes) {
+    if (bytes) SDFT_CUDA(cudaMemcpyAsync(base + at, from, bytes, cudaMemcpyHostToDevice, ctx.stream));
+  };
+  SDFT_CUDA(cudaMemsetAsync(base, 0, zeroed, ctx.stream));
+  upload(o_bits, s.bits.data(), 8 * s.bits.size());
+  upload(o_rank, s.rank.data(), 4 * s.rank.size());
+  const KeyMap map{reinterpret_cast<const std::uint64_t*>(base + o_bits),
+                   reinterpret_cast<const std::uint32_t*>(base + o_rank),
+                   {s.extent[0], s.extent[1], s.extent[2]}};
+  const double* r = s.reciprocal;
+  const V3 b0{r[0], r[1], r[2]}, b1{r[3], r[4], r[5]}, b2{r[6], r[7], r[8]};
+  auto* flags = base + o_flags;
+  auto* index = reinterpret_cast<long long*>(base + o_index);
+  auto* opposite = reinterpret_cast<long long*>(base + o_opp);
+  auto* opposite_key = reinterpret_cast<int*>(base + o_okey);
+  auto* q = reinterpret_cast<double*>(base + o_q);
+  for (int f = 0; f < s.fields; ++f) {
+    const KeyField& field = s.field[f];
+    if (!field.count) continue;
+    upload(o_hkl[f], field.hkl, 12 * field.count);
+    upload(o_in[f], field.values, 16 * field.count);
+    const std::size_t to = s.bit[f] == 1 ? o_val : s.bit[f] == 2 ? o_core : o_down;
+    const unsigned blocks = static_cast<unsigned>(std::min<std::size_t>(ceil_div(field.count, kKeyThreads), 148 * 8));
+    place_keys_kernel<<<blocks, kKeyThreads, 0, ctx.stream>>>(
+        reinterpret_cast<const int*>(base + o_hkl[f]), reinterpret_cast<const Cx<double>*>(base + o_in[f]),
+        field.count, map, s.shape[0], s.shape[1], s.shape[2], b0, b1, b2, s.bit[f],
+        reinterpret_cast<Cx<double>*>(base + to), flags, index, opposite, opposite_key, q);
+    SDFT_LAUNCH("place_keys_kernel");
+  }
+  DeviceSupport d;
+  d.keys.index = index;
+  d.keys.opposite = opposite;
+  d.keys.q = q;
+  d.keys.valence = reinterpret_cast<const Cx<double>*>(base + o_val);
+  d.keys.core = reinterpret_cast<const Cx<double>*>(base + o_core);
+  d.keys.flags = flags;
+  d.keys.opposite_key = opposite_key;
+  d.down = reinterpret_cast<const Cx<double>*>(base + o_down);
+  return d;
 }
 
 }  // namespace
@@ -437,41 +590,19 @@ FunctionalSupport functional_support(const double lattice[9], std::size_t count,
   auto scale = [](V3 v, double t) { return V3{v.x * t, v.y * t, v.z * t}; };
   const V3 b[3] = {scale(cross(a1, a2), 2.0 * kPi / det), scale(cross(a2, a0), 2.0 * kPi / det),
                    scale(cross(a0, a1), 2.0 * kPi / det)};
-  SortedField valence = sorted_field(count, hkl, density, "density");
-  for (const auto& v : valence.values)
-    if (!std::isfinite(v.re) || !std::isfinite(v.im))
-      throw InvalidArgument("non-finite valence density Fourier coefficient");
-  SortedField frozen;
-  if (core_count) frozen = sorted_field(core_count, core_hkl, core, "core");
+  s.fields = core_count ? 2 : 1;
+  s.field[0] = key_field(count, hkl, density);
+  s.field[1] = key_field(core_count, core_hkl, core);
+  s.bit[0] = 1;
+  s.bit[1] = 2;
   s.with_core = core_count != 0;
-  // Union in map order (the xc density's support).
-  std::size_t i = 0, j = 0;
-  while (i < valence.keys.size() || j < frozen.keys.size()) {
-    Cx<double> v{0, 0}, c{0, 0};
-    unsigned char f = 0;
-    Key k;
-    if (j == frozen.keys.size() || (i < valence.keys.size() && valence.keys[i] < frozen.keys[j])) {
-      k = valence.keys[i];
-      v = valence.values[i++];
-      f = 1;
-    } else if (i == valence.keys.size() || frozen.keys[j] < valence.keys[i]) {
-      k = frozen.keys[j];
-      c = frozen.values[j++];
-      f = 2;
-    } else {
-      k = valence.keys[i];
-      v = valence.values[i++];
-      c = frozen.values[j++];
-      f = 3;
-    }
-    const double xr = (f & 1 ? v.re : 0.0) + (f & 2 ? c.re : 0.0), xi = (f & 1 ? v.im : 0.0) + (f & 2 ? c.im : 0.0);
-    if (!std::isfinite(xr) || !std::isfinite(xi))
-      throw InvalidArgument("non-finite valence plus pseudo-core Fourier coefficient");
-    s.keys.push_back(k);
-    s.valence.push_back(v);
-    s.core.push_back(c);
-    s.flags.push_back(f);
-  }
+  const char* const names[] = {"density", "core"};
+  mark_keys(s, s.fields, names, [&](int f) {
+    if (f == 0 && !std::isfinite(largest(s.field[0])))
+      throw InvalidArgument("non-finite valence density Fourier coefficient");
+  });
+  if (s.with_core && !finite_sum(s.field[0], s.field[1]))
+    throw InvalidArgument("non-finite valence plus pseudo-core Fourier coefficient");
   int padding = env_padding();
   if (quadrature_padding) {
     if (quadrature_padding < 1 || quadrature_padding > 8) throw InvalidArgument("invalid XC quadrature override");
@@ -481,41 +612,40 @@ FunctionalSupport functional_support(const double lattice[9], std::size_t count,
   return s;
 }
 
-void density_functionals(Context& ctx, const FunctionalSupport& s, Cx<double>* potential, Cx<double>* xc_potential,
-                         FunctionalResult& result) {
+// The support's keys in map order: the bitmap's marked cells in raster order.
+void write_support(const FunctionalSupport& s, std::int32_t* hkl) {
+  const int n1 = 2 * s.extent[1] + 1, n2 = 2 * s.extent[2] + 1;
+  for (std::size_t w = 0; w < s.bits.size(); ++w) {
+    std::uint64_t word = s.bits[w];
+    if (!word) continue;
+    const long long first = static_cast<long long>(w) * 64;
+    long long row = first / n2;
+    int l = static_cast<int>(first - row * n2), bit = 0;
+    while (word) {
+      const int next = __builtin_ctzll(word);
+      word &= word - 1;
+      l += next - bit;
+      bit = next;
+      while (l >= n2) {
+        l -= n2;
+        ++row;
+      }
+      hkl[0] = static_cast<int>(row / n1) - s.extent[0];
+      hkl[1] = static_cast<int>(row % n1) - s.extent[1];
+      hkl[2] = l - s.extent[2];
+      hkl += 3;
+    }
+  }
+}
+
+void density_functionals(Context& ctx, const FunctionalSupport& s, std::int32_t* support_hkl, Cx<double>* potential,
+                         Cx<double>* xc_potential, FunctionalResult& result) {
   SDFT_CUDA(cudaSetDevice(ctx.device));
-  const int count = static_cast<int>(s.keys.size());
+  const int count = static_cast<int>(s.count);
+  const std::size_t n = s.count;
   const long long points = s.points;
   const int grids_used = s.with_core ? 4 : 2;
-  // Key arrays, packed into one upload.
-  const std::size_t n = s.keys.size();
-  std::size_t offset = 0;
-  auto take = [&](std::size_t bytes) {
-    const std::size_t at = offset;
-    offset += (bytes + 255) / 256 * 256;
-    return at;
-  };
-  const std::size_t o_index = take(8 * n), o_opp = take(8 * n), o_q = take(24 * n), o_val = take(16 * n),
-                    o_core = take(16 * n), o_flags = take(n), o_okey = take(4 * n);
-  std::vector<unsigned char> host(offset);
-  std::memcpy(host.data() + o_index, s.index.data(), 8 * n);
-  std::memcpy(host.data() + o_opp, s.opposite.data(), 8 * n);
-  std::memcpy(host.data() + o_q, s.q.data(), 24 * n);
-  std::memcpy(host.data() + o_val, s.valence.data(), 16 * n);
-  std::memcpy(host.data() + o_core, s.core.data(), 16 * n);
-  std::memcpy(host.data() + o_flags, s.flags.data(), n);
-  std::memcpy(host.data() + o_okey, s.opposite_key.data(), 4 * n);
-  auto* dkeys = static_cast<unsigned char*>(ctx.staging_in.reserve(offset));
-  SDFT_CUDA(cudaMemcpyAsync(dkeys, host.data(), offset, cudaMemcpyHostToDevice, ctx.stream));
-  KeyData keys;
-  keys.index = reinterpret_cast<const long long*>(dkeys + o_index);
-  keys.opposite = reinterpret_cast<const long long*>(dkeys + o_opp);
-  keys.q = reinterpret_cast<const double*>(dkeys + o_q);
-  keys.valence = reinterpret_cast<const Cx<double>*>(dkeys + o_val);
-  keys.core = reinterpret_cast<const Cx<double>*>(dkeys + o_core);
-  keys.flags = dkeys + o_flags;
-  keys.opposite_key = reinterpret_cast<const int*>(dkeys + o_okey);
-
+  const KeyData keys = upload_support(ctx, s).keys;
   auto* grids = static_cast<Cx<double>*>(ctx.slab64.reserve(sizeof(Cx<double>) * points * grids_used));
   SDFT_CUDA(cudaMemsetAsync(grids, 0, sizeof(Cx<double>) * points * grids_used, ctx.stream));
   const unsigned key_blocks = static_cast<unsigned>(std::min<long long>(ceil_div(count, kKeyThreads), 148LL * 8));
@@ -550,6 +680,7 @@ void density_functionals(Context& ctx, const FunctionalSupport& s, Cx<double>* p
   xc_merge_kernel<<<1, kTileThreads, 0, ctx.stream>>>(key_partials, key_blocks, kKeySums, nullptr, nullptr,
                                                       merged + 2 * kSums + 2);
   SDFT_LAUNCH("xc_merge_kernel keys");
+  write_support(s, support_hkl);  // while the device works
   std::vector<double> scalars(2 * (kSums + kKeySums) + 4);
   SDFT_CUDA(cudaMemcpyAsync(scalars.data(), merged, sizeof(double) * scalars.size(), cudaMemcpyDeviceToHost,
                             ctx.stream));
@@ -813,43 +944,17 @@ FunctionalSupport collinear_support(const double lattice[9], const std::size_t c
   auto scale = [](V3 v, double t) { return V3{v.x * t, v.y * t, v.z * t}; };
   const V3 b[3] = {scale(cross(a1, a2), 2.0 * kPi / det), scale(cross(a2, a0), 2.0 * kPi / det),
                    scale(cross(a0, a1), 2.0 * kPi / det)};
-  const SortedField up = sorted_field(count[0], hkl[0], density[0], "spin density");
-  const SortedField dn = sorted_field(count[1], hkl[1], density[1], "spin density");
-  SortedField frozen;
-  if (core_count) frozen = sorted_field(core_count, core_hkl, core, "core");
+  s.fields = core_count ? 3 : 2;
+  for (int c = 0; c < 2; ++c) s.field[c] = key_field(count[c], hkl[c], density[c]);
+  s.field[2] = key_field(core_count, core_hkl, core);
+  s.bit[0] = 1;
+  s.bit[1] = 4;
+  s.bit[2] = 2;
   s.with_core = core_count != 0;
-  // Three-way union in map order.
-  std::size_t i = 0, j = 0, k = 0;
-  while (i < up.keys.size() || j < dn.keys.size() || k < frozen.keys.size()) {
-    Key least{INT32_MAX, INT32_MAX, INT32_MAX};
-    if (i < up.keys.size()) least = std::min(least, up.keys[i]);
-    if (j < dn.keys.size()) least = std::min(least, dn.keys[j]);
-    if (k < frozen.keys.size()) least = std::min(least, frozen.keys[k]);
-    Cx<double> u{0, 0}, d{0, 0}, c{0, 0};
-    unsigned char f = 0;
-    if (i < up.keys.size() && up.keys[i] == least) {
-      u = up.values[i++];
-      f |= 1;
-    }
-    if (j < dn.keys.size() && dn.keys[j] == least) {
-      d = dn.values[j++];
-      f |= 4;
-    }
-    if (k < frozen.keys.size() && frozen.keys[k] == least) {
-      c = frozen.values[k++];
-      f |= 2;
-    }
-    // The total density (:752-756) must be finite.
-    if (f & 5) {
-      const double tr = (f & 1 ? u.re : 0.0) + (f & 4 ? d.re : 0.0), ti = (f & 1 ? u.im : 0.0) + (f & 4 ? d.im : 0.0);
-      if (!std::isfinite(tr) || !std::isfinite(ti)) throw InvalidArgument("nonfinite spin density");
-    }
-    s.keys.push_back(least);
-    s.valence.push_back(u);
-    s.down.push_back(d);
-    s.core.push_back(c);
-    s.flags.push_back(f);
-  }
+  const char* const names[] = {"spin density", "spin density", "core"};
+  mark_keys(s, s.fields, names, [](int) {});
+  // The total density (:752-756) must be finite.
+  if (!finite_sum(s.field[0], s.field[1])) throw InvalidArgument("nonfinite spin density");
   if (!padding) {
     padding = 2;
     if (const char* v = std::getenv("SDFT_FFT_OVERSAMPLING")) {
@@ -864,41 +969,17 @@ FunctionalSupport collinear_support(const double lattice[9], const std::size_t c
   return s;
 }
 
-void collinear_functionals(Context& ctx, const FunctionalSupport& s, Cx<double>* const potential[2],
-                           Cx<double>* const xc_potential[2], FunctionalResult result[2]) {
+void collinear_functionals(Context& ctx, const FunctionalSupport& s, std::int32_t* support_hkl,
+                           Cx<double>* const potential[2], Cx<double>* const xc_potential[2],
+                           FunctionalResult result[2]) {
   if (!s.collinear) throw InvalidArgument("collinear functional needs a collinear support");
   SDFT_CUDA(cudaSetDevice(ctx.device));
-  const int count = static_cast<int>(s.keys.size());
+  const int count = static_cast<int>(s.count);
+  const std::size_t n = s.count;
   const long long points = s.points;
-  const std::size_t n = s.keys.size();
-  std::size_t offset = 0;
-  auto take = [&](std::size_t bytes) {
-    const std::size_t at = offset;
-    offset += (bytes + 255) / 256 * 256;
-    return at;
-  };
-  const std::size_t o_index = take(8 * n), o_opp = take(8 * n), o_q = take(24 * n), o_val = take(16 * n),
-                    o_core = take(16 * n), o_down = take(16 * n), o_flags = take(n), o_okey = take(4 * n);
-  std::vector<unsigned char> host(offset);
-  std::memcpy(host.data() + o_index, s.index.data(), 8 * n);
-  std::memcpy(host.data() + o_opp, s.opposite.data(), 8 * n);
-  std::memcpy(host.data() + o_q, s.q.data(), 24 * n);
-  std::memcpy(host.data() + o_val, s.valence.data(), 16 * n);
-  std::memcpy(host.data() + o_core, s.core.data(), 16 * n);
-  std::memcpy(host.data() + o_down, s.down.data(), 16 * n);
-  std::memcpy(host.data() + o_flags, s.flags.data(), n);
-  std::memcpy(host.data() + o_okey, s.opposite_key.data(), 4 * n);
-  auto* dkeys = static_cast<unsigned char*>(ctx.staging_in.reserve(offset));
-  SDFT_CUDA(cudaMemcpyAsync(dkeys, host.data(), offset, cudaMemcpyHostToDevice, ctx.stream));
-  KeyData keys;
-  keys.index = reinterpret_cast<const long long*>(dkeys + o_index);
-  keys.opposite = reinterpret_cast<const long long*>(dkeys + o_opp);
-  keys.q = reinterpret_cast<const double*>(dkeys + o_q);
-  keys.valence = reinterpret_cast<const Cx<double>*>(dkeys + o_val);
-  keys.core = reinterpret_cast<const Cx<double>*>(dkeys + o_core);
-  keys.flags = dkeys + o_flags;
-  keys.opposite_key = reinterpret_cast<const int*>(dkeys + o_okey);
-  const auto* down = reinterpret_cast<const Cx<double>*>(dkeys + o_down);
+  const DeviceSupport support = upload_support(ctx, s);
+  const KeyData keys = support.keys;
+  const Cx<double>* down = support.down;
 
   auto* grids = static_cast<Cx<double>*>(ctx.slab64.reserve(sizeof(Cx<double>) * points * 4));
   SDFT_CUDA(cudaMemsetAsync(grids, 0, sizeof(Cx<double>) * points * 4, ctx.stream));
@@ -944,6 +1025,7 @@ void collinear_functionals(Context& ctx, const FunctionalSupport& s, Cx<double>*
   xc_merge_kernel<<<1, kTileThreads, 0, ctx.stream>>>(key_partials, key_blocks, kSpinKeySums, nullptr, nullptr,
                                                       merged + 2 * stride);
   SDFT_LAUNCH("xc_merge_kernel spin keys");
+  write_support(s, support_hkl);  // while the device works
   std::vector<double> scalars(3 * stride);
   unsigned int bad = 0;
   SDFT_CUDA(cudaMemcpyAsync(scalars.data(), merged, sizeof(double) * scalars.size(), cudaMemcpyDeviceToHost,
@@ -979,9 +1061,9 @@ void collinear_functionals(Context& ctx, const FunctionalSupport& s, Cx<double>*
     r.grid_points = static_cast<std::uint64_t>(points);
     for (int a = 0; a < 3; ++a) r.grid[a] = s.shape[a];
     r.sampled_electrons = 0.0;
-    for (std::size_t u = 0; u < n; ++u)
-      if (s.keys[u] == Key{0, 0, 0} && (s.flags[u] & (c == 0 ? 1 : 4)))
-        r.sampled_electrons = s.volume * (c == 0 ? s.valence[u].re : s.down[u].re);
+    for (std::size_t u = 0; u < s.field[c].count; ++u)
+      if (!s.field[c].hkl[3 * u] && !s.field[c].hkl[3 * u + 1] && !s.field[c].hkl[3 * u + 2])
+        r.sampled_electrons = s.volume * s.field[c].values[2 * u];
   }
 }
 

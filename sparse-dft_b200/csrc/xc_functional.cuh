@@ -2,7 +2,6 @@
 // (xc_functional.cu): the reference's evaluate_density_functionals,
 // src/density_functionals.hpp:40-47 (src/density_functionals.cpp:462-729).
 #pragma once
-#include <array>
 #include <cstdint>
 #include <vector>
 
@@ -10,20 +9,30 @@
 
 namespace sdft_b200 {
 
-// The union support of the density and the frozen core in the reference's
-// map order, with what the device passes need per key.
+// One Fourier field in the caller's arrays (hkl x3, interleaved values).
+struct KeyField {
+  std::size_t count = 0;
+  const int* hkl = nullptr;
+  const double* values = nullptr;
+};
+
+// The union support of the density and the frozen core: a bitmap of the box
+// |h|, |k|, |l| <= extent whose raster order is the reference's map order, and
+// the fields, still in the caller's arrays (which outlive the call).
 struct FunctionalSupport {
   double volume = 0;
+  double reciprocal[9] = {};  // rows b1, b2, b3
   bool with_core = false;
+  bool collinear = false;  // two spin channels
   int shape[3] = {0, 0, 0};
   long long points = 0;
-  bool collinear = false;                // two spin channels: valence = up, down = down
-  std::vector<std::array<int, 3>> keys;  // sorted lexicographically
-  std::vector<Cx<double>> valence, core, down;  // 0 where the key is absent
-  std::vector<unsigned char> flags;      // bit 0: density (up) key, bit 1: core key, bit 2: down key
-  std::vector<long long> index, opposite;  // wrapped grid index of +G, -G
-  std::vector<int> opposite_key;           // union position of -G, or -1
-  std::vector<double> q;                   // G per key, 3 values
+  int extent[3] = {0, 0, 0};
+  std::vector<std::uint64_t> bits;   // bit `cell` of the box
+  std::vector<std::uint32_t> rank;   // support keys before each word
+  std::size_t count = 0;             // keys of the union
+  int fields = 0;
+  KeyField field[3];
+  unsigned char bit[3] = {};  // flag of each field: 1 density (up), 2 core, 4 down
 };
 
 // Scalars of the reference's DensityFunctionals (stresses row-major 3 x 3).
@@ -44,10 +53,10 @@ FunctionalSupport functional_support(const double lattice[9], std::size_t count,
                                      const double* density, std::size_t core_count, const int* core_hkl,
                                      const double* core, int quadrature_padding);
 
-// Device part: potential (Hartree + v_xc) and v_xc on the support's keys, in
-// its order, into host arrays; the scalars into result.
-void density_functionals(Context& ctx, const FunctionalSupport& support, Cx<double>* potential,
-                         Cx<double>* xc_potential, FunctionalResult& result);
+// Device part: the support's keys, and the potential (Hartree + v_xc) and v_xc
+// on them, into host arrays; the scalars into result.
+void density_functionals(Context& ctx, const FunctionalSupport& support, std::int32_t* support_hkl,
+                         Cx<double>* potential, Cx<double>* xc_potential, FunctionalResult& result);
 
 // Collinear spin form (the reference's evaluate_collinear_density_functionals,
 // src/density_functionals.hpp:52-56, src/density_functionals.cpp:732-806):
@@ -59,7 +68,8 @@ void density_functionals(Context& ctx, const FunctionalSupport& support, Cx<doub
 FunctionalSupport collinear_support(const double lattice[9], const std::size_t count[2], const int* const hkl[2],
                                     const double* const density[2], std::size_t core_count, const int* core_hkl,
                                     const double* core, int padding);
-void collinear_functionals(Context& ctx, const FunctionalSupport& support, Cx<double>* const potential[2],
-                           Cx<double>* const xc_potential[2], FunctionalResult result[2]);
+void collinear_functionals(Context& ctx, const FunctionalSupport& support, std::int32_t* support_hkl,
+                           Cx<double>* const potential[2], Cx<double>* const xc_potential[2],
+                           FunctionalResult result[2]);
 
 }  // namespace sdft_b200

@@ -205,3 +205,47 @@ def test_collinear_support_query_and_checks_are_host_only(golden):
                                       np.zeros(0), support_only=True)
     with pytest.raises(C.InvalidArgument, match="invalid collinear XC padding"):
         density.collinear_functionals(None, *args, padding=9, support_only=True)
+
+
+def support_count(keys, values, core_keys=None, core=None, padding=0):
+    """(status, union size) of the functional's host-only support query."""
+    lib = C.library()
+    lat = np.ascontiguousarray(np.eye(3) * 10.0).reshape(9)
+    k = np.ascontiguousarray(keys, dtype=np.int32).reshape(-1, 3)
+    v = np.ascontiguousarray(values, dtype=np.complex128)
+    ck = np.ascontiguousarray(np.zeros((0, 3)) if core_keys is None else core_keys, dtype=np.int32).reshape(-1, 3)
+    cv = np.ascontiguousarray(np.zeros(0) if core is None else core, dtype=np.complex128)
+    count = ctypes.c_size_t()
+    status = lib.sdft_b200_density_functionals(None, lat.ctypes.data_as(C.D), k.shape[0], k.ctypes.data_as(C.I32),
+                                               v.ctypes.data_as(C.D), ck.shape[0], ck.ctypes.data_as(C.I32),
+                                               cv.ctypes.data_as(C.D), padding, None, None, None, 0,
+                                               ctypes.byref(count), None)
+    return status, count.value
+
+
+@pytest.mark.parametrize("box", [(0, 0, 0), (1, 0, 5), (0, 7, 0), (3, 4, 5), (31, 1, 0), (127, 2, 3)])
+def test_support_bitmap_counts_the_union(box):
+    """Random key sets in boxes down to a point or a line, the core inside and past the density's box."""
+    rng = np.random.Generator(np.random.PCG64(sum(box)))
+    every = np.stack(np.meshgrid(*[np.arange(-m, m + 1) for m in box], indexing="ij"), axis=-1).reshape(-1, 3)
+    keys = every[rng.permutation(len(every))[:max(1, len(every) // 2)]]
+    core = np.concatenate([every[rng.permutation(len(every))[:max(1, len(every) // 3)]], [[0, 0, 9], [0, -8, 0]]])
+    core = np.unique(core, axis=0)[::-1]
+    union = {tuple(k) for k in keys.tolist()} | {tuple(k) for k in core.tolist()}
+    assert support_count(keys, np.ones(len(keys))) == (C.OK, len(keys))
+    assert support_count(keys, np.ones(len(keys)), core, np.ones(len(core))) == (C.OK, len(union))
+
+
+def test_support_checks_keep_their_order():
+    """Repeated keys are reported before the grid limit, on both sides of the bitmap's box; sums of finite
+    values that overflow are refused; the widest padding-1 grid (511 points) is accepted."""
+    for far in (3, 300, 10**6):
+        assert support_count([[far, 0, 0], [far, 0, 0]], [1.0, 1.0])[0] == C.INVALID_ARGUMENT
+        assert "duplicate" in C.last_error()
+    assert support_count([[256, 0, 0], [0, 0, 0]], [1.0, 1.0], padding=1)[0] == C.INVALID_ARGUMENT
+    assert "above 512" in C.last_error()
+    assert support_count([[255, 0, 0], [-255, 0, 0]], [1.0, 1.0], padding=1) == (C.OK, 2)
+    big = [1.5e308]
+    assert support_count([[1, 0, 0]], big, [[0, 1, 0]], big) == (C.OK, 2)
+    assert support_count([[1, 0, 0]], big, [[1, 0, 0]], big)[0] == C.INVALID_ARGUMENT
+    assert "pseudo-core" in C.last_error()
