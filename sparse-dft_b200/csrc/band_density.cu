@@ -1,16 +1,18 @@
 // Band density Sum_b f_b/Omega |psi_b(r)|^2 and its Fourier coefficients on a
-// support (src/density_functionals.cpp:407-460), as three pruned FP64 passes
-// over all occupied bands followed by one forward 3D FFT:
+// support (src/density_functionals.cpp:407-460), as pruned FP64 passes over all
+// occupied bands followed by one forward 3D FFT:
 //
-//   rows     (per active i0 row, block of active i1 rows, band): scatter the
-//            sphere points into shared memory, backward FFT along i2, store
-//            only the active (i0, i1) rows.
-//   columns  (per active i0 row, 32 i2 columns, band): zero-pad the active i1
-//            entries to n1, backward FFT along i1, store the i0 plane.
-//   pencils  (per 32 (i1, i2) lines, looping over the bands): zero-pad the
-//            active i0 entries to n0, backward FFT along i0 and accumulate
-//            f_b/Omega |.|^2 in shared memory in band order; the density
-//            line is written once.
+//   planes   (per active i0 row and band; split_planes_in): scatter the sphere
+//            points into shared memory, backward FFT along i2 on the active i1
+//            rows and along i1, store the i0 plane.
+//   pencils  (per block of (i1, i2) lines, looping over the bands;
+//            split_density_pencils): zero-pad the active i0 entries to n0,
+//            backward FFT along i0 and accumulate f_b/Omega |.|^2 in registers
+//            in band order; the density line is written once.
+//
+// Axis lengths without a split into two transforms of at most 16 points (125),
+// and planes beyond shared memory, take rows (i2 transforms of the active rows
+// through HBM), columns (i1) and pencils kernels on radix stages in shared memory.
 //
 // The density grid is then transformed forward in place (unnormalised) and
 // the support keys gathered and divided by N (src/density_functionals.cpp:269-284).
@@ -23,6 +25,7 @@
 
 #include "band_density.cuh"
 #include "operator.cuh"
+#include "split_fft.cuh"
 
 namespace sdft_b200 {
 
@@ -203,20 +206,23 @@ int wrap(int p, int n) {
 }
 
 template <int TL>
-void launch_passes(const DensityArgs& a, const Cx<double>* psi, long long npw, int bands, int rows_per_cta,
-                   Cx<double>* rows, Cx<double>* planes, bool accumulate, Cx<double>* grid, unsigned int* flags,
-                   cudaStream_t stream) {
-  const std::size_t rows_smem =
-      sizeof(Cx<double>) * (a.n2 + 2 * static_cast<std::size_t>(rows_per_cta) * (a.n2 | 1));
-  allow(density_rows_kernel, rows_smem);
-  const dim3 g1(a.slots, static_cast<unsigned>(ceil_div(a.krows, rows_per_cta)), bands);
-  density_rows_kernel<<<g1, kThreads, rows_smem, stream>>>(psi, npw, a, rows_per_cta, rows, flags);
-  SDFT_LAUNCH("density_rows_kernel");
-  const std::size_t c_smem = column_smem(a.n1, TL);
-  allow(density_columns_kernel<TL>, c_smem);
-  const dim3 g2(static_cast<unsigned>(ceil_div(a.n2, TL)), a.slots, bands);
-  density_columns_kernel<TL><<<g2, kThreads, c_smem, stream>>>(rows, a, planes);
-  SDFT_LAUNCH("density_columns_kernel");
+void launch_passes(const SpherePlan& plan, const DensityArgs& a, const Cx<double>* psi, long long npw, int bands,
+                   int rows_per_cta, Cx<double>* rows, Cx<double>* planes, bool accumulate, Cx<double>* grid,
+                   unsigned int* flags, cudaStream_t stream) {
+  if (!split_planes_in<double>(plan, psi, npw, a.band, bands, planes, a.tw1, a.tw2, flags, stream)) {
+    const std::size_t rows_smem =
+        sizeof(Cx<double>) * (a.n2 + 2 * static_cast<std::size_t>(rows_per_cta) * (a.n2 | 1));
+    allow(density_rows_kernel, rows_smem);
+    const dim3 g1(a.slots, static_cast<unsigned>(ceil_div(a.krows, rows_per_cta)), bands);
+    density_rows_kernel<<<g1, kThreads, rows_smem, stream>>>(psi, npw, a, rows_per_cta, rows, flags);
+    SDFT_LAUNCH("density_rows_kernel");
+    const std::size_t c_smem = column_smem(a.n1, TL);
+    allow(density_columns_kernel<TL>, c_smem);
+    const dim3 g2(static_cast<unsigned>(ceil_div(a.n2, TL)), a.slots, bands);
+    density_columns_kernel<TL><<<g2, kThreads, c_smem, stream>>>(rows, a, planes);
+    SDFT_LAUNCH("density_columns_kernel");
+  }
+  if (split_density_pencils(plan, planes, a.weight, bands, accumulate, grid, a.tw0, stream)) return;
   const std::size_t p_smem = pencil_smem(a.n0, TL);
   allow(density_pencils_kernel<TL>, p_smem);
   const unsigned g3 = static_cast<unsigned>(ceil_div(static_cast<std::size_t>(a.n12), TL));
@@ -325,7 +331,8 @@ void band_density(Context& ctx, const std::int32_t* hkl, std::size_t npw, const 
   const int rows_per_cta = std::max(
       1, std::min<int>(plan.krows, static_cast<int>((kSmemLimit - sizeof(Cx<double>) * shape[2]) /
                                                     (2 * sizeof(Cx<double>) * n2p))));
-  const std::size_t rows_band = static_cast<std::size_t>(plan.slots) * plan.krows * shape[2];
+  const std::size_t rows_band =
+      split_planes_fit<double>(plan) ? 0 : static_cast<std::size_t>(plan.slots) * plan.krows * shape[2];
   const std::size_t planes_band = static_cast<std::size_t>(plan.slots) * n12;
   const std::size_t per_band = sizeof(Cx<double>) * (rows_band + planes_band);
   const std::size_t chunk = std::max<std::size_t>(
@@ -342,13 +349,13 @@ void band_density(Context& ctx, const std::int32_t* hkl, std::size_t npw, const 
       c.weight = d_weight + first;
       const bool accumulate = first > 0;
       if (tl == 32)
-        launch_passes<32>(c, psi, static_cast<long long>(npw), width, rows_per_cta, rows, planes, accumulate, grid,
+        launch_passes<32>(plan, c, psi, static_cast<long long>(npw), width, rows_per_cta, rows, planes, accumulate, grid,
                           flags, ctx.stream);
       else if (tl == 16)
-        launch_passes<16>(c, psi, static_cast<long long>(npw), width, rows_per_cta, rows, planes, accumulate, grid,
+        launch_passes<16>(plan, c, psi, static_cast<long long>(npw), width, rows_per_cta, rows, planes, accumulate, grid,
                           flags, ctx.stream);
       else
-        launch_passes<8>(c, psi, static_cast<long long>(npw), width, rows_per_cta, rows, planes, accumulate, grid,
+        launch_passes<8>(plan, c, psi, static_cast<long long>(npw), width, rows_per_cta, rows, planes, accumulate, grid,
                          flags, ctx.stream);
     }
   }

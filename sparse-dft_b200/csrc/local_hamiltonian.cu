@@ -12,6 +12,11 @@
 //   plane_out  (per active i0 and column): forward FFT along i1 and i2, gather
 //              the sphere points, y = T x + value/N.
 //
+// In FP32 the common lengths take the register-resident line kernels below, all
+// other splittable lengths and FP64 the four-step kernels of split_fft.cu; the
+// radix-stage kernels here remain for lengths without a split and planes beyond
+// shared memory.
+//
 // Rows i0 outside the sphere's span never reach HBM: the slab holds
 // slots*n1*n2 complex values per column instead of n0*n1*n2.
 #include <algorithm>
@@ -21,6 +26,7 @@
 #include <type_traits>
 
 #include "local_hamiltonian.cuh"
+#include "split_fft.cuh"
 
 namespace sdft_b200 {
 
@@ -28,15 +34,6 @@ namespace {
 
 constexpr int kThreads = 256;
 constexpr int kPencilLines = 32;
-// Resident CTAs per SM the fixed plane and pencil kernels are compiled for:
-// four in FP32 (64 registers; at N = 70 plane_out spills 144 B and still
-// runs faster than at three CTAs: the passes are latency-bound), one in FP64,
-// whose butterfly registers would spill under a tighter bound.
-template <typename T>
-constexpr int plane_blocks() {
-  return sizeof(T) == 4 ? 4 : 1;
-}
-
 template <typename T>
 struct LocalArgs {
   int n0, n1, n2, n2p, slots, krows;
@@ -116,68 +113,6 @@ __global__ void __launch_bounds__(kThreads) pencil_kernel(Cx<T>* __restrict__ sl
   __syncthreads();
   Cx<T>* back = fft_lines_pp<T, false>(field, field == tile_a ? tile_b : tile_a, lines, 1, STRIDE, nullptr, a.p0, tw0);
   for (int idx = tid; idx < a.slots * TL; idx += blockDim.x) {
-    const int s = idx / TL, t = idx - s * TL;
-    if (t < lines) base[static_cast<long long>(s) * a.n12 + t] = back[a.slot_row[s] * STRIDE + t];
-  }
-}
-
-// pencil_kernel for a compile-time axis length N0: every entry of the tile is
-// written once (slab value or zero), and the stages unroll with constant
-// index arithmetic.
-template <typename T, int N0>
-__global__ void __launch_bounds__(kThreads, plane_blocks<T>()) pencil_fixed_kernel(Cx<T>* __restrict__ slab, LocalArgs<T> a,
-                                                                const T* __restrict__ potential) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  constexpr int TL = kPencilLines, STRIDE = TL + 1;
-  Cx<T>* tw0 = reinterpret_cast<Cx<T>*>(smem_raw);
-  Cx<T>* tile_a = tw0 + N0;
-  Cx<T>* tile_b = tile_a + N0 * STRIDE;
-  int* slot_of_row = reinterpret_cast<int*>(tile_b + N0 * STRIDE);
-  const long long kl0 = static_cast<long long>(blockIdx.x) * TL;
-  const int c = blockIdx.y;
-  const int lines = static_cast<int>(min(static_cast<long long>(TL), a.n12 - kl0));
-  const int tid = threadIdx.x;
-  for (int i = tid; i < N0; i += kThreads) {
-    tw0[i] = a.tw0[i];
-    slot_of_row[i] = -1;
-  }
-  __syncthreads();
-  for (int s = tid; s < a.slots; s += kThreads) slot_of_row[a.slot_row[s]] = s;
-  __syncthreads();
-  Cx<T>* base = slab + static_cast<long long>(c) * a.slots * a.n12 + kl0;
-  // All of the thread's slab entries and V(r) values are loaded before the
-  // first transform, so the loads are in flight together.
-  constexpr int PER = (N0 * TL + kThreads - 1) / kThreads;
-  Cx<T> entry[PER];
-  T pot[PER];
-#pragma unroll
-  for (int q = 0; q < PER; ++q) {
-    const int idx = tid + q * kThreads;
-    const int i = idx / TL, t = idx - i * TL;
-    entry[q] = Cx<T>{0, 0};
-    pot[q] = T(0);
-    if (idx < N0 * TL && t < lines) {
-      const int s = slot_of_row[i];
-      if (s >= 0) entry[q] = base[static_cast<long long>(s) * a.n12 + t];
-      pot[q] = potential[static_cast<long long>(i) * a.n12 + kl0 + t];
-    }
-  }
-#pragma unroll
-  for (int q = 0; q < PER; ++q) {
-    const int idx = tid + q * kThreads;
-    if (idx < N0 * TL) tile_a[(idx / TL) * STRIDE + idx % TL] = entry[q];
-  }
-  __syncthreads();
-  Cx<T>* field = fft_lines_fixed<T, true, N0, TL, kThreads>(tile_a, tile_b, 1, STRIDE, tw0);
-#pragma unroll
-  for (int q = 0; q < PER; ++q) {
-    const int idx = tid + q * kThreads;
-    const int i = idx / TL, t = idx - i * TL;
-    if (idx < N0 * TL && t < lines) field[i * STRIDE + t] = cscale(field[i * STRIDE + t], pot[q]);
-  }
-  __syncthreads();
-  Cx<T>* back = fft_lines_fixed<T, false, N0, TL, kThreads>(field, field == tile_a ? tile_b : tile_a, 1, STRIDE, tw0);
-  for (int idx = tid; idx < a.slots * TL; idx += kThreads) {
     const int s = idx / TL, t = idx - s * TL;
     if (t < lines) base[static_cast<long long>(s) * a.n12 + t] = back[a.slot_row[s] * STRIDE + t];
   }
@@ -459,105 +394,6 @@ long long resident_ctas(Kernel kernel, int threads, std::size_t smem) {
   return static_cast<long long>(std::max(per_sm, 1)) * sms;
 }
 
-// plane_in_kernel for compile-time axis lengths N1 = N2 = N, one plane
-// buffer (in-place stages): backward FFT along i2 on the active i1 rows, then
-// along i1 on every i2 column.
-template <typename T, int N>
-__global__ void __launch_bounds__(kThreads, plane_blocks<T>()) plane_in_fixed_kernel(const Cx<double>* __restrict__ x, long long ldx,
-                                                                  LocalArgs<T> a, Cx<T>* __restrict__ slab) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  Cx<T>* tw = reinterpret_cast<Cx<T>*>(smem_raw);
-  const int np = a.n2p, plane_elems = N * np;
-  Cx<T>* plane = tw + N;
-  int* rows = reinterpret_cast<int*>(plane + plane_elems);
-  const int s = blockIdx.x, c = blockIdx.y;
-  const int tid = threadIdx.x;
-  for (int i = tid; i < N; i += kThreads) tw[i] = a.tw2[i];
-  for (int i = tid; i < a.krows; i += kThreads) rows[i] = a.krow[i];
-  for (int i = tid; i < plane_elems; i += kThreads) plane[i] = Cx<T>{0, 0};
-  __syncthreads();
-  const Cx<double>* xc = x + static_cast<long long>(c) * ldx;
-  const int p_end = a.point_offset[s + 1];
-  for (int p = a.point_offset[s] + tid; p < p_end; p += kThreads)
-    plane[a.point_smem[p]] = cconvert<T>(xc[a.point_g[p]]);
-  __syncthreads();
-  fft_inplace_fixed<T, true, N, true, kThreads>(plane, a.krows, rows, np, 1, tw);
-  fft_inplace_fixed<T, true, N, false, kThreads>(plane, N, nullptr, 1, np, tw);
-  Cx<T>* out = slab + (static_cast<long long>(c) * a.slots + s) * (N * N);
-  for (int i = tid; i < N * N; i += kThreads) {
-    const int i1 = i / N, i2 = i - i1 * N;
-    out[i] = plane[i1 * np + i2];
-  }
-}
-
-// plane_out_kernel for N1 = N2 = N, one plane buffer: forward FFT along i1
-// on every column, along i2 on the active rows, gather, y = T x + value / count.
-template <typename T, int N>
-__global__ void __launch_bounds__(kThreads, plane_blocks<T>()) plane_out_fixed_kernel(const Cx<T>* __restrict__ slab, LocalArgs<T> a,
-                                                                   const Cx<double>* __restrict__ x, long long ldx,
-                                                                   const double* __restrict__ kinetic, double count,
-                                                                   Cx<double>* __restrict__ y, long long ldy) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  Cx<T>* tw = reinterpret_cast<Cx<T>*>(smem_raw);
-  const int np = a.n2p, plane_elems = N * np;
-  Cx<T>* plane = tw + N;
-  int* rows = reinterpret_cast<int*>(plane + plane_elems);
-  const int s = blockIdx.x, c = blockIdx.y;
-  const int tid = threadIdx.x;
-  for (int i = tid; i < N; i += kThreads) tw[i] = a.tw2[i];
-  for (int i = tid; i < a.krows; i += kThreads) rows[i] = a.krow[i];
-  const Cx<T>* in = slab + (static_cast<long long>(c) * a.slots + s) * (N * N);
-  // The plane's slab entries and the first points' x and T values are all
-  // requested before the transforms (one round of memory latency).
-  constexpr int PER = (N * N + kThreads - 1) / kThreads, POINTS = 4;
-  {
-    Cx<T> entry[PER];
-#pragma unroll
-    for (int q = 0; q < PER; ++q) {
-      const int i = tid + q * kThreads;
-      entry[q] = i < N * N ? in[i] : Cx<T>{0, 0};
-    }
-#pragma unroll
-    for (int q = 0; q < PER; ++q) {
-      const int i = tid + q * kThreads;
-      if (i < N * N) plane[(i / N) * np + i % N] = entry[q];
-    }
-  }
-  const Cx<double>* xc = x + static_cast<long long>(c) * ldx;
-  Cx<double>* yc = y + static_cast<long long>(c) * ldy;
-  const int p_begin = a.point_offset[s], p_end = a.point_offset[s + 1];
-  int pg[POINTS], ps[POINTS];
-  Cx<double> px[POINTS];
-  double pt[POINTS];
-#pragma unroll
-  for (int q = 0; q < POINTS; ++q) {
-    const int p = p_begin + tid + q * kThreads;
-    pg[q] = -1;
-    if (p < p_end) {
-      pg[q] = a.point_g[p];
-      ps[q] = a.point_smem[p];
-      px[q] = xc[pg[q]];
-      pt[q] = kinetic[pg[q]];
-    }
-  }
-  __syncthreads();
-  fft_inplace_fixed<T, false, N, false, kThreads>(plane, N, nullptr, 1, np, tw);
-  fft_inplace_fixed<T, false, N, true, kThreads>(plane, a.krows, rows, np, 1, tw);
-#pragma unroll
-  for (int q = 0; q < POINTS; ++q)
-    if (pg[q] >= 0) {
-      const Cx<double> v = cconvert<double>(plane[ps[q]]);
-      yc[pg[q]] = Cx<double>{pt[q] * px[q].re + v.re / count, pt[q] * px[q].im + v.im / count};
-    }
-  for (int p = p_begin + tid + POINTS * kThreads; p < p_end; p += kThreads) {
-    const int g = a.point_g[p];
-    const Cx<double> v = cconvert<double>(plane[a.point_smem[p]]);
-    const Cx<double> in_g = xc[g];
-    const double t = kinetic[g];
-    yc[g] = Cx<double>{t * in_g.re + v.re / count, t * in_g.im + v.im / count};
-  }
-}
-
 // FP32 plane passes with pair-split lines (fft_pair_dif / fft_pair_dit):
 // one CTA per (slot, column) plane, lane pair (l, l ^ 16) of warp w on line
 // 16 w + (l & 15). The i1 transform runs on the i2 columns, the i2 transform
@@ -778,51 +614,6 @@ bool launch_planes_pair(const SpherePlan& plan, const LocalArgs<T>& a, bool inwa
   }
 }
 
-// Plane passes with the compile-time kernels for square planes of the common
-// lengths; false when the plane has another shape.
-template <typename T>
-bool launch_planes_fixed(const LocalArgs<T>& a, bool inward, int columns, const Cx<double>* x, long long ldx,
-                         Cx<T>* slab, const double* kinetic, double count, Cx<double>* y, long long ldy,
-                         cudaStream_t stream) {
-  if (a.n1 != a.n2) return false;
-  const std::size_t smem = sizeof(Cx<T>) * (a.n1 + static_cast<std::size_t>(a.n1) * a.n2p) +
-                           sizeof(int) * static_cast<std::size_t>(a.krows);
-  const dim3 grid(a.slots, columns);
-  auto go = [&](auto in_kernel, auto out_kernel) {
-    if (inward) {
-      allow_smem(in_kernel, smem);
-      in_kernel<<<grid, kThreads, smem, stream>>>(x, ldx, a, slab);
-      SDFT_LAUNCH("plane_in_fixed_kernel");
-    } else {
-      allow_smem(out_kernel, smem);
-      out_kernel<<<grid, kThreads, smem, stream>>>(slab, a, x, ldx, kinetic, count, y, ldy);
-      SDFT_LAUNCH("plane_out_fixed_kernel");
-    }
-    return true;
-  };
-#define SDFT_PLANES(N) \
-  case N:              \
-    return go(plane_in_fixed_kernel<T, N>, plane_out_fixed_kernel<T, N>);
-  switch (a.n1) {
-    SDFT_PLANES(24)
-    SDFT_PLANES(35)
-    SDFT_PLANES(36)
-    SDFT_PLANES(45)
-    SDFT_PLANES(48)
-    SDFT_PLANES(60)
-    SDFT_PLANES(64)
-    SDFT_PLANES(70)
-    SDFT_PLANES(72)
-    SDFT_PLANES(80)
-    SDFT_PLANES(81)
-    SDFT_PLANES(84)
-    SDFT_PLANES(90)
-    SDFT_PLANES(96)
-    default: return false;
-  }
-#undef SDFT_PLANES
-}
-
 // FP32 pencil pass with the register kernel where n0 has one; false otherwise.
 template <typename T>
 bool launch_pencil_registers(const SpherePlan& plan, int columns, const T* potential, Cx<T>* slab,
@@ -890,37 +681,6 @@ bool launch_pencil_registers(const SpherePlan& plan, int columns, const T* poten
     }
   }
 }
-
-// Pencil pass with the compile-time kernel for the common axis lengths.
-template <typename T>
-bool launch_pencil_fixed(const LocalArgs<T>& a, int columns, const T* potential, Cx<T>* slab, cudaStream_t stream) {
-  const std::size_t smem =
-      sizeof(Cx<T>) * (a.n0 + 2 * static_cast<std::size_t>(a.n0) * (kPencilLines + 1)) + sizeof(int) * a.n0;
-  const dim3 grid(static_cast<unsigned>(ceil_div(static_cast<std::size_t>(a.n12), kPencilLines)), columns);
-  auto go = [&](auto kernel) {
-    allow_smem(kernel, smem);
-    kernel<<<grid, kThreads, smem, stream>>>(slab, a, potential);
-    SDFT_LAUNCH("pencil_fixed_kernel");
-    return true;
-  };
-  switch (a.n0) {
-    case 35: return go(pencil_fixed_kernel<T, 35>);
-    case 36: return go(pencil_fixed_kernel<T, 36>);
-    case 45: return go(pencil_fixed_kernel<T, 45>);
-    case 48: return go(pencil_fixed_kernel<T, 48>);
-    case 60: return go(pencil_fixed_kernel<T, 60>);
-    case 64: return go(pencil_fixed_kernel<T, 64>);
-    case 70: return go(pencil_fixed_kernel<T, 70>);
-    case 72: return go(pencil_fixed_kernel<T, 72>);
-    case 80: return go(pencil_fixed_kernel<T, 80>);
-    case 81: return go(pencil_fixed_kernel<T, 81>);
-    case 84: return go(pencil_fixed_kernel<T, 84>);
-    case 90: return go(pencil_fixed_kernel<T, 90>);
-    case 96: return go(pencil_fixed_kernel<T, 96>);
-    default: return false;
-  }
-}
-
 
 template <typename T>
 LocalArgs<T> make_args(const SpherePlan& plan) {
@@ -1042,7 +802,7 @@ void run_local_passes(const SpherePlan& plan, const LocalArgs<T>& a, double coun
   const dim3 planes(a.slots, columns);
   const bool planes_fit = plane_smem <= kMaxDynamicSmem;
   if (!launch_planes_pair<T>(plan, a, true, columns, x, ldx, slab, kinetic, count, y, ldy, stream) &&
-      !launch_planes_fixed<T>(a, true, columns, x, ldx, slab, kinetic, count, y, ldy, stream)) {
+      !split_planes_in<T>(plan, x, ldx, nullptr, columns, slab, a.tw1, a.tw2, nullptr, stream)) {
     if (planes_fit) {
       allow_smem(plane_in_kernel<T>, plane_smem);
       plane_in_kernel<T><<<planes, kThreads, plane_smem, stream>>>(x, ldx, a, slab);
@@ -1055,14 +815,14 @@ void run_local_passes(const SpherePlan& plan, const LocalArgs<T>& a, double coun
     }
   }
   if (!launch_pencil_registers<T>(plan, columns, potential, slab, stream) &&
-      !launch_pencil_fixed<T>(a, columns, potential, slab, stream)) {
+      !split_pencils<T>(plan, columns, potential, slab, a.tw0, stream)) {
     const dim3 pencils(static_cast<unsigned>(ceil_div(static_cast<std::size_t>(a.n12), kPencilLines)), columns);
     allow_smem(pencil_kernel<T>, pencil_smem);
     pencil_kernel<T><<<pencils, kThreads, pencil_smem, stream>>>(slab, a, potential);
     SDFT_LAUNCH("pencil_kernel");
   }
   if (!launch_planes_pair<T>(plan, a, false, columns, x, ldx, slab, kinetic, count, y, ldy, stream) &&
-      !launch_planes_fixed<T>(a, false, columns, x, ldx, slab, kinetic, count, y, ldy, stream)) {
+      !split_planes_out<T>(plan, slab, x, ldx, kinetic, count, y, ldy, columns, a.tw1, a.tw2, stream)) {
     if (planes_fit) {
       allow_smem(plane_out_kernel<T>, plane_smem);
       plane_out_kernel<T><<<planes, kThreads, plane_smem, stream>>>(slab, a, x, ldx, kinetic, count, y, ldy);

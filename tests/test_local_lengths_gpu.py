@@ -82,3 +82,27 @@ def test_operator_above_65535_plane_waves(context):
             assert relative_error(y32.T.cpu().numpy(), y64.T.cpu().numpy()) < 2e-5
     finally:
         op.close()
+
+
+# (Ecut, k) -> grid: axes of different lengths and splits (12 = 3 x 4, 14 = 2 x 7, 20 = 4 x 5, 18 = 3 x 6,
+# 30 = 5 x 6, 27 = 3 x 9, 49 = 7 x 7, 48 = 6 x 8), and 125 = 5 x 25, which has none.
+MIXED_AXES = {(4.0, (0.5, 0.0, 0.0)): (12, 14, 14), (9.0, (0.5, 0.25, 0.0)): (20, 18, 18),
+              (20.0, (0.0, 0.5, 0.5)): (30, 27, 27), (60.0, (0.0, 0.5, 0.0)): (49, 48, 49),
+              (390.0, (0.0, 0.0, 0.0)): (125, 125, 125)}
+
+
+@pytest.mark.parametrize("cell", list(MIXED_AXES), ids=lambda c: "x".join(str(n) for n in MIXED_AXES[c]))
+def test_local_apply_on_unequal_axes(context, cell):
+    """FP64 against the numpy oracle: both sum about 3 x 2 x log2(n^3) < 130 rounded terms of 1.1e-16 in
+    another order, so 130 x 1.1e-16 = 1.5e-14 bounds their relative difference; the mixed form at its bar."""
+    ecut, k = cell
+    inputs = synthetic.tiny(ecut_ha=ecut, kpoint=k, roots=4)
+    op = PlaneWaveOperator(context, inputs)
+    try:
+        assert op.shape == MIXED_AXES[cell]
+        x = probe_block(op.npw, 3, 7)
+        expected = sdft_oracle.Operator(inputs).local(x)
+        assert relative_error(op.local_apply(x, precision="fp64"), expected) < 1.5e-14
+        assert relative_error(op.local_apply(x, precision="mixed"), expected) < 2e-5
+    finally:
+        op.close()
