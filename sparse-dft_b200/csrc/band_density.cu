@@ -359,7 +359,7 @@ void band_density(Context& ctx, const std::int32_t* hkl, std::size_t npw, const 
                          flags, ctx.stream);
     }
   }
-  fft3d<double>(grid, shape, 1, false, ctx.stream);
+  fft3d(grid, shape, 1, false, ctx.stream);
   const unsigned blocks = static_cast<unsigned>(std::min<std::size_t>(ceil_div(count, 256), 148ULL * 16));
   gather_support_kernel<<<blocks, 256, 0, ctx.stream>>>(grid, shape[0], shape[1], shape[2], d_keys, count,
                                                         static_cast<double>(points), out);

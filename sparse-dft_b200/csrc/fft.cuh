@@ -381,86 +381,124 @@ __device__ Cx<T>* fft_lines_pp(Cx<T>* src, Cx<T>* dst, int count, int line_strid
   return src;
 }
 
+// D = A B + C of one warp, 8 x 8 x 4 in FP64. Lane l holds A(l / 4, l % 4),
+// B(l % 4, l / 4) and the pair C(l / 4, 2 (l % 4) + {0, 1}).
+__device__ __forceinline__ void mma_f64(double (&c)[2], double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+               : "+d"(c[0]), "+d"(c[1])
+               : "d"(a), "d"(b));
+}
+
 // Radix-R stage for a runtime odd prime R > 7 (a general length's large
 // factors), in two passes so that no thread holds R values. Pass 1 (src ->
 // dst), one butterfly (j, line) per item: applies the stage twiddles and
 // stores x0, the pair sums a_r = x_r + x_{R-r} and differences
 // b_r = x_r - x_{R-r} (r = 1..H, H = (R-1)/2) in the butterfly's R output
-// slots. Pass 2 (dst -> src), one output q per item: y_0 = x0 + sum_r a_r and
-// y_q = x0 + sum_r a_r cos(2 pi rq/R) -/+ i sum_r b_r sin(2 pi rq/R), the
-// arithmetic of radix_dft for the compiled odd radices, with the roots read
-// from the length-n table. The result is left in src.
-template <typename T, bool INV>
-__device__ void pp_stage_prime(Cx<T>* src, Cx<T>* dst, int count, int line_stride, int es, const int* rows, int n,
-                               int ns, int R, const Cx<T>* tw) {
-  const int m = n / R, twstride = n / (ns * R), unit = n / R, H = (R - 1) / 2;
-  for (int item = threadIdx.x; item < count * m; item += blockDim.x) {
+// slots. Pass 2 (dst -> src): C_q = sum_r a_r cos(2 pi rq/R) and
+// S_q = sum_r b_r sin(2 pi rq/R) for q = 1..H are two real matrix products over
+// all butterflies' (re, im) columns, on the FP64 matrix instruction, and
+// y_q = x0 + C_q -/+ i S_q, y_{R-q} = x0 + C_q +/- i S_q; y_0 = x0 + sum_r a_r.
+// A warp takes 8 outputs x 16 butterflies: each shared-memory value serves 8
+// outputs, where one output per thread read two values and a root for four
+// multiply-adds and was bound by shared memory (142 = 2 x 71 points: with the
+// lines that fft3d now leaves out, the Si64 functional's call went from 8.3 to
+// 5.5 ms). The result is left in src.
+template <bool INV>
+__device__ void pp_stage_prime(Cx<double>* src, Cx<double>* dst, int count, int line_stride, int es, int n, int ns,
+                               int R, const Cx<double>* tw) {
+  using C = Cx<double>;
+  const int m = n / R, twstride = n / (ns * R), unit = n / R, H = (R - 1) / 2, butterflies = count * m;
+  for (int item = threadIdx.x; item < butterflies; item += blockDim.x) {
     const int j = item / count, t = item - j * count;
     const int k = j % ns;
-    const int offset = (rows ? rows[t] : t) * line_stride;
-    const Cx<T>* in = src + offset;
-    Cx<T>* out = dst + offset + ((j / ns) * ns * R + k) * es;
+    const C* in = src + t * line_stride;
+    C* out = dst + t * line_stride + ((j / ns) * ns * R + k) * es;
     out[0] = in[j * es];
     for (int r = 1; r <= H; ++r) {
-      Cx<T> x = in[(j + r * m) * es], y = in[(j + (R - r) * m) * es];
+      C x = in[(j + r * m) * es], y = in[(j + (R - r) * m) * es];
       if (k > 0) {
-        x = cmul(x, twiddle<T, INV>(tw, r * k * twstride));
-        y = cmul(y, twiddle<T, INV>(tw, (R - r) * k * twstride));
+        x = cmul(x, twiddle<double, INV>(tw, r * k * twstride));
+        y = cmul(y, twiddle<double, INV>(tw, (R - r) * k * twstride));
       }
       out[r * ns * es] = x + y;
       out[(H + r) * ns * es] = x - y;
     }
   }
   __syncthreads();
-  for (int item = threadIdx.x; item < count * n; item += blockDim.x) {
-    const int o = item / count, t = item - o * count;
-    const int j = o / R, q = o - j * R;
-    const int k = j % ns;
-    const int offset = (rows ? rows[t] : t) * line_stride;
-    const Cx<T>* packed = dst + offset + ((j / ns) * ns * R + k) * es;
-    const Cx<T> x0 = packed[0];
-    Cx<T> y;
-    if (q == 0) {
-      y = x0;
-      for (int r = 1; r <= H; ++r) y = y + packed[r * ns * es];
-    } else {
-      const int qq = q <= H ? q : R - q;
-      T cre = x0.re, cim = x0.im, sre = 0, sim = 0;
-      int root = 0;
-      for (int r = 1; r <= H; ++r) {
-        root += qq;
-        if (root >= R) root -= R;
-        const Cx<T> w = tw[root * unit];  // cos, -sin (forward)
-        const Cx<T> a = packed[r * ns * es], b = packed[(H + r) * ns * es];
-        cre += a.re * w.re;
-        cim += a.im * w.re;
-        const T s = INV ? -w.im : w.im;
-        sre -= b.im * s;
-        sim += b.re * s;
-      }
-      y = q <= H ? Cx<T>{cre + sre, cim + sim} : Cx<T>{cre - sre, cim - sim};
+  const int lane = threadIdx.x & 31, row = lane >> 2, quad = lane & 3;
+  const int outputs = (H + 7) / 8, groups = (butterflies + 15) / 16, warps = blockDim.x / kWarp;
+  // Slot 0 of butterfly f in either buffer.
+  auto slot = [&](int f) {
+    const int j = f / count, t = f - j * count;
+    return t * line_stride + ((j / ns) * ns * R + j % ns) * es;
+  };
+  for (int item = threadIdx.x / kWarp; item < outputs * groups; item += warps) {
+    const int group = item / outputs, q = (item - group * outputs) * 8 + row + 1;  // this lane's output
+    double c[4][2] = {}, s[4][2] = {};
+    const double* column[4];  // this lane's B column (butterfly row / 2, component row % 2)
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int f = min(group * 16 + u * 4 + (row >> 1), butterflies - 1);
+      column[u] = reinterpret_cast<const double*>(dst + slot(f)) + (row & 1);
     }
-    src[offset + ((j / ns) * ns * R + k + q * ns) * es] = y;
+    const long long step = 2LL * ns * es;
+    int r = quad + 1, angle = (r * q) % R;
+    const int turn = (4 * q) % R;
+    for (int k = 0; k < H; k += 4, r += 4) {
+      const bool in = r <= H && q <= H;
+      const Cx<double> w = tw[in ? angle * unit : 0];
+      const double cosine = in ? w.re : 0.0, sine = in ? -w.im : 0.0;
+      const int at = r <= H ? r : 1;
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        mma_f64(c[u], cosine, column[u][at * step]);
+        mma_f64(s[u], sine, column[u][(H + at) * step]);
+      }
+      angle += turn;
+      if (angle >= R) angle -= R;
+    }
+    if (q <= H) {
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int f = group * 16 + u * 4 + quad;  // this lane's C pair: (re, im) of butterfly f
+        if (f < butterflies) {
+          const int at = slot(f);
+          const C x0 = dst[at];
+          const C even{x0.re + c[u][0], x0.im + c[u][1]};
+          // forward: -i S = (S.im, -S.re); backward: +i S = (-S.im, S.re)
+          const C odd = INV ? C{-s[u][1], s[u][0]} : C{s[u][1], -s[u][0]};
+          src[at + q * ns * es] = even + odd;
+          src[at + (R - q) * ns * es] = even - odd;
+        }
+      }
+    }
+  }
+  for (int f = threadIdx.x; f < butterflies; f += blockDim.x) {
+    const int at = slot(f);
+    C sum = dst[at];
+    for (int r = 1; r <= H; ++r) sum = sum + dst[at + r * ns * es];
+    src[at] = sum;
   }
 }
 
-// fft_lines_pp for plans that may hold odd prime radices above 7 (general
+// fft_lines_pp for FP64 plans that may hold odd prime radices above 7 (general
 // lengths); the compiled radices run the same ping-pong stages.
-template <typename T, bool INV>
-__device__ Cx<T>* fft_lines_pp_general(Cx<T>* src, Cx<T>* dst, int count, int line_stride, int elem_stride,
-                                       const int* rows, const LinePlan& plan, const Cx<T>* tw) {
+template <bool INV>
+__device__ Cx<double>* fft_lines_pp_general(Cx<double>* src, Cx<double>* dst, int count, int line_stride,
+                                            int elem_stride, const LinePlan& plan, const Cx<double>* tw) {
+  using T = double;
   int ns = 1;
   for (int s = 0; s < plan.stages; ++s) {
     const int r = plan.radix[s];
     bool swapped = true;
     switch (r) {
-      case 2: pp_stage_flat<T, 2, INV>(src, dst, count, line_stride, elem_stride, rows, plan.n, ns, tw); break;
-      case 3: pp_stage_flat<T, 3, INV>(src, dst, count, line_stride, elem_stride, rows, plan.n, ns, tw); break;
-      case 4: pp_stage_flat<T, 4, INV>(src, dst, count, line_stride, elem_stride, rows, plan.n, ns, tw); break;
-      case 5: pp_stage_flat<T, 5, INV>(src, dst, count, line_stride, elem_stride, rows, plan.n, ns, tw); break;
-      case 7: pp_stage_flat<T, 7, INV>(src, dst, count, line_stride, elem_stride, rows, plan.n, ns, tw); break;
+      case 2: pp_stage_flat<T, 2, INV>(src, dst, count, line_stride, elem_stride, nullptr, plan.n, ns, tw); break;
+      case 3: pp_stage_flat<T, 3, INV>(src, dst, count, line_stride, elem_stride, nullptr, plan.n, ns, tw); break;
+      case 4: pp_stage_flat<T, 4, INV>(src, dst, count, line_stride, elem_stride, nullptr, plan.n, ns, tw); break;
+      case 5: pp_stage_flat<T, 5, INV>(src, dst, count, line_stride, elem_stride, nullptr, plan.n, ns, tw); break;
+      case 7: pp_stage_flat<T, 7, INV>(src, dst, count, line_stride, elem_stride, nullptr, plan.n, ns, tw); break;
       default:
-        pp_stage_prime<T, INV>(src, dst, count, line_stride, elem_stride, rows, plan.n, ns, r, tw);
+        pp_stage_prime<INV>(src, dst, count, line_stride, elem_stride, plan.n, ns, r, tw);
         swapped = false;
         break;
     }

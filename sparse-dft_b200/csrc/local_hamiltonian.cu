@@ -323,12 +323,22 @@ __global__ void __launch_bounds__(kThreads) plane_out_kernel(const Cx<T>* __rest
   }
 }
 
-// Lines along a strided axis: element e of line i at base + e*stride + i.
-// GENERAL plans may hold prime radices above 7 (general lengths).
+// The indices of an axis that a transform visits: all of them, or only
+// |i| <= m (wrapped), `active` in number.
+struct AxisBox {
+  int n, active, m;
+  __device__ int index(int i) const { return i <= m ? i : n - active + i; }
+};
+AxisBox whole_axis(int n) { return {n, n, n}; }
+AxisBox axis_box(int n, int m) { return 2 * m + 1 < n ? AxisBox{n, 2 * m + 1, m} : whole_axis(n); }
+
+// Lines along a strided axis: element e of line i at base + e*stride + i,
+// base of outer index y (batch, then the box's planes). GENERAL (FP64) plans
+// may hold prime radices above 7 (general lengths).
 template <typename T, bool INV, int TL, bool GENERAL>
 __global__ void __launch_bounds__(kThreads) fft_strided_kernel(Cx<T>* __restrict__ data, int n, long long stride,
-                                                               long long inner, long long outer_stride, LinePlan p,
-                                                               const Cx<T>* __restrict__ tw_global) {
+                                                               long long inner, long long outer_stride, AxisBox outer,
+                                                               LinePlan p, const Cx<T>* __restrict__ tw_global) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   constexpr int STRIDE = TL + 1;
   Cx<T>* tw = reinterpret_cast<Cx<T>*>(smem_raw);
@@ -336,7 +346,10 @@ __global__ void __launch_bounds__(kThreads) fft_strided_kernel(Cx<T>* __restrict
   Cx<T>* tile_b = tile_a + n * STRIDE;
   const long long i0 = static_cast<long long>(blockIdx.x) * TL;
   const int lines = static_cast<int>(min(static_cast<long long>(TL), inner - i0));
-  Cx<T>* base = data + static_cast<long long>(blockIdx.y) * outer_stride + i0;
+  const int batch = static_cast<int>(blockIdx.y) / outer.active;
+  const long long plane =
+      static_cast<long long>(batch) * outer.n + outer.index(static_cast<int>(blockIdx.y) - batch * outer.active);
+  Cx<T>* base = data + plane * outer_stride + i0;
   const int tid = threadIdx.x;
   for (int i = tid; i < n; i += blockDim.x) tw[i] = tw_global[i];
   for (int idx = tid; idx < n * TL; idx += blockDim.x) {
@@ -344,37 +357,48 @@ __global__ void __launch_bounds__(kThreads) fft_strided_kernel(Cx<T>* __restrict
     if (t < lines) tile_a[e * STRIDE + t] = base[e * stride + t];
   }
   __syncthreads();
-  const Cx<T>* done = GENERAL ? fft_lines_pp_general<T, INV>(tile_a, tile_b, lines, 1, STRIDE, nullptr, p, tw)
-                              : fft_lines_pp<T, INV>(tile_a, tile_b, lines, 1, STRIDE, nullptr, p, tw);
+  const Cx<T>* done;
+  if constexpr (GENERAL) done = fft_lines_pp_general<INV>(tile_a, tile_b, lines, 1, STRIDE, p, tw);
+  else done = fft_lines_pp<T, INV>(tile_a, tile_b, lines, 1, STRIDE, nullptr, p, tw);
   for (int idx = tid; idx < n * TL; idx += blockDim.x) {
     const int e = idx / TL, t = idx - e * TL;
     if (t < lines) base[e * stride + t] = done[e * STRIDE + t];
   }
 }
 
-// Contiguous rows of length n (the innermost axis).
+// Contiguous rows of length n (the innermost axis): row index r runs over the
+// batch and the box's (i0, i1).
 template <typename T, bool INV, int TR, bool GENERAL>
 __global__ void __launch_bounds__(kThreads) fft_rows_kernel(Cx<T>* __restrict__ data, int n, int np, long long rows,
-                                                            LinePlan p, const Cx<T>* __restrict__ tw_global) {
+                                                            AxisBox b0, AxisBox b1, LinePlan p,
+                                                            const Cx<T>* __restrict__ tw_global) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ long long start[TR];
   Cx<T>* tw = reinterpret_cast<Cx<T>*>(smem_raw);
   Cx<T>* tile_a = tw + n;
   Cx<T>* tile_b = tile_a + TR * np;
   const long long r0 = static_cast<long long>(blockIdx.x) * TR;
   const int count = static_cast<int>(min(static_cast<long long>(TR), rows - r0));
-  Cx<T>* base = data + r0 * n;
   const int tid = threadIdx.x;
+  if (tid < count) {
+    const long long r = r0 + tid, outer = r / b1.active, batch = outer / b0.active;
+    start[tid] = ((batch * b0.n + b0.index(static_cast<int>(outer - batch * b0.active))) * b1.n +
+                  b1.index(static_cast<int>(r - outer * b1.active))) *
+                 n;
+  }
   for (int i = tid; i < n; i += blockDim.x) tw[i] = tw_global[i];
+  __syncthreads();
   for (int idx = tid; idx < count * n; idx += blockDim.x) {
     const int r = idx / n, e = idx - r * n;
-    tile_a[r * np + e] = base[idx];
+    tile_a[r * np + e] = data[start[r] + e];
   }
   __syncthreads();
-  const Cx<T>* done = GENERAL ? fft_lines_pp_general<T, INV>(tile_a, tile_b, count, np, 1, nullptr, p, tw)
-                              : fft_lines_pp<T, INV>(tile_a, tile_b, count, np, 1, nullptr, p, tw);
+  const Cx<T>* done;
+  if constexpr (GENERAL) done = fft_lines_pp_general<INV>(tile_a, tile_b, count, np, 1, p, tw);
+  else done = fft_lines_pp<T, INV>(tile_a, tile_b, count, np, 1, nullptr, p, tw);
   for (int idx = tid; idx < count * n; idx += blockDim.x) {
     const int r = idx / n, e = idx - r * n;
-    base[idx] = done[r * np + e];
+    data[start[r] + e] = done[r * np + e];
   }
 }
 
@@ -758,7 +782,7 @@ void slab_rows(const LocalArgs<T>& a, int columns, Cx<T>* slab, cudaStream_t str
     if (smem > kMaxDynamicSmem) return false;
     allow_smem(fft_rows_kernel<T, INV, TR, false>, smem);
     fft_rows_kernel<T, INV, TR, false><<<static_cast<unsigned>(ceil_div(rows, TR)), kThreads, smem, stream>>>(
-        slab, a.n2, np, rows, a.p2, a.tw2);
+        slab, a.n2, np, rows, whole_axis(columns * a.slots), whole_axis(a.n1), a.p2, a.tw2);
     SDFT_LAUNCH("fft_rows_kernel slab planes");
     return true;
   };
@@ -780,8 +804,8 @@ void slab_columns(const LocalArgs<T>& a, int columns, Cx<T>* slab, cudaStream_t 
     for (long long first = 0; first < planes; first += 65535) {
       const dim3 blocks(static_cast<unsigned>(ceil_div(a.n2, TL)),
                         static_cast<unsigned>(std::min<long long>(65535, planes - first)));
-      fft_strided_kernel<T, INV, TL, false><<<blocks, kThreads, smem, stream>>>(slab + first * a.n12, a.n1, a.n2,
-                                                                               a.n2, a.n12, a.p1, a.tw1);
+      fft_strided_kernel<T, INV, TL, false><<<blocks, kThreads, smem, stream>>>(
+          slab + first * a.n12, a.n1, a.n2, a.n2, a.n12, whole_axis(static_cast<int>(blocks.y)), a.p1, a.tw1);
       SDFT_LAUNCH("fft_strided_kernel slab planes");
     }
     return true;
@@ -845,51 +869,65 @@ void local_hamiltonian_impl(const SpherePlan& plan, const Cx<double>* x, long lo
                       stream);
 }
 
+// Backward: rows, then axis 1, then axis 0; forward: the other way round. With
+// an extent, lines that are zero before a backward transform, or that no wanted
+// mode needs in a forward one, are left out: rows outside the box's (i0, i1)
+// and planes outside its i0.
 template <typename T, bool INV, int TL, bool GENERAL>
-void fft3d_tiles(Cx<T>* grid, const int n[3], int batch, cudaStream_t stream) {
+void fft3d_tiles(Cx<T>* grid, const int n[3], int batch, const int* extent, cudaStream_t stream) {
   const long long n12 = static_cast<long long>(n[1]) * n[2];
   const long long count = n12 * n[0];
-  // axis 2: contiguous rows
-  {
+  const AxisBox b0 = extent ? axis_box(n[0], extent[0]) : whole_axis(n[0]);
+  const AxisBox b1 = extent ? axis_box(n[1], extent[1]) : whole_axis(n[1]);
+  auto rows = [&] {  // axis 2: contiguous
     const LinePlan p = make_line_plan(n[2], GENERAL);
     const int np = n[2] | 1;
     const std::size_t smem = sizeof(Cx<T>) * (n[2] + 2 * static_cast<std::size_t>(TL) * np);
     allow_smem(fft_rows_kernel<T, INV, TL, GENERAL>, smem);
-    const long long rows = count / n[2] * batch;
-    fft_rows_kernel<T, INV, TL, GENERAL><<<static_cast<unsigned>(ceil_div(rows, TL)), kThreads, smem, stream>>>(
-        grid, n[2], np, rows, p, device_twiddles<T>(n[2]));
+    const long long lines = static_cast<long long>(batch) * b0.active * b1.active;
+    fft_rows_kernel<T, INV, TL, GENERAL><<<static_cast<unsigned>(ceil_div(lines, TL)), kThreads, smem, stream>>>(
+        grid, n[2], np, lines, b0, b1, p, device_twiddles<T>(n[2]));
     SDFT_LAUNCH("fft_rows_kernel");
-  }
-  // axis 1: stride n2, n0*batch outer blocks
-  {
+  };
+  auto axis1 = [&] {  // stride n2, the box's i0 of every grid
     const LinePlan p = make_line_plan(n[1], GENERAL);
     const std::size_t smem = sizeof(Cx<T>) * (n[1] + 2 * static_cast<std::size_t>(n[1]) * (TL + 1));
     allow_smem(fft_strided_kernel<T, INV, TL, GENERAL>, smem);
-    const dim3 blocks(static_cast<unsigned>(ceil_div(n[2], TL)), static_cast<unsigned>(n[0] * batch));
-    fft_strided_kernel<T, INV, TL, GENERAL><<<blocks, kThreads, smem, stream>>>(grid, n[1], n[2], n[2], n12, p,
+    const dim3 blocks(static_cast<unsigned>(ceil_div(n[2], TL)), static_cast<unsigned>(b0.active * batch));
+    fft_strided_kernel<T, INV, TL, GENERAL><<<blocks, kThreads, smem, stream>>>(grid, n[1], n[2], n[2], n12, b0, p,
                                                                             device_twiddles<T>(n[1]));
     SDFT_LAUNCH("fft_strided_kernel axis1");
-  }
-  // axis 0: stride n1*n2
-  {
+  };
+  auto axis0 = [&] {  // stride n1*n2
     const LinePlan p = make_line_plan(n[0], GENERAL);
     const std::size_t smem = sizeof(Cx<T>) * (n[0] + 2 * static_cast<std::size_t>(n[0]) * (TL + 1));
     allow_smem(fft_strided_kernel<T, INV, TL, GENERAL>, smem);
     const dim3 blocks(static_cast<unsigned>(ceil_div(n12, TL)), static_cast<unsigned>(batch));
-    fft_strided_kernel<T, INV, TL, GENERAL><<<blocks, kThreads, smem, stream>>>(grid, n[0], n12, n12, count, p,
-                                                                            device_twiddles<T>(n[0]));
+    fft_strided_kernel<T, INV, TL, GENERAL><<<blocks, kThreads, smem, stream>>>(
+        grid, n[0], n12, n12, count, whole_axis(batch), p, device_twiddles<T>(n[0]));
     SDFT_LAUNCH("fft_strided_kernel axis0");
+  };
+  if (INV) {
+    rows();
+    axis1();
+    axis0();
+  } else {
+    axis0();
+    axis1();
+    rows();
   }
 }
 
-// Tile width: 32 lines when the widest axis fits in shared memory, else 16 or 8.
+// Tile width: the widest of 32, 16, 8 lines whose two buffers fit in shared
+// memory beside the rows kernel's table; the prime stage of general lengths
+// runs 16 lines so that two CTAs share an SM.
 template <typename T, bool INV, bool GENERAL>
-void fft3d_impl(Cx<T>* grid, const int n[3], int batch, cudaStream_t stream) {
+void fft3d_impl(Cx<T>* grid, const int n[3], int batch, const int* extent, cudaStream_t stream) {
   const std::size_t nmax = std::max({n[0], n[1], n[2]});
-  auto fits = [&](std::size_t tl) { return sizeof(Cx<T>) * (nmax + 2 * nmax * (tl + 1)) <= 227 * 1024; };
-  if (fits(32)) fft3d_tiles<T, INV, 32, GENERAL>(grid, n, batch, stream);
-  else if (fits(16)) fft3d_tiles<T, INV, 16, GENERAL>(grid, n, batch, stream);
-  else fft3d_tiles<T, INV, 8, GENERAL>(grid, n, batch, stream);
+  auto fits = [&](std::size_t tl) { return sizeof(Cx<T>) * (nmax + 2 * nmax * (tl + 1)) + 8 * tl <= 226 * 1024; };
+  if (fits(32) && !GENERAL) fft3d_tiles<T, INV, 32, GENERAL>(grid, n, batch, extent, stream);
+  else if (fits(16)) fft3d_tiles<T, INV, 16, GENERAL>(grid, n, batch, extent, stream);
+  else fft3d_tiles<T, INV, 8, GENERAL>(grid, n, batch, extent, stream);
 }
 
 }  // namespace
@@ -974,18 +1012,18 @@ void local_hamiltonian(const SpherePlan& plan, const Cx<double>* x, long long ld
   local_hamiltonian_impl<T>(plan, x, ldx, columns, potential, kinetic, y, ldy, slab, stream);
 }
 
-template <typename T>
-void fft3d(Cx<T>* grid, const int n[3], int batch, bool backward, cudaStream_t stream, bool general) {
+void fft3d(Cx<double>* grid, const int n[3], int batch, bool backward, cudaStream_t stream, bool general,
+           const int* extent) {
   const int nmax = std::max({n[0], n[1], n[2]});
   if (nmax > kMaxLine) throw InvalidArgument("3D FFT axes above 512 points are not supported");
   // Smooth lengths keep the compiled-radix kernels even when general lengths are allowed.
   general = general && !(fft_length_supported(n[0]) && fft_length_supported(n[1]) && fft_length_supported(n[2]));
   if (general) {
-    if (backward) fft3d_impl<T, true, true>(grid, n, batch, stream);
-    else fft3d_impl<T, false, true>(grid, n, batch, stream);
+    if (backward) fft3d_impl<double, true, true>(grid, n, batch, extent, stream);
+    else fft3d_impl<double, false, true>(grid, n, batch, extent, stream);
   } else {
-    if (backward) fft3d_impl<T, true, false>(grid, n, batch, stream);
-    else fft3d_impl<T, false, false>(grid, n, batch, stream);
+    if (backward) fft3d_impl<double, true, false>(grid, n, batch, extent, stream);
+    else fft3d_impl<double, false, false>(grid, n, batch, extent, stream);
   }
 }
 
@@ -1029,7 +1067,5 @@ template void local_hamiltonian<float>(const SpherePlan&, const Cx<double>*, lon
                                        const double*, Cx<double>*, long long, Cx<float>*, cudaStream_t);
 template void local_hamiltonian<double>(const SpherePlan&, const Cx<double>*, long long, int, const double*,
                                         const double*, Cx<double>*, long long, Cx<double>*, cudaStream_t);
-template void fft3d<float>(Cx<float>*, const int[3], int, bool, cudaStream_t, bool);
-template void fft3d<double>(Cx<double>*, const int[3], int, bool, cudaStream_t, bool);
 
 }  // namespace sdft_b200

@@ -340,7 +340,7 @@ LocalPotential local_potential(Context& ctx, const int span[3], std::size_t pote
   Cx<double>* dgrid = static_cast<Cx<double>*>(stream_alloc(sizeof(Cx<double>) * count, ctx.stream));
   try {
     SDFT_CUDA(cudaMemcpyAsync(dgrid, grid.data(), sizeof(Cx<double>) * count, cudaMemcpyHostToDevice, ctx.stream));
-    fft3d<double>(dgrid, out.shape, 1, true, ctx.stream);
+    fft3d(dgrid, out.shape, 1, true, ctx.stream);
     SDFT_CUDA(cudaMemcpyAsync(grid.data(), dgrid, sizeof(Cx<double>) * count, cudaMemcpyDeviceToHost, ctx.stream));
     SDFT_CUDA(cudaStreamSynchronize(ctx.stream));
   } catch (...) {

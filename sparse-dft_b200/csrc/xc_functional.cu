@@ -651,7 +651,7 @@ void density_functionals(Context& ctx, const FunctionalSupport& s, std::int32_t*
   const unsigned key_blocks = static_cast<unsigned>(std::min<long long>(ceil_div(count, kKeyThreads), 148LL * 8));
   xc_scatter_kernel<<<key_blocks, kKeyThreads, 0, ctx.stream>>>(keys, count, grids, points, s.with_core);
   SDFT_LAUNCH("xc_scatter_kernel");
-  fft3d<double>(grids, s.shape, grids_used, true, ctx.stream, true);
+  fft3d(grids, s.shape, grids_used, true, ctx.stream, true, s.extent);
 
   const long long tiles = ceil_div(points, static_cast<long long>(kTile));
   const std::size_t tile_bytes = sizeof(double) * tiles * (2 * kSums + 1) + sizeof(unsigned long long) * tiles;
@@ -667,7 +667,7 @@ void density_functionals(Context& ctx, const FunctionalSupport& s, std::int32_t*
   const unsigned point_blocks = static_cast<unsigned>(std::min<long long>(tiles, 148LL * 4));
   xc_points_kernel<<<point_blocks, kTileThreads, 0, ctx.stream>>>(grids, points, s.with_core, tiles, tile_out);
   SDFT_LAUNCH("xc_points_kernel");
-  fft3d<double>(grids, s.shape, 2, false, ctx.stream, true);
+  fft3d(grids, s.shape, 2, false, ctx.stream, true, s.extent);
 
   auto* out = static_cast<Cx<double>*>(ctx.staging_out.reserve(sizeof(Cx<double>) * 2 * n));
   xc_gather_kernel<<<key_blocks, kKeyThreads, 0, ctx.stream>>>(keys, count, grids, points, out, out + n);
@@ -986,7 +986,7 @@ void collinear_functionals(Context& ctx, const FunctionalSupport& s, std::int32_
   const unsigned key_blocks = static_cast<unsigned>(std::min<long long>(ceil_div(count, kKeyThreads), 148LL * 8));
   spin_scatter_kernel<<<key_blocks, kKeyThreads, 0, ctx.stream>>>(keys, down, count, grids, points);
   SDFT_LAUNCH("spin_scatter_kernel");
-  fft3d<double>(grids, s.shape, 4, true, ctx.stream, true);
+  fft3d(grids, s.shape, 4, true, ctx.stream, true, s.extent);
 
   const long long tiles = ceil_div(points, static_cast<long long>(kTile));
   const std::size_t tile_bytes = sizeof(double) * tiles * (2 * kSpinSums + 2) + sizeof(unsigned long long) * tiles * 2;
@@ -1006,7 +1006,7 @@ void collinear_functionals(Context& ctx, const FunctionalSupport& s, std::int32_
   const unsigned point_blocks = static_cast<unsigned>(std::min<long long>(tiles, 148LL * 4));
   spin_points_kernel<<<point_blocks, kTileThreads, 0, ctx.stream>>>(grids, points, tiles, tile_out, flag_word);
   SDFT_LAUNCH("spin_points_kernel");
-  fft3d<double>(grids, s.shape, 4, false, ctx.stream, true);
+  fft3d(grids, s.shape, 4, false, ctx.stream, true, s.extent);
 
   auto* out = static_cast<Cx<double>*>(ctx.staging_out.reserve(sizeof(Cx<double>) * 4 * n));
   spin_gather_kernel<<<key_blocks, kKeyThreads, 0, ctx.stream>>>(keys, down, count, grids, points, out, out + 2 * n);

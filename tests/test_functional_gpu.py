@@ -108,3 +108,26 @@ def test_fast_grid_and_padding_match_oracle(context):
         assert d["grid"] == o["grid"], (padding, fast)
         assert abs(d["xc_energy"] - o["xc_energy"]) <= 1e-12 * abs(o["xc_energy"])
         assert relative_error(d["potential"], o["potential"]) < 1e-11
+
+
+@pytest.mark.parametrize("box,padding", [((5, 63, 3), 1), ((8, 5, 11), 1), ((125, 1, 6), 1), ((6, 5, 8), 2)],
+                         ids=lambda v: "x".join(map(str, v)) if isinstance(v, tuple) else f"p{v}")
+def test_functional_on_prime_grids(context, box, padding):
+    """Axes of 11, 127, 7 / 17, 11, 23 / 251, 3, 13 points and of twice a prime (26, 22, 34): prime stages whose
+    half-length is not a multiple of the matrix instruction's tiles, lines that fill no tile of 16, and boxes as
+    wide as the grid (padding 1: every line is visited) or half of it. At the module's bars."""
+    rng = np.random.Generator(np.random.PCG64(sum(box)))
+    lattice = np.diag([9.0, 10.0, 11.0])
+    keys = np.unique(np.concatenate([np.concatenate([k, -k]) for k in (
+        rng.integers(-np.array(box), np.array(box) + 1, size=(60, 3)), np.diag(box))] + [np.zeros((1, 3), int)]), axis=0)
+    values = 1e-4 * (rng.standard_normal(len(keys)) + 1j * rng.standard_normal(len(keys)))
+    values = 0.5 * (values + np.conj(values[::-1]))  # sorted keys: -G mirrors G
+    values[len(keys) // 2] = 0.05
+    d = density.density_functionals(context, lattice, keys, values, quadrature_padding=padding)
+    o = sdft_oracle.density_functionals(lattice, keys, values, padding=padding)
+    assert d["grid"] == o["grid"] == tuple(padding * max(3, 2 * m + 1) for m in box)
+    assert np.array_equal(d["hkl"], o["hkl"])
+    for name in ("hartree_energy", "xc_energy", "vxc_density", "sampled_electrons"):
+        assert abs(d[name] - o[name]) <= 1e-12 * abs(o[name]), name
+    for name in ("potential", "xc_potential"):
+        assert relative_error(d[name], o[name]) < 1e-11, name
