@@ -9,17 +9,22 @@
 // and fills the compact form table F_LM(G) = 4 pi (-i)^L Y_LM(G^) I_L(|G|)
 // with the real harmonics of :116-139.
 //
+// The arrays follow the keys in lexicographic order; results go back to the
+// caller's. Phases come from per-atom tables of each axis (two complex
+// products a key and atom) instead of a sincospi of the summed argument.
+//
 // Per call: the (L,M) moments M_a = transform . rho_a (one thread per atom and
-// LM), then one thread per G sums exp(-i G.tau_a) (F(G) . M_a) / Omega over the
-// atoms in order (src/paw_compensation.cpp:508-520). Products and sums use
-// explicitly rounded operations so the device arithmetic follows the
-// reference's unfused order.
+// LM), then one thread per two G sums exp(-i G.tau_a) (F(G) . M_a) / Omega over
+// the atoms in order (src/paw_compensation.cpp:508-520). Si64, f = 8 (542 369
+// keys, 64 atoms), both directions: 781 -> 398 us a pair of calls, errors 1.3e-15
+// -> 6.9e-16; FP64 and load issue bound it.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <limits>
-#include <map>
 #include <unordered_map>
+#include <utility>
+#include <vector>
 
 #include "operator.cuh"
 #include "paw_density.cuh"
@@ -161,7 +166,8 @@ __global__ void multipoles_kernel(const Cx<double>* __restrict__ rho, const Cx<d
 // e^{-i G.tau_a} for the integer key (h, k, l): G.tau = 2 pi (h f1 + k f2 +
 // l f3) for G on the reciprocal lattice and fractional coordinates f, so the
 // phase is sincospi of -2 (h f1 + k f2 + l f3), an argument formed without
-// the 2 pi scaling and reduced exactly by sincospi.
+// the 2 pi scaling and reduced exactly by sincospi. Used where the keys span
+// too wide a box for tables.
 __device__ __forceinline__ Cx<double> atom_phase(const double* __restrict__ fractional, int a, int h, int k, int l) {
   const double x = __dadd_rn(__dadd_rn(__dmul_rn(static_cast<double>(h), __ldg(fractional + 3 * a)),
                                        __dmul_rn(static_cast<double>(k), __ldg(fractional + 3 * a + 1))),
@@ -171,108 +177,231 @@ __device__ __forceinline__ Cx<double> atom_phase(const double* __restrict__ frac
   return Cx<double>{c, s};
 }
 
-template <int LMS>
-__global__ void compensation_kernel(const int* __restrict__ keys, const double* __restrict__ form, std::size_t count,
-                                    const double* __restrict__ fractional, const Cx<double>* __restrict__ moments,
-                                    int atoms, int lms_runtime, double volume, Cx<double>* __restrict__ out) {
+// Per atom e^{-2 pi i n f} for n = -m..m of each axis, one table after the
+// other. n f is reduced with its rounding error, so an entry is exact to about
+// an ulp, where the sum h f1 + k f2 + l f3 carries the rounding of its largest term.
+struct PhaseTables {
+  const Cx<double>* entries;
+  int m[3];
+  int stride;  // entries per atom
+};
+
+__global__ void phase_tables_kernel(const double* __restrict__ fractional, int atoms, PhaseTables t,
+                                    Cx<double>* __restrict__ entries) {
+  const long long total = static_cast<long long>(atoms) * t.stride;
+  for (long long id = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; id < total;
+       id += static_cast<long long>(gridDim.x) * blockDim.x) {
+    const int a = static_cast<int>(id / t.stride);
+    int e = static_cast<int>(id - static_cast<long long>(a) * t.stride), axis = 0;
+    while (e > 2 * t.m[axis]) {
+      e -= 2 * t.m[axis] + 1;
+      ++axis;
+    }
+    const double n = e - t.m[axis], f = fractional[3 * a + axis];
+    const double product = __dmul_rn(n, f), error = fma(n, f, -product);
+    double s, c;
+    sincospi(-2.0 * (product - rint(product) + error), &s, &c);
+    entries[id] = Cx<double>{c, s};
+  }
+}
+
+// The key's phase for atom a, from the tables or directly.
+template <bool TABLES>
+__device__ __forceinline__ Cx<double> key_phase(const PhaseTables& t, const double* __restrict__ fractional, int a,
+                                                int h, int k, int l) {
+  if constexpr (TABLES) {
+    const auto* e = reinterpret_cast<const double2*>(t.entries) + static_cast<long long>(a) * t.stride;
+    const double2 x = __ldg(e + h + t.m[0]), y = __ldg(e + 2 * t.m[0] + 1 + k + t.m[1]),
+                  z = __ldg(e + 2 * (t.m[0] + t.m[1]) + 2 + l + t.m[2]);
+    const Cx<double> xy{fma(x.x, y.x, -x.y * y.y), fma(x.x, y.y, x.y * y.x)};
+    return Cx<double>{fma(xy.re, z.x, -xy.im * z.y), fma(xy.re, z.y, xy.im * z.x)};
+  } else {
+    return atom_phase(fractional, a, h, k, l);
+  }
+}
+
+// One thread per KEYS keys, kCompensationThreads apart, atoms in order; the
+// moments of an atom serve all of the thread's keys. The keys are in
+// lexicographic order (order[g]: the caller's index), so a warp's keys mostly
+// share h and k and run through l: its table reads are broadcasts and one
+// contiguous row.
+constexpr int kCompensationThreads = 128;
+
+template <int LMS, int KEYS, bool TABLES>
+__global__ void __launch_bounds__(kCompensationThreads) compensation_kernel(
+    const int* __restrict__ keys, const int* __restrict__ order, const double* __restrict__ form, std::size_t count,
+    const double* __restrict__ fractional, PhaseTables tables, const Cx<double>* __restrict__ moments, int atoms,
+    int lms_runtime, double volume, Cx<double>* __restrict__ out) {
   const int lms = LMS > 0 ? LMS : lms_runtime;
-  for (std::size_t g = blockIdx.x * static_cast<std::size_t>(blockDim.x) + threadIdx.x; g < count;
-       g += static_cast<std::size_t>(gridDim.x) * blockDim.x) {
-    const int h = keys[3 * g], k = keys[3 * g + 1], l = keys[3 * g + 2];
-    double f[LMS > 0 ? LMS : 1];
+  const std::size_t first = blockIdx.x * static_cast<std::size_t>(kCompensationThreads) * KEYS + threadIdx.x;
+  int h[KEYS], k[KEYS], l[KEYS];
+  double f[KEYS][LMS > 0 ? LMS : 1];
+  Cx<double> sum[KEYS];
+#pragma unroll
+  for (int u = 0; u < KEYS; ++u) {
+    const std::size_t g = min(first + u * kCompensationThreads, count - 1);
+    h[u] = keys[3 * g];
+    k[u] = keys[3 * g + 1];
+    l[u] = keys[3 * g + 2];
     if (LMS > 0) {
 #pragma unroll
-      for (int lm = 0; lm < (LMS > 0 ? LMS : 1); ++lm) f[lm] = form[static_cast<std::size_t>(lm) * count + g];
+      for (int lm = 0; lm < (LMS > 0 ? LMS : 1); ++lm) f[u][lm] = form[static_cast<std::size_t>(lm) * count + g];
     }
-    // Atoms in order; F.M_a by fused multiply-adds, one division by the
-    // volume per G (within the 1e-12 relative bar of the reference's
-    // per-atom division).
-    Cx<double> sum{0.0, 0.0};
-    for (int a = 0; a < atoms; ++a) {
-      Cx<double> value{0.0, 0.0};
-      const Cx<double>* m = moments + static_cast<std::size_t>(a) * lms;
-      int lm = 0;
-      for (int L = 0; lm < lms; ++L) {
-        const bool imaginary = L & 1;
-        for (int M = 0; M <= 2 * L; ++M, ++lm) {
-          const double fv = LMS > 0 ? f[lm] : form[static_cast<std::size_t>(lm) * count + g];
-          const Cx<double> mv = m[lm];
+    sum[u] = Cx<double>{0.0, 0.0};
+  }
+  // F.M_a by fused multiply-adds, one division by the volume per G (within
+  // the 1e-12 relative bar of the reference's per-atom division).
+  for (int a = 0; a < atoms; ++a) {
+    Cx<double> value[KEYS] = {};
+    const Cx<double>* m = moments + static_cast<std::size_t>(a) * lms;
+    int lm = 0;
+#pragma unroll
+    for (int L = 0; L <= 6; ++L) {
+      if (lm >= lms) break;
+#pragma unroll
+      for (int M = 0; M <= 2 * L; ++M, ++lm) {
+        const Cx<double> mv = m[lm];
+#pragma unroll
+        for (int u = 0; u < KEYS; ++u) {
+          const double fv = LMS > 0 ? f[u][LMS > 0 ? lm : 0]
+                                    : form[static_cast<std::size_t>(lm) * count +
+                                           min(first + u * kCompensationThreads, count - 1)];
           // (fv, 0) or (0, fv) times the moment.
-          if (imaginary) value = {fma(-fv, mv.im, value.re), fma(fv, mv.re, value.im)};
-          else value = {fma(fv, mv.re, value.re), fma(fv, mv.im, value.im)};
+          if (L & 1) value[u] = {fma(-fv, mv.im, value[u].re), fma(fv, mv.re, value[u].im)};
+          else value[u] = {fma(fv, mv.re, value[u].re), fma(fv, mv.im, value[u].im)};
         }
       }
-      const Cx<double> p = atom_phase(fractional, a, h, k, l);
-      sum = {fma(p.re, value.re, fma(-p.im, value.im, sum.re)), fma(p.re, value.im, fma(p.im, value.re, sum.im))};
     }
-    out[g] = Cx<double>{sum.re / volume, sum.im / volume};
+#pragma unroll
+    for (int u = 0; u < KEYS; ++u) {
+      const Cx<double> p = key_phase<TABLES>(tables, fractional, a, h[u], k[u], l[u]);
+      sum[u] = {fma(p.re, value[u].re, fma(-p.im, value[u].im, sum[u].re)),
+                fma(p.re, value[u].im, fma(p.im, value[u].re, sum[u].im))};
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < KEYS; ++u) {
+    const std::size_t g = first + u * kCompensationThreads;
+    if (g < count) out[order[g]] = Cx<double>{sum[u].re / volume, sum[u].im / volume};
   }
 }
 
-// Adjoint partial sums: CTA b adds, for every atom in order, V(-G)
-// e^{-iG.tau_a} F_LM(G) over its grid-stride share of G (F imaginary for odd
-// L), reduced over the CTA in a fixed order into partials[(b * atoms + a) * LMS + lm].
+// Adjoint partial sums of V(-G) e^{-iG.tau_a} F_LM(G) (F imaginary for odd L).
+// A CTA stages kProjectKeys keys, their form factors and V(-G) in shared memory
+// once for all atoms (reading them again per atom made the pass L2-bound: 92
+// bytes a key and atom); a warp takes ATOMS atoms at a time over its share of
+// the keys, so one reduction over lanes follows kProjectKeys / 32 keys a lane.
+// With few atoms the warps split the keys into `parts`. CTA b adds its chunks b,
+// b + grid, ... in order into slots b * parts + part: the sums' order is fixed.
 constexpr int kProjectThreads = 256;
+constexpr int kProjectKeys = 512;
 
 template <int LMS>
-__global__ void __launch_bounds__(kProjectThreads) project_partials_kernel(
-    const int* __restrict__ keys, const double* __restrict__ form, std::size_t count,
-    const double* __restrict__ fractional,
-    int atoms, const int* __restrict__ opposite, const Cx<double>* __restrict__ potential,
-    Cx<double>* __restrict__ partials) {
-  __shared__ Cx<double> red[kProjectThreads / 32][LMS];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int a = 0; a < atoms; ++a) {
-    Cx<double> acc[LMS];
+constexpr std::size_t project_smem() {
+  return kProjectKeys * (sizeof(double) * LMS + sizeof(Cx<double>) + 3 * sizeof(int));
+}
+
+// Sum over the warp of each of N values: lane i ends with value i (mod 32) of
+// each block of 32, halving the values with every exchange.
+template <int N>
+__device__ __forceinline__ void warp_totals(double (&v)[N], int lane) {
 #pragma unroll
-    for (int lm = 0; lm < LMS; ++lm) acc[lm] = Cx<double>{0.0, 0.0};
-    for (std::size_t g = blockIdx.x * static_cast<std::size_t>(blockDim.x) + threadIdx.x; g < count;
-         g += static_cast<std::size_t>(gridDim.x) * blockDim.x) {
-      const int o = opposite[g];
-      if (o < 0) continue;
-      const Cx<double> w = mul_rn(potential[o], atom_phase(fractional, a, keys[3 * g], keys[3 * g + 1], keys[3 * g + 2]));
-      int lm = 0;
+  for (int first = 0; first < N; first += 32) {
 #pragma unroll
-      for (int L = 0; L * L < LMS; ++L) {
+    for (int o = 16; o > 0; o >>= 1) {
 #pragma unroll
-        for (int M = 0; M <= 2 * L; ++M, ++lm) {
-          const double fv = form[static_cast<std::size_t>(lm) * count + g];
-          if (L & 1) acc[lm] = {acc[lm].re - w.im * fv, acc[lm].im + w.re * fv};
-          else acc[lm] = {acc[lm].re + w.re * fv, acc[lm].im + w.im * fv};
-        }
+      for (int i = 0; i < o; ++i) {
+        const bool upper = lane & o;
+        const double low = first + i < N ? v[first + i] : 0.0;
+        const double high = first + i + o < N ? v[first + i + o < N ? first + i + o : 0] : 0.0;
+        if (first + i < N) v[first + i] = (upper ? high : low) + __shfl_xor_sync(0xffffffffu, upper ? low : high, o);
       }
     }
-#pragma unroll
-    for (int lm = 0; lm < LMS; ++lm) {
-      double re = acc[lm].re, im = acc[lm].im;
-#pragma unroll
-      for (int s = 16; s > 0; s >>= 1) {
-        re += __shfl_xor_sync(0xffffffffu, re, s);
-        im += __shfl_xor_sync(0xffffffffu, im, s);
-      }
-      if (lane == 0) red[warp][lm] = Cx<double>{re, im};
-    }
-    __syncthreads();
-    if (threadIdx.x < LMS) {
-      Cx<double> sum{0.0, 0.0};
-      for (int w = 0; w < kProjectThreads / 32; ++w) sum = {sum.re + red[w][threadIdx.x].re, sum.im + red[w][threadIdx.x].im};
-      partials[(static_cast<std::size_t>(blockIdx.x) * atoms + a) * LMS + threadIdx.x] = sum;
-    }
-    __syncthreads();
   }
 }
 
-// responses[a][lm] = sum over CTAs in order; then out[a][e] = sum_lm responses * transform.
-__global__ void project_responses_kernel(const Cx<double>* __restrict__ partials, int blocks, int atoms, int lms,
+template <int LMS, int ATOMS, bool TABLES>
+__global__ void __launch_bounds__(kProjectThreads, 2) project_partials_kernel(
+    const int* __restrict__ keys, const double* __restrict__ form, std::size_t count,
+    const double* __restrict__ fractional, PhaseTables tables, int atoms, const int* __restrict__ opposite,
+    const Cx<double>* __restrict__ potential, int parts, Cx<double>* __restrict__ partials) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  Cx<double>* v = reinterpret_cast<Cx<double>*>(smem_raw);
+  double* f = reinterpret_cast<double*>(v + kProjectKeys);  // [LMS][kProjectKeys]
+  int* hkl = reinterpret_cast<int*>(f + LMS * kProjectKeys);  // [3][kProjectKeys]
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int group = warp / parts, part = warp - group * parts, groups = kProjectThreads / 32 / parts;
+  const int share = kProjectKeys / parts;
+  const std::size_t chunks = (count + kProjectKeys - 1) / kProjectKeys;
+  Cx<double>* slot = partials + (static_cast<std::size_t>(blockIdx.x) * parts + part) * atoms * LMS;
+  for (std::size_t chunk = blockIdx.x; chunk < chunks; chunk += gridDim.x) {
+    const std::size_t g0 = chunk * kProjectKeys;
+    __syncthreads();  // the previous chunk is done with
+    for (int i = tid; i < kProjectKeys; i += kProjectThreads) {
+      const std::size_t g = g0 + i;
+      const bool in = g < count;
+      const int o = in ? opposite[g] : -1;
+      v[i] = o >= 0 ? potential[o] : Cx<double>{0.0, 0.0};
+#pragma unroll
+      for (int c = 0; c < 3; ++c) hkl[c * kProjectKeys + i] = in ? keys[3 * g + c] : 0;
+#pragma unroll
+      for (int lm = 0; lm < LMS; ++lm)
+        f[lm * kProjectKeys + i] = in ? form[static_cast<std::size_t>(lm) * count + g] : 0.0;
+    }
+    __syncthreads();
+    for (int a0 = group * ATOMS; a0 < atoms; a0 += groups * ATOMS) {
+      double acc[ATOMS * LMS * 2] = {};
+      for (int i = part * share + lane; i < (part + 1) * share; i += 32) {
+        const int h = hkl[i], k = hkl[kProjectKeys + i], l = hkl[2 * kProjectKeys + i];
+        const Cx<double> vi = v[i];
+        Cx<double> w[ATOMS];
+#pragma unroll
+        for (int u = 0; u < ATOMS; ++u) {
+          const Cx<double> p = key_phase<TABLES>(tables, fractional, min(a0 + u, atoms - 1), h, k, l);
+          w[u] = Cx<double>{fma(vi.re, p.re, -vi.im * p.im), fma(vi.re, p.im, vi.im * p.re)};
+        }
+#pragma unroll
+        for (int lm = 0; lm < LMS; ++lm) {
+          const double fv = f[lm * kProjectKeys + i];
+          const bool imaginary = lm >= 1 && lm < 4 || lm >= 9;  // L = 1, 3
+#pragma unroll
+          for (int u = 0; u < ATOMS; ++u) {
+            double* s = acc + (u * LMS + lm) * 2;
+            s[0] = imaginary ? fma(-w[u].im, fv, s[0]) : fma(w[u].re, fv, s[0]);
+            s[1] = imaginary ? fma(w[u].re, fv, s[1]) : fma(w[u].im, fv, s[1]);
+          }
+        }
+      }
+      warp_totals(acc, lane);
+#pragma unroll
+      for (int first = 0; first < ATOMS * LMS * 2; first += 32) {
+        const int i = first + lane, u = i / (2 * LMS);
+        if (i < ATOMS * LMS * 2 && a0 + u < atoms) {
+          double* to = reinterpret_cast<double*>(slot + static_cast<std::size_t>(a0) * LMS) + i;
+          *to = chunk == blockIdx.x ? acc[first] : *to + acc[first];
+        }
+      }
+    }
+  }
+}
+
+// responses[a][lm] = sum over the slots in a fixed order, one warp each; then
+// out[a][e] = sum_lm responses * transform.
+__global__ void project_responses_kernel(const Cx<double>* __restrict__ partials, int slots, int atoms, int lms,
                                          Cx<double>* __restrict__ responses) {
-  const int id = blockIdx.x * blockDim.x + threadIdx.x;
+  const int id = (blockIdx.x * blockDim.x + threadIdx.x) / 32, lane = threadIdx.x & 31;
   if (id >= atoms * lms) return;
   Cx<double> sum{0.0, 0.0};
-  for (int b = 0; b < blocks; ++b) {
+  for (int b = lane; b < slots; b += 32) {
     const Cx<double> v = partials[static_cast<std::size_t>(b) * atoms * lms + id];
     sum = {sum.re + v.re, sum.im + v.im};
   }
-  responses[id] = sum;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    sum.re += __shfl_xor_sync(0xffffffffu, sum.re, o);
+    sum.im += __shfl_xor_sync(0xffffffffu, sum.im, o);
+  }
+  if (lane == 0) responses[id] = sum;
 }
 
 __global__ void project_contract_kernel(const Cx<double>* __restrict__ responses,
@@ -385,46 +514,70 @@ CompensationCharge::CompensationCharge(Context& ctx, const CompensationInput& in
   const double scale = 2.0 * kPi / signed_volume;
   const V3 b[3] = {scaled(cross(a[1], a[2]), scale), scaled(cross(a[2], a[0]), scale),
                    scaled(cross(a[0], a[1]), scale)};
+  // Keys in lexicographic order (ties in the caller's order); the arrays below
+  // follow it, order_ leads back.
+  auto packed = [](int h, int k, int l) {
+    const auto b = [](int v) { return static_cast<std::uint64_t>(static_cast<std::int64_t>(v) + (1LL << 20)) & 0x1FFFFF; };
+    return (b(h) << 42) | (b(k) << 21) | b(l);
+  };
+  std::vector<std::pair<std::uint64_t, int>> sorted(count_);
+  for (std::size_t g = 0; g < count_; ++g)
+    sorted[g] = {packed(in.keys[3 * g], in.keys[3 * g + 1], in.keys[3 * g + 2]), static_cast<int>(g)};
+  std::sort(sorted.begin(), sorted.end());
+  std::vector<int> order(count_), keys(3 * count_), opposite(count_);
   std::vector<double> q(3 * count_);
   std::vector<int> shell(count_);
-  std::map<double, int> shells;
+  std::unordered_map<double, int> shells;
   std::vector<double> radii;
-  for (std::size_t g = 0; g < count_; ++g) {
+  long long m[3] = {0, 0, 0};
+  for (std::size_t i = 0; i < count_; ++i) {
+    const std::size_t g = static_cast<std::size_t>(sorted[i].second);
+    order[i] = sorted[i].second;
+    for (int c = 0; c < 3; ++c) {
+      keys[3 * i + c] = in.keys[3 * g + c];
+      m[c] = std::max(m[c], std::llabs(in.keys[3 * g + c]));
+    }
     const V3 v = combine(b, static_cast<double>(in.keys[3 * g]), static_cast<double>(in.keys[3 * g + 1]),
                          static_cast<double>(in.keys[3 * g + 2]));
-    q[3 * g] = v.x;
-    q[3 * g + 1] = v.y;
-    q[3 * g + 2] = v.z;
+    q[3 * i] = v.x;
+    q[3 * i + 1] = v.y;
+    q[3 * i + 2] = v.z;
     const double radius = std::sqrt(dot(v, v)) * kBohrPerAngstrom;
     auto found = shells.try_emplace(radius, static_cast<int>(radii.size()));
     if (found.second) radii.push_back(radius);
-    shell[g] = found.first->second;
+    shell[i] = found.first->second;
   }
   for (std::size_t i = 0; i < 3 * atoms_; ++i)
     if (!std::isfinite(in.fractional[i])) throw InvalidArgument("nonfinite PAW compensation position");
   q_ = upload(q.data(), q.size());
-  keys_ = upload(in.keys, 3 * count_);
+  keys_ = upload(keys.data(), 3 * count_);
+  order_ = upload(order.data(), count_);
   fractional_ = upload(in.fractional, 3 * atoms_);
   transform_ = upload(reinterpret_cast<const Cx<double>*>(in.transform), static_cast<std::size_t>(lms_) * dim_ * dim_);
   SDFT_CUDA(cudaMalloc(&form_, sizeof(double) * lms_ * count_));
   SDFT_CUDA(cudaMalloc(&moments_, sizeof(Cx<double>) * lms_ * atoms_));
   SDFT_CUDA(cudaMalloc(&flags_, sizeof(unsigned int)));
-  {
-    // index of -G in the support (the adjoint samples V(-G)), -1 when absent
-    std::unordered_map<std::uint64_t, int> where;
-    where.reserve(count_ * 2);
-    auto key = [](int h, int k, int l) {
-      const auto b = [](int v) { return static_cast<std::uint64_t>(static_cast<std::int64_t>(v) + (1LL << 20)) & 0x1FFFFF; };
-      return (b(h) << 42) | (b(k) << 21) | b(l);
-    };
-    for (std::size_t g = 0; g < count_; ++g)
-      where[key(in.keys[3 * g], in.keys[3 * g + 1], in.keys[3 * g + 2])] = static_cast<int>(g);
-    std::vector<int> opposite(count_);
-    for (std::size_t g = 0; g < count_; ++g) {
-      const auto found = where.find(key(-in.keys[3 * g], -in.keys[3 * g + 1], -in.keys[3 * g + 2]));
-      opposite[g] = found == where.end() ? -1 : found->second;
-    }
-    opposite_ = upload(opposite.data(), opposite.size());
+  // The caller's index of -G (the adjoint samples V(-G)), -1 when absent, the
+  // last of repeated keys: -G walks the order backwards as G walks it forwards.
+  for (std::size_t i = 0, j = count_; i < count_; ++i) {
+    const std::uint64_t target = packed(-keys[3 * i], -keys[3 * i + 1], -keys[3 * i + 2]);
+    while (j > 0 && sorted[j - 1].first > target) --j;
+    opposite[i] = j > 0 && sorted[j - 1].first == target ? sorted[j - 1].second : -1;
+  }
+  opposite_ = upload(opposite.data(), opposite.size());
+  // Phase tables while they stay small: a support's box is far smaller than its key count.
+  constexpr long long kTableEntries = 3 * 4096, kTableBytes = 256LL << 20;
+  const long long entries = 2 * (m[0] + m[1] + m[2]) + 3;
+  if (entries <= kTableEntries &&
+      entries * static_cast<long long>(atoms_) * static_cast<long long>(sizeof(Cx<double>)) <= kTableBytes) {
+    table_stride_ = static_cast<int>(entries);
+    for (int c = 0; c < 3; ++c) extent_[c] = static_cast<int>(m[c]);
+    SDFT_CUDA(cudaMalloc(&tables_, sizeof(Cx<double>) * entries * atoms_));
+    const PhaseTables t{nullptr, {extent_[0], extent_[1], extent_[2]}, table_stride_};
+    const unsigned table_blocks =
+        static_cast<unsigned>(std::min<std::size_t>(ceil_div(static_cast<std::size_t>(entries) * atoms_, 256), 148ULL * 16));
+    phase_tables_kernel<<<table_blocks, 256, 0, ctx.stream>>>(fractional_, static_cast<int>(atoms_), t, tables_);
+    SDFT_LAUNCH("phase_tables_kernel");
   }
   int* d_shell = upload(shell.data(), shell.size());
   double* d_radii = upload(radii.data(), radii.size());
@@ -450,35 +603,46 @@ CompensationCharge::~CompensationCharge() {
   for (void* p : {static_cast<void*>(q_), static_cast<void*>(keys_), static_cast<void*>(fractional_),
                   static_cast<void*>(form_),
                   static_cast<void*>(transform_), static_cast<void*>(moments_), static_cast<void*>(flags_),
-                  static_cast<void*>(opposite_), static_cast<void*>(partials_), static_cast<void*>(responses_)})
+                  static_cast<void*>(opposite_), static_cast<void*>(order_), static_cast<void*>(tables_),
+                  static_cast<void*>(partials_), static_cast<void*>(responses_)})
     if (p) cudaFree(p);
 }
 
 void CompensationCharge::project(const Cx<double>* potential, Cx<double>* out) {
   const int atoms = static_cast<int>(atoms_), entries = static_cast<int>(dim_ * dim_);
-  const int blocks = static_cast<int>(std::min<std::size_t>(std::max<std::size_t>(1, ceil_div(count_, kProjectThreads)),
-                                                            148ULL * 4));
+  // Warps that have no atoms of their own split the keys.
+  int parts = 1;
+  while (parts < kProjectThreads / 32 && static_cast<int>(ceil_div(atoms_, 2)) * parts * 2 <= kProjectThreads / 32)
+    parts *= 2;
+  const int blocks = static_cast<int>(std::min<std::size_t>(ceil_div(count_, kProjectKeys), 148ULL * 4));
+  const int slots = blocks * parts;
   if (!partials_) {
-    SDFT_CUDA(cudaMalloc(&partials_, sizeof(Cx<double>) * static_cast<std::size_t>(148 * 4) * atoms_ * lms_));
+    SDFT_CUDA(cudaMalloc(&partials_, sizeof(Cx<double>) * static_cast<std::size_t>(slots) * atoms_ * lms_));
     SDFT_CUDA(cudaMalloc(&responses_, sizeof(Cx<double>) * atoms_ * lms_));
   }
-#define SDFT_PROJECT_CASE(N)                                                                                     \
-  case N:                                                                                                        \
-    project_partials_kernel<N><<<blocks, kProjectThreads, 0, ctx_.stream>>>(keys_, form_, count_, fractional_, \
-                                                                          atoms, opposite_, potential, partials_); \
+  const PhaseTables tables{tables_, {extent_[0], extent_[1], extent_[2]}, table_stride_};
+  auto go = [&](auto kernel, std::size_t smem) {
+    allow_dynamic_smem(kernel, smem);
+    kernel<<<blocks, kProjectThreads, smem, ctx_.stream>>>(keys_, form_, count_, fractional_, tables, atoms, opposite_,
+                                                           potential, parts, partials_);
+    SDFT_LAUNCH("project_partials_kernel");
+  };
+#define SDFT_PROJECT_CASE(N, ATOMS)                                                          \
+  case N:                                                                                    \
+    if (tables_) go(project_partials_kernel<N, ATOMS, true>, project_smem<N>());             \
+    else go(project_partials_kernel<N, ATOMS, false>, project_smem<N>());                    \
     break;
   switch (lms_) {
-    SDFT_PROJECT_CASE(1)
-    SDFT_PROJECT_CASE(4)
-    SDFT_PROJECT_CASE(9)
-    SDFT_PROJECT_CASE(16)
+    SDFT_PROJECT_CASE(1, 2)
+    SDFT_PROJECT_CASE(4, 2)
+    SDFT_PROJECT_CASE(9, 2)
+    SDFT_PROJECT_CASE(16, 1)
     default:
       throw InvalidArgument("compensation potential projection supports L_max <= 3");
   }
 #undef SDFT_PROJECT_CASE
-  SDFT_LAUNCH("project_partials_kernel");
-  project_responses_kernel<<<static_cast<unsigned>(ceil_div(atoms * lms_, 128)), 128, 0, ctx_.stream>>>(
-      partials_, blocks, atoms, lms_, responses_);
+  project_responses_kernel<<<static_cast<unsigned>(ceil_div(static_cast<std::size_t>(atoms) * lms_ * 32, 128)), 128, 0,
+                             ctx_.stream>>>(partials_, slots, atoms, lms_, responses_);
   SDFT_LAUNCH("project_responses_kernel");
   project_contract_kernel<<<static_cast<unsigned>(ceil_div(atoms * entries, 128)), 128, 0, ctx_.stream>>>(
       responses_, transform_, atoms, lms_, entries, out);
@@ -495,23 +659,25 @@ void CompensationCharge::density(const Cx<double>* onsite, Cx<double>* out) {
   multipoles_kernel<<<static_cast<unsigned>(ceil_div(atoms * lms_, 128)), 128, 0, ctx_.stream>>>(
       onsite, transform_, atoms, dim, lms_, moments_);
   SDFT_LAUNCH("multipoles_kernel");
-  const unsigned blocks = static_cast<unsigned>(std::min<std::size_t>(ceil_div(count_, 128), 148ULL * 32));
-#define SDFT_COMPENSATION_CASE(N)                                                                                \
-  case N:                                                                                                        \
-    compensation_kernel<N><<<blocks, 128, 0, ctx_.stream>>>(keys_, form_, count_, fractional_, moments_, atoms, \
-                                                            lms_, volume_, out);                                \
-    break;
+  const PhaseTables tables{tables_, {extent_[0], extent_[1], extent_[2]}, table_stride_};
+  auto go = [&](auto kernel, int keys) {
+    const unsigned blocks =
+        static_cast<unsigned>(ceil_div(count_, static_cast<std::size_t>(kCompensationThreads) * keys));
+    kernel<<<blocks, kCompensationThreads, 0, ctx_.stream>>>(keys_, order_, form_, count_, fractional_, tables,
+                                                             moments_, atoms, lms_, volume_, out);
+    SDFT_LAUNCH("compensation_kernel");
+  };
+#define SDFT_COMPENSATION_CASE(N, KEYS)                                  \
+  if (tables_) go(compensation_kernel<N, KEYS, true>, KEYS);             \
+  else go(compensation_kernel<N, KEYS, false>, KEYS);
   switch (lms_) {
-    SDFT_COMPENSATION_CASE(1)
-    SDFT_COMPENSATION_CASE(4)
-    SDFT_COMPENSATION_CASE(9)
-    SDFT_COMPENSATION_CASE(16)
-    default:
-      compensation_kernel<0><<<blocks, 128, 0, ctx_.stream>>>(keys_, form_, count_, fractional_, moments_, atoms,
-                                                              lms_, volume_, out);
+    case 1: SDFT_COMPENSATION_CASE(1, 2) break;
+    case 4: SDFT_COMPENSATION_CASE(4, 2) break;
+    case 9: SDFT_COMPENSATION_CASE(9, 2) break;
+    case 16: SDFT_COMPENSATION_CASE(16, 2) break;
+    default: SDFT_COMPENSATION_CASE(0, 1)
   }
 #undef SDFT_COMPENSATION_CASE
-  SDFT_LAUNCH("compensation_kernel");
   unsigned int host = 0;
   SDFT_CUDA(cudaMemcpyAsync(&host, flags_, sizeof(host), cudaMemcpyDeviceToHost, ctx_.stream));
   SDFT_CUDA(cudaStreamSynchronize(ctx_.stream));

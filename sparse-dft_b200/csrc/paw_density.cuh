@@ -57,23 +57,25 @@ class CompensationCharge {
   std::size_t dimension() const { return dim_; }
   int multipoles() const { return lms_; }
   Context& context() const { return ctx_; }
-  // Compact form factors, (L,M)-major: form[lm * count + g] (device).
-  const double* form() const { return form_; }
 
  private:
   Context& ctx_;
   std::size_t count_ = 0, atoms_ = 0, dim_ = 0;
   int lms_ = 0, max_l_ = 0;
   double volume_ = 0;
+  // Per key in lexicographic (h, k, l) order; order_ holds the caller's indices.
   double* q_ = nullptr;          // count x 3 cartesian G, 1/bohr
   int* keys_ = nullptr;          // count x 3 integer keys
+  int* order_ = nullptr;
   double* fractional_ = nullptr; // atoms x 3 fractional positions
   double* form_ = nullptr;       // lms x count
   Cx<double>* transform_ = nullptr;
   Cx<double>* moments_ = nullptr;  // atoms x lms
   unsigned int* flags_ = nullptr;
-  int* opposite_ = nullptr;         // index of -G in the support, or -1
-  Cx<double>* partials_ = nullptr;  // per-CTA sums of the adjoint
+  int* opposite_ = nullptr;         // caller's index of -G, or -1
+  Cx<double>* tables_ = nullptr;    // per-atom phase tables, or none (keys too far apart)
+  int table_stride_ = 0, extent_[3] = {0, 0, 0};
+  Cx<double>* partials_ = nullptr;  // per-slot sums of the adjoint
   Cx<double>* responses_ = nullptr; // atoms x lms
 };
 

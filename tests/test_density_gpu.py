@@ -310,3 +310,40 @@ def test_compensation_projection_is_the_adjoint_at_si64_f16(context):
     right = x.volume * np.sum(v_opposite * n)
     assert abs(left - right) < 1e-10 * max(abs(left), 1.0)
     charge.close()
+
+
+@pytest.mark.parametrize("atoms,max_l,count", [(1, 0, 5), (2, 1, 511), (3, 2, 513), (5, 2, 1200), (9, 3, 700),
+                                               (17, 2, 2100)])
+@pytest.mark.parametrize("far", [False, True])
+def test_compensation_small_supports_match_oracle(context, atoms, max_l, count, far):
+    """Atom counts that split the adjoint's warps between atoms and keys, every multipole table, key counts
+    around its chunks of 512, keys in random order with modes whose opposite is absent; far: one key so far
+    out that the phases come without tables. Both directions sum about atoms x 16 or count terms of a few eps;
+    the oracle's own phases carry eps times their argument, 2 pi max|h| (2e-13 at 150, 3e-11 at 20000)."""
+    from conftest import relative_error
+    from sdft_b200 import density, synthetic
+    rng = np.random.Generator(np.random.PCG64(1000 * atoms + count))
+    aug = synthetic.augmentation(max_l=max_l)
+    lattice = np.diag([10.0, 11.0, 12.0])
+    fractional = rng.uniform(0.0, 1.0, size=(atoms, 3))
+    every = np.stack(np.meshgrid(*[np.arange(-9, 10)] * 3, indexing="ij"), axis=-1).reshape(-1, 3)
+    keys = every[rng.permutation(len(every))[:count]].astype(np.int32)
+    if far:
+        keys[0] = (20000, -3, 1)
+    lms, dim = (max_l + 1) ** 2, 4
+    transform = rng.standard_normal((lms, dim * dim)) + 1j * rng.standard_normal((lms, dim * dim))
+    onsite = rng.standard_normal((atoms, dim, dim)) + 1j * rng.standard_normal((atoms, dim, dim))
+    onsite = onsite + np.conj(np.transpose(onsite, (0, 2, 1)))
+    potential = rng.standard_normal(count) + 1j * rng.standard_normal(count)
+    charge = density.CompensationCharge(context, lattice, fractional, keys, aug, transform)
+    tolerance = 3e-11 if far else 1e-12
+    try:
+        out = charge.density(onsite)
+        expected = sdft_oracle.compensation_density(lattice, fractional, keys, aug, transform, onsite)
+        assert relative_error(out, expected) < tolerance
+        projected = charge.project(potential)
+        expected = sdft_oracle.compensation_project(lattice, fractional, keys, aug, transform, potential)
+        assert np.max(np.abs(projected - expected)) <= tolerance * max(np.max(np.abs(expected)), 1e-300)
+        assert np.array_equal(charge.project(potential), projected)
+    finally:
+        charge.close()
