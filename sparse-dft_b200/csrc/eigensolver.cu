@@ -6,15 +6,12 @@
 //    the last 256 rows of larger matrices, in one 16-CTA cluster;
 //    tridiagonalize_kernel for the steps before: one cooperative launch, one
 //    CTA per SM, columns distributed cyclically and held in shared memory.
-//    Its step j needs one grid-wide barrier: after it every CTA forms
-//    w = p - tau/2 (p^H v) v from the published p and shares of p^H v,
-//    recomputes the next reflector redundantly from the published next column
-//    (plus this rank-2 update), then in one pass over its own columns applies
-//    the update and accumulates p = tau A22 v for the next reflector, and
-//    publishes p, its share of p^H v and the column after next. Exchange
-//    buffers are double-buffered by step parity. The barrier is a counting
-//    barrier with a time limit: on expiry an error word is set and every CTA
-//    returns.
+//    Its step j needs one grid-wide barrier: every CTA forms w and the next
+//    reflector's x redundantly from the published A x and head row, applies
+//    the update to its own columns, accumulates the next A x in the same pass,
+//    and publishes it with the next head row. Exchange buffers are
+//    double-buffered by step parity. The barrier is a counting barrier with a
+//    time limit: on expiry an error word is set and every CTA returns.
 // 2. bisect_kernel: one warp per wanted eigenvalue, 64-point multisection on
 //    division-free Sturm counts of the tridiagonal matrix.
 // 3. inverse_iteration_kernel: one thread per wanted eigenvalue, factors in
@@ -82,11 +79,11 @@ __device__ __forceinline__ Cx<double> cdot1(Cx<double> a, Cx<double> b) {
 }
 
 // Counting grid barrier with a time limit. Returns false (and every CTA
-// should return) when the limit expired here or the error word is set. The
-// CTA's writes (ordered before thread 0 by __syncthreads) are released by the
-// arrival; the acquire fence after the wait orders the reads that follow.
+// should return) when the limit expired here or the error word is set. Warp
+// 0's writes (ordered before thread 0 by its __syncwarp) are released by the
+// arrival; the acquire fence after the wait and the CTA barrier order the reads
+// that follow.
 __device__ bool grid_barrier(unsigned int* arrive, unsigned int* error, unsigned int target, int* ok) {
-  __syncthreads();
   if (threadIdx.x == 0) {
     asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(arrive) : "memory");
     const unsigned long long start = global_ns();
@@ -115,297 +112,272 @@ __device__ bool grid_barrier(unsigned int* arrive, unsigned int* error, unsigned
 struct TridiagArgs {
   Cx<double>* a;
   int m, grid, cpc;
-  int stop;  // reflectors formed here: m - 1 for the whole reduction, fewer when the cluster kernel takes the rest
+  int rows;  // column stride in shared memory: m rounded up to kTridiagThreads
+  int stop;  // reflectors formed here; the cluster kernel takes the trailing matrix
   double* d;
   double* e;
   Cx<double>* tau;
   Cx<double>* reflectors;  // m x m, column j holds v_j in rows j+1..m-1
-  Cx<double>* colbuf;      // 2 x m
-  Cx<double>* pbuf;        // 2 x m
-  Cx<double>* dotbuf;      // 2 x grid
+  Cx<double>* abuf;        // 2 x m: A x
+  Cx<double>* hbuf;        // 2 x m: head row
+  double* shares;          // 2 x grid: each CTA's part of x^H A x
   unsigned int* arrive;
   unsigned int* error;  // set when a barrier wait runs out; every CTA then returns
 };
 
-// Reflector scalars of one Householder step, formed redundantly by every
-// thread from the same shared inputs (so every thread holds equal values).
+// Scalars of the reflector that reduces a column with `head` and, below it, a
+// part of squared norm xnorm2 (LAPACK zlarfg): H = I - tau v v^H with v = e +
+// scale x, and the real off-diagonal beta; tau = scale = 0 where there is
+// nothing to reduce. A whole warp calls this: its two reciprocals run on two
+// lanes at once.
 struct Reflector {
   Cx<double> tau, scale;
   double beta;
-  bool trivial;
 };
 
-__device__ __forceinline__ Reflector make_reflector(Cx<double> alpha, double xnorm2) {
-  Reflector h;
-  if (xnorm2 == 0.0 && alpha.im == 0.0) {
-    h.trivial = true;
-    h.tau = Cx<double>{0.0, 0.0};
-    h.beta = alpha.re;
-    h.scale = Cx<double>{0.0, 0.0};
-  } else {
-    const double beta = -copysign(sqrt(alpha.re * alpha.re + alpha.im * alpha.im + xnorm2), alpha.re);
-    h.trivial = false;
-    h.tau = Cx<double>{(beta - alpha.re) / beta, -alpha.im / beta};
-    h.beta = beta;
-    // 1 / (alpha - beta)
-    const double dr = alpha.re - beta, di = alpha.im, den = dr * dr + di * di;
-    h.scale = Cx<double>{dr / den, -di / den};
-  }
-  return h;
+__device__ __forceinline__ Reflector make_reflector(int lane, Cx<double> head, double xnorm2) {
+  const bool trivial = xnorm2 == 0.0 && head.im == 0.0;
+  const double beta = -copysign(sqrt(head.re * head.re + head.im * head.im + xnorm2), head.re);
+  const double dr = head.re - beta;
+  const double inverse = 1.0 / ((lane & 1) ? dr * dr + head.im * head.im : beta);
+  const double inv_beta = __shfl_sync(0xffffffffu, inverse, 0), inv_den = __shfl_sync(0xffffffffu, inverse, 1);
+  if (trivial) return {{0.0, 0.0}, {0.0, 0.0}, head.re};
+  return {{-dr * inv_beta, -head.im * inv_beta}, {dr * inv_den, -head.im * inv_den}, beta};
 }
 
-// Rows r = tid + kTridiagThreads k of the reflector and rank-2 vectors live in
-// registers; own columns c = cta + G s in shared memory. Step j+1's reflector
-// is formed before step j's rank-2 update, so the update of each own column
-// and its product with the next reflector share one pass. Per step: one CTA
-// barrier for the next column's norm, one for the column products, and the
-// grid barrier.
+// Sum over the warp of each of N <= 32 values: lane i returns value i, the
+// values halving with every exchange.
+template <int N>
+__device__ __forceinline__ double warp_total(double (&v)[N], int lane) {
+  static_assert(N <= 32, "one value per lane");
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+#pragma unroll
+    for (int i = 0; i < o; ++i) {
+      if (i >= N) continue;
+      const bool upper = lane & o;
+      const double low = v[i], high = i + o < N ? v[i + o < N ? i + o : 0] : 0.0;
+      v[i] = (upper ? high : low) + __shfl_xor_sync(0xffffffffu, upper ? low : high, o);
+    }
+  }
+  return v[0];
+}
+
+// The reduction's first `stop` steps, one CTA per SM: column c = cta + G q in
+// the CTA's shared memory, rows r = tid + kTridiagThreads k per thread, whose
+// entries of v, w and x live in registers. A step is the cluster kernel's below
+// (the same vector phase, pass and publication, A x and head rows through
+// global memory) with one CTA barrier between the pass's sums and their
+// publication, and the grid barrier; the reflector's scalars are formed by the
+// last warp while the barrier is waited for, so neither their square root and
+// divisions nor a norm reduction lie on the step's chain.
+// Bound by that chain: the barrier's release, poll and L2 round trips, and the
+// pass over own columns. 5.0 us a step at orders 320 to 640, 5.8 at 1280; with
+// p and the next column published instead of A x and the head row (a second
+// CTA barrier, and the norm, the square root and the divisions behind the grid
+// barrier) 9.3, 7.3 and 8.3 us. Orders 320, 640, 1280 whole: 1.06 -> 0.79,
+// 3.25 -> 2.38, 8.91 -> 6.41 ms.
 __global__ void __launch_bounds__(kTridiagThreads, 1) tridiagonalize_kernel(TridiagArgs t) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  constexpr int R = kRowsPerThread;
-  const int m = t.m, G = t.grid, cpc = t.cpc, cta = blockIdx.x, tid = threadIdx.x;
+  constexpr int R = kRowsPerThread, SUMS = 2 * kMaxCpc + 1;
+  const int m = t.m, G = t.grid, cpc = t.cpc, LD = t.rows, cta = blockIdx.x, tid = threadIdx.x;
   const int lane = tid & 31, warp = tid >> 5;
   Cx<double>* cols = reinterpret_cast<Cx<double>*>(smem_raw);
-  Cx<double>* red = cols + static_cast<long long>(cpc) * m;  // kTridiagWarps x kMaxCpc column-product partials
-  Cx<double>* colv = red + kTridiagWarps * kMaxCpc;                  // 2 x kMaxCpc: v at own columns, by step parity
-  Cx<double>* colw = colv + 2 * kMaxCpc;                      // kMaxCpc: w at own columns
-  Cx<double>* pick = colw + kMaxCpc;                          // alpha (row jc+1), diagonal (row jc)
-  double* nrm = reinterpret_cast<double*>(pick + 2);          // kTridiagWarps norm partials
+  Cx<double>* own = cols + static_cast<long long>(cpc) * LD + 2 * kMaxCpc * warp;  // per warp: w, then v at own columns
+  Cx<double>* xown = cols + static_cast<long long>(cpc) * LD + 2 * kMaxCpc * kTridiagWarps;  // [2][kMaxCpc], by step parity
+  Cx<double>* pick = xown + 2 * kMaxCpc;  // entry below the head
+  Cx<double>* scalars = pick + 1;         // tau, scale
+  double* red = reinterpret_cast<double*>(scalars + 2);  // [kTridiagWarps][32]
   __shared__ int ok;
 
-  int slot_of_row[R];
+  for (int q = 0; q < cpc; ++q) {
+    const int c = cta + q * G;
+    for (int r = tid; r < LD; r += kTridiagThreads)
+      cols[static_cast<long long>(q) * LD + r] =
+          c < m && r < m ? t.a[r + static_cast<long long>(c) * m] : Cx<double>{0.0, 0.0};
+  }
+
+  Cx<double> x[R];
+  int slot[R];  // own column of the same index as the row, or -1
 #pragma unroll
   for (int k = 0; k < R; ++k) {
     const int r = tid + k * kTridiagThreads;
-    slot_of_row[k] = (r < m && r >= cta && (r - cta) % G == 0) ? (r - cta) / G : -1;
+    x[k] = Cx<double>{0.0, 0.0};
+    slot[k] = r < m && r >= cta && (r - cta) % G == 0 ? (r - cta) / G : -1;
   }
-  for (int s = 0; s < cpc; ++s) {
-    const int c = cta + s * G;
-    if (c < m)
-      for (int r = tid; r < m; r += kTridiagThreads) cols[static_cast<long long>(s) * m + r] = t.a[r + static_cast<long long>(c) * m];
-  }
-
-  Cx<double> v[R], w[R], vn[R], col[R];
-  Reflector cur, next;
-
-  // Reflector of column jc from col[] (rows >= jc): vn[] for rows >= jc+1,
-  // v at own columns into colv[jc & 1], and CTA 0's outputs. Contains the
-  // step's first CTA barrier (after which colw, written before it, is visible).
-  auto reflect = [&](int jc) -> Reflector {
-    double part = 0.0;
-#pragma unroll
-    for (int k = 0; k < R; ++k) {
-      const int r = tid + k * kTridiagThreads;
-      if (r < m && r >= jc + 2) part += col[k].re * col[k].re + col[k].im * col[k].im;
-      if (r == jc + 1) pick[0] = col[k];
-      if (r == jc) pick[1] = col[k];
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
-    if (lane == 0) nrm[warp] = part;
-    __syncthreads();
-    double xnorm2 = 0.0;
-#pragma unroll
-    for (int q = 0; q < kTridiagWarps; ++q) xnorm2 += nrm[q];
-    const Reflector h = make_reflector(pick[0], xnorm2);
-    if (cta == 0 && tid == 0) {
-      t.d[jc] = pick[1].re;
-      t.e[jc] = h.beta;
-      t.tau[jc] = h.tau;
-    }
-    Cx<double>* cv = colv + (jc & 1) * kMaxCpc;
-#pragma unroll
-    for (int k = 0; k < R; ++k) {
-      const int r = tid + k * kTridiagThreads;
-      Cx<double> vr{0.0, 0.0};
-      if (r == jc + 1) vr = Cx<double>{1.0, 0.0};
-      else if (r > jc + 1 && r < m && !h.trivial) vr = cmulz(col[k], h.scale);
-      vn[k] = vr;
-      if (cta == 0 && r > jc && r < m) t.reflectors[r + static_cast<long long>(jc) * m] = vr;
-      if (slot_of_row[k] >= 0) cv[slot_of_row[k]] = vr;
-    }
-    return h;
-  };
-
-  // Column products conj(A(:,c)) . vn over the CTA (acc), then p = tau A v at
-  // own columns c > jc, the CTA share of p^H v, and column jc+1 published.
-  auto publish = [&](int jc, const Reflector& h, Cx<double> (&acc)[kMaxCpc]) {
-#pragma unroll
-    for (int q = 0; q < kMaxCpc; ++q) {
-      if (q < cpc) {
-        double re = acc[q].re, im = acc[q].im;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-          re += __shfl_xor_sync(0xffffffffu, re, o);
-          im += __shfl_xor_sync(0xffffffffu, im, o);
-        }
-        if (lane == 0) red[warp * kMaxCpc + q] = Cx<double>{re, im};
-      }
-    }
-    __syncthreads();
-    if (warp == 0) {
-      Cx<double> dot{0.0, 0.0};
-      const int c = cta + lane * G;
-      if (lane < cpc && c > jc && c < m) {
-        Cx<double> s{0.0, 0.0};
-        for (int q = 0; q < kTridiagWarps; ++q) s = cadd(s, red[q * kMaxCpc + lane]);
-        const Cx<double> p = cmulz(h.tau, s);
-        t.pbuf[static_cast<long long>(jc & 1) * m + c] = p;
-        dot = cdot1(p, colv[(jc & 1) * kMaxCpc + lane]);
-      }
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        dot.re += __shfl_xor_sync(0xffffffffu, dot.re, o);
-        dot.im += __shfl_xor_sync(0xffffffffu, dot.im, o);
-      }
-      if (lane == 0) t.dotbuf[static_cast<long long>(jc & 1) * G + cta] = dot;
-    }
-    // Column jc+1 (updates 0..jc-1 applied) for step jc+1.
-    if (jc + 1 < m && (jc + 1) % G == cta) {
-      const long long slot = (jc + 1) / G;
-      Cx<double>* dst = t.colbuf + static_cast<long long>((jc + 1) & 1) * m;
-      for (int r = jc + 1 + tid; r < m; r += kTridiagThreads) dst[r] = cols[slot * m + r];
-    }
-  };
-
-  // Step 0: reflector of column 0, p_0 over own columns, column 1 published.
-#pragma unroll
-  for (int k = 0; k < R; ++k) {
-    const int r = tid + k * kTridiagThreads;
-    col[k] = r < m ? t.a[r] : Cx<double>{0.0, 0.0};
-  }
-  __syncthreads();  // own columns in shared memory
-  cur = reflect(0);
-#pragma unroll
-  for (int k = 0; k < R; ++k) v[k] = vn[k];
-  {
-    Cx<double> acc[kMaxCpc];
-#pragma unroll
-    for (int q = 0; q < kMaxCpc; ++q) {
-      acc[q] = Cx<double>{0.0, 0.0};
-      const int c = cta + q * G;
-      if (q >= cpc || c < 1 || c >= m) continue;
-      const Cx<double>* a = cols + static_cast<long long>(q) * m;
-#pragma unroll
-      for (int k = 0; k < R; ++k) {
-        const int r = tid + k * kTridiagThreads;
-        if (r >= 1 && r < m) acc[q] = cadd(acc[q], cdot1(a[r], v[k]));
-      }
-    }
-    publish(0, cur, acc);
-  }
-  if (!grid_barrier(t.arrive, t.error, static_cast<unsigned int>(G), &ok)) return;
-
-  for (int j = 0; j < m - 1; ++j) {
+  int turn = G - 1;  // j mod G: the CTA that stores reflector j
+  for (int j = -1; j < t.stop; ++j, turn = turn + 1 == G ? 0 : turn + 1) {
+    const int par = j & 1, next = par ^ 1, h = j + 1;
     const bool last = j == t.stop - 1;
-    // All of this step's global reads first (one round of L2 latency): p on
-    // own rows, column j+1, p at own columns and at row j+1, the CTA shares
-    // of p^H v (every warp sums them in the same order).
-    const double2* pb = reinterpret_cast<const double2*>(t.pbuf + static_cast<long long>(j & 1) * m);
-    const double2* cb = reinterpret_cast<const double2*>(t.colbuf + static_cast<long long>((j + 1) & 1) * m);
-    const double2* db = reinterpret_cast<const double2*>(t.dotbuf + static_cast<long long>(j & 1) * G);
-    const double2 zero2 = make_double2(0.0, 0.0);
-    double2 pq[R], cq[R], shares[kMaxShares];
+    const int first_k = h / kTridiagThreads, last_k = LD / kTridiagThreads;  // rows of a thread that are alive
+    const int first_q = last ? (h - cta + G - 1) / G : (h - cta + G) / G;     // own columns c > h (c >= h at the end)
+    Cx<double> v[R], w[R];
+    double sums[SUMS];
 #pragma unroll
-    for (int k = 0; k < R; ++k) {
-      const int r = tid + k * kTridiagThreads;
-      const bool row = r > j && r < m;
-      pq[k] = (row && !cur.trivial) ? __ldcg(pb + r) : zero2;
-      cq[k] = (row && !last) ? __ldcg(cb + r) : zero2;
-    }
-    const int own_c = cta + tid * G;
-    const bool own_w = !cur.trivial && tid < cpc && own_c > j && own_c < m;
-    const double2 pc = own_w ? __ldcg(pb + own_c) : zero2;
-    const double2 ph = cur.trivial ? zero2 : __ldcg(pb + j + 1);
-#pragma unroll
-    for (int i = 0; i < kMaxShares; ++i) {
-      const int g = lane + 32 * i;
-      shares[i] = (!cur.trivial && g < G) ? __ldcg(db + g) : zero2;
-    }
-    Cx<double> sum{0.0, 0.0};
-#pragma unroll
-    for (int i = 0; i < kMaxShares; ++i) sum = cadd(sum, Cx<double>{shares[i].x, shares[i].y});
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      sum.re += __shfl_xor_sync(0xffffffffu, sum.re, o);
-      sum.im += __shfl_xor_sync(0xffffffffu, sum.im, o);
-    }
-    const Cx<double> alpha = cmulz(Cx<double>{-0.5 * cur.tau.re, -0.5 * cur.tau.im}, sum);
-    // w = p + alpha v on own rows; w at own columns for the update; w[j+1] (v[j+1] = 1).
-#pragma unroll
-    for (int k = 0; k < R; ++k) {
-      const int r = tid + k * kTridiagThreads;
-      w[k] = (r > j && r < m && !cur.trivial) ? cadd(Cx<double>{pq[k].x, pq[k].y}, cmulz(alpha, v[k]))
-                                               : Cx<double>{0.0, 0.0};
-      col[k] = Cx<double>{cq[k].x, cq[k].y};
-    }
-    const Cx<double> head_w = cur.trivial ? Cx<double>{0.0, 0.0} : cadd(Cx<double>{ph.x, ph.y}, alpha);
-    if (own_w) colw[tid] = cadd(Cx<double>{pc.x, pc.y}, cmulz(alpha, colv[(j & 1) * kMaxCpc + tid]));
-
-    // Step j+1's reflector from column j+1 with update j applied.
-    if (!last) {
-      const Cx<double> hw = cconj(head_w);
+    for (int i = 0; i < SUMS; ++i) sums[i] = 0.0;
+    {
+      const double2* ab = reinterpret_cast<const double2*>(t.abuf + static_cast<long long>(par) * m);
+      const double2* hb = reinterpret_cast<const double2*>(t.hbuf + static_cast<long long>(par) * m);
+      const double* sb = t.shares + static_cast<long long>(par) * G;
+      // All of the step's global reads first (one round of L2 latency).
+      const double2 zero2 = make_double2(0.0, 0.0);
+      double2 aq[R], hq[R], ah = zero2, hh = zero2, ac = zero2, hc = zero2;
+      double part[kMaxShares];
+      const int c = cta + lane * G;
+      const bool mine = j >= 0 && lane < cpc && c >= h && c < m;
 #pragma unroll
       for (int k = 0; k < R; ++k) {
         const int r = tid + k * kTridiagThreads;
-        if (r > j && r < m) col[k] = csub(col[k], cadd(cmulz(v[k], hw), w[k]));
+        const bool row = j >= 0 && r >= h && r < m;
+        aq[k] = row ? __ldcg(ab + r) : zero2;
+        hq[k] = row ? __ldcg(hb + r) : zero2;
       }
-      next = reflect(j + 1);
-    } else {
-      __syncthreads();  // colw visible
+      if (j >= 0) {
+        ah = __ldcg(ab + h);
+        hh = __ldcg(hb + h);
+      }
+      if (mine) {
+        ac = __ldcg(ab + c);
+        hc = __ldcg(hb + c);
+      }
+#pragma unroll
+      for (int i = 0; i < kMaxShares; ++i) part[i] = j >= 0 && lane + 32 * i < G ? __ldcg(sb + lane + 32 * i) : 0.0;
+      Cx<double> tau{0.0, 0.0}, scale{0.0, 0.0}, head_w{0.0, 0.0};
+      double alpha = 0.0;
+      if (j >= 0) {
+        tau = scalars[0];
+        scale = scalars[1];
+        double xax = 0.0;
+#pragma unroll
+        for (int i = 0; i < kMaxShares; ++i) xax += part[i];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) xax += __shfl_xor_sync(0xffffffffu, xax, o);
+        const double vav = fma(scale.re * scale.re + scale.im * scale.im, xax,
+                               fma(2.0, scale.re * ah.x - scale.im * ah.y, hh.x));
+        alpha = (-0.5 * (tau.re * tau.re + tau.im * tau.im)) * vav;
+        head_w = cmulz(tau, cadd(Cx<double>{hh.x, -hh.y}, cmulz(scale, Cx<double>{ah.x, ah.y})));
+        head_w.re += alpha;  // v[h] = 1
+        head_w.im = -head_w.im;
+      }
+      // w and v at own columns, for this warp's pass.
+      if (lane < cpc) {
+        Cx<double> vc{0.0, 0.0}, wc{0.0, 0.0};
+        if (mine) {
+          vc = c == h ? Cx<double>{1.0, 0.0} : cmulz(scale, xown[par * kMaxCpc + lane]);
+          wc = cmulz(tau, cadd(Cx<double>{hc.x, -hc.y}, cmulz(scale, Cx<double>{ac.x, ac.y})));
+          wc.re += alpha * vc.re;
+          wc.im += alpha * vc.im;
+        }
+        own[lane] = cconj(wc);
+        own[kMaxCpc + lane] = cconj(vc);
+      }
+      __syncwarp();
+      const bool writer = turn == cta;
+#pragma unroll
+      for (int k = 0; k < R; ++k) {
+        const int r = tid + k * kTridiagThreads;
+        Cx<double> col{0.0, 0.0};
+        v[k] = w[k] = Cx<double>{0.0, 0.0};
+        if (r < m && r >= h) {
+          if (j < 0) {
+            col = t.a[r];
+          } else {
+            const Cx<double> hr{hq[k].x, -hq[k].y};
+            v[k] = r == h ? Cx<double>{1.0, 0.0} : cmulz(x[k], scale);
+            w[k] = cmulz(tau, cadd(hr, cmulz(scale, Cx<double>{aq[k].x, aq[k].y})));
+            w[k].re += alpha * v[k].re;
+            w[k].im += alpha * v[k].im;
+            col = csub(hr, cadd(cmulz(v[k], head_w), w[k]));
+            if (writer) t.reflectors[r + static_cast<long long>(j) * m] = v[k];
+          }
+          if (r == h && cta == 0 && !last) t.d[h] = col.re;
+          if (r == h + 1) pick[0] = col;
+        }
+        x[k] = r > h + 1 && r < m ? col : Cx<double>{0.0, 0.0};
+        sums[2 * kMaxCpc] += x[k].re * x[k].re + x[k].im * x[k].im;
+        if (slot[k] >= 0) xown[next * kMaxCpc + slot[k]] = x[k];
+      }
     }
 
-    // Update j on own columns c > j; p_{j+1} partial sums over rows/columns > j+1.
-    Cx<double> acc[kMaxCpc];
+    // Update j on own columns, and the products A x of the next reflector.
+    // Finished rows meet zeros of v, w and x; whole finished rows and columns
+    // are skipped.
 #pragma unroll
     for (int q = 0; q < kMaxCpc; ++q) {
-      acc[q] = Cx<double>{0.0, 0.0};
-      const int c = cta + q * G;
-      if (q >= cpc || c <= j || c >= m) continue;
-      const Cx<double> wc = cconj(colw[q]), vc = cconj(colv[(j & 1) * kMaxCpc + q]);
-      Cx<double>* a = cols + static_cast<long long>(q) * m;
-      const bool dot_column = !last && c > j + 1;
+      if (q < first_q || q >= cpc) continue;
+      const Cx<double> wc = own[q], vc = own[kMaxCpc + q];
+      Cx<double>* a = cols + static_cast<long long>(q) * LD + tid;
+      Cx<double> y[R];
 #pragma unroll
-      for (int k = 0; k < R; ++k) {
-        const int r = tid + k * kTridiagThreads;
-        if (r > j && r < m) {
-          Cx<double> x = a[r];
-          if (!cur.trivial) {
-            x = csub(x, cadd(cmulz(v[k], wc), cmulz(w[k], vc)));
-            a[r] = x;
-          }
-          if (dot_column && r > j + 1) acc[q] = cadd(acc[q], cdot1(x, vn[k]));
+      for (int k = 0; k < R; ++k)
+        if (k >= first_k && k < last_k) y[k] = a[k * kTridiagThreads];
+#pragma unroll
+      for (int k = 0; k < R; ++k)
+        if (k >= first_k && k < last_k) {
+          y[k].re = fma(-v[k].re, wc.re, fma(v[k].im, wc.im, fma(-w[k].re, vc.re, fma(w[k].im, vc.im, y[k].re))));
+          y[k].im = fma(-v[k].re, wc.im, fma(-v[k].im, wc.re, fma(-w[k].re, vc.im, fma(-w[k].im, vc.re, y[k].im))));
+          const Cx<double> p = cdot1(y[k], x[k]);
+          sums[2 * q] += p.re;
+          sums[2 * q + 1] += p.im;
         }
-      }
+#pragma unroll
+      for (int k = 0; k < R; ++k)
+        if (k >= first_k && k < last_k) a[k * kTridiagThreads] = y[k];
     }
     if (last) break;
-    publish(j + 1, next, acc);
-    if (!grid_barrier(t.arrive, t.error, static_cast<unsigned int>(G) * static_cast<unsigned int>(j + 2), &ok))
-      return;
-    cur = next;
+
+    const double total = warp_total(sums, lane);
+    if (lane < SUMS) red[warp * 32 + lane] = total;
+    __syncthreads();
+    if (warp == 0) {
+      const int c = cta + lane * G;
+      double share = 0.0;
+      if (lane < cpc && c > h && c < m) {
+        Cx<double> ax{0.0, 0.0};
 #pragma unroll
-    for (int k = 0; k < R; ++k) v[k] = vn[k];
+        for (int k = 0; k < kTridiagWarps; ++k) ax = cadd(ax, Cx<double>{red[k * 32 + 2 * lane], red[k * 32 + 2 * lane + 1]});
+        const Cx<double> xc = xown[next * kMaxCpc + lane];
+        t.abuf[static_cast<long long>(next) * m + c] = ax;
+        t.hbuf[static_cast<long long>(next) * m + c] = cols[static_cast<long long>(lane) * LD + h + 1];
+        share = ax.re * xc.re + ax.im * xc.im;
+      }
+#pragma unroll
+      for (int o = 8; o > 0; o >>= 1) share += __shfl_xor_sync(0xffffffffu, share, o);
+      if (lane == 0) t.shares[static_cast<long long>(next) * G + cta] = share;
+      __syncwarp();
+    } else if (warp == kTridiagWarps - 1) {
+      double xnorm2 = lane < kTridiagWarps ? red[lane * 32 + 2 * kMaxCpc] : 0.0;
+#pragma unroll
+      for (int o = kTridiagWarps / 2; o > 0; o >>= 1) xnorm2 += __shfl_xor_sync(0xffffffffu, xnorm2, o);
+      xnorm2 = __shfl_sync(0xffffffffu, xnorm2, 0);
+      const Reflector f = make_reflector(lane, pick[0], xnorm2);
+      if (lane == 0) {
+        scalars[0] = f.tau;
+        scalars[1] = f.scale;
+        if (cta == 0) {
+          t.e[h] = f.beta;
+          t.tau[h] = f.tau;
+        }
+      }
+    }
+    if (!grid_barrier(t.arrive, t.error, static_cast<unsigned int>(G) * static_cast<unsigned int>(j + 2), &ok)) return;
   }
   __syncthreads();
-  if (t.stop == m - 1) {
-    if ((m - 1) % G == cta && tid == 0) t.d[m - 1] = cols[static_cast<long long>((m - 1) / G) * m + m - 1].re;
-    return;
-  }
   // The trailing matrix, every update applied, for the cluster kernel.
-  for (int s = 0; s < cpc; ++s) {
-    const int c = cta + s * G;
+  for (int q = 0; q < cpc; ++q) {
+    const int c = cta + q * G;
     if (c >= t.stop && c < m)
       for (int r = t.stop + tid; r < m; r += kTridiagThreads)
-        t.a[r + static_cast<long long>(c) * m] = cols[static_cast<long long>(s) * m + r];
+        t.a[r + static_cast<long long>(c) * m] = cols[static_cast<long long>(q) * LD + r];
   }
 }
 
 // Householder reduction of a matrix of order m <= kClusterOrder by one
 // cluster of 16 CTAs: column c = rank + 16 q on CTA `rank`, held in registers
-// for the whole reduction, every exchange through distributed shared memory. The grid kernel above pays a global release, a
-// polled counter and L2 round trips per step: about 5 us whatever the order,
-// against 1.25 us at order 64, 1.3 at 128 and 1.8 at 256 here (0.5 -> 0.28 ms
-// for order 160, 4.07 -> 2.9 ms for the 640 whose last 256 rows end here). The
+// for the whole reduction, every exchange through distributed shared memory.
+// The grid kernel above pays a global release, a polled counter and L2 round
+// trips per step: about 5 us whatever the order, against 1.25 us at order 64,
+// 1.3 at 128 and 1.8 at 256 here (0.5 -> 0.28 ms for order 160 as a whole). The
 // step is bound by its serial chain of instructions, not by a pipe or memory.
 // It reduces whole matrices up to kClusterOrder and the trailing kClusterOrder
 // rows of larger ones; a solve below kClusterOrder needs no cooperative
@@ -630,22 +602,14 @@ __global__ void __cluster_dims__(kClusterCtas, 1, 1) __launch_bounds__(kClusterT
       double xnorm2 = re2 + im2;
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) xnorm2 += __shfl_xor_sync(0xffffffffu, xnorm2, o);
-      // make_reflector with its two reciprocals on two lanes at once.
-      const Cx<double> a = pick[0];
-      const bool trivial = xnorm2 == 0.0 && a.im == 0.0;
-      const double beta = -copysign(sqrt(a.re * a.re + a.im * a.im + xnorm2), a.re);
-      const double dr = a.re - beta;
-      const double inverse = 1.0 / ((lane & 1) ? dr * dr + a.im * a.im : beta);
-      const double inv_beta = __shfl_sync(0xffffffffu, inverse, 0), inv_den = __shfl_sync(0xffffffffu, inverse, 1);
+      const Reflector f = make_reflector(lane, pick[0], xnorm2);
       if (lane == 0) {
-        const Cx<double> zero{0.0, 0.0};
-        const Cx<double> th = trivial ? zero : Cx<double>{-dr * inv_beta, -a.im * inv_beta};
-        scalars[0] = th;
-        scalars[1] = trivial ? zero : Cx<double>{dr * inv_den, -a.im * inv_den};
+        scalars[0] = f.tau;
+        scalars[1] = f.scale;
         asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(barriers + 8 * next) : "memory");
         if (rank == 0) {
-          t.e[h] = trivial ? a.re : beta;
-          t.tau[h] = th;
+          t.e[h] = f.beta;
+          t.tau[h] = f.tau;
         }
       }
     } else if (warp == kShareWarp) {
@@ -817,7 +781,10 @@ __global__ void bisect_kernel(const double* __restrict__ d, const double* __rest
   // eps * max(|gl|, |gu|)), beside the relative one: eigenvalues near zero
   // stop at eps * |T| instead of running every round.
   const double atol = DBL_EPSILON * tnorm;
-  constexpr int P = 4;
+  // P points per lane trade rounds (53 bits / log2(32 P + 1)) for the length of
+  // a Sturm step's chain: 0.252 ms at order 640 with 320 values and 0.496 at
+  // 1280 with P = 2, 0.332 and 0.654 with P = 4.
+  constexpr int P = 2;
   for (int round = 0; round < 64; ++round) {
     const double width = hi - lo;
     if (width <= 2.0 * DBL_EPSILON * fmax(fabs(lo), fabs(hi)) || width <= atol || width <= pivmin) break;
@@ -1118,9 +1085,13 @@ int sm_count() {
   return count;
 }
 
+// Column stride of the grid kernel's shared memory.
+int tridiag_rows(int m) { return static_cast<int>(ceil_div(m, kTridiagThreads)) * kTridiagThreads; }
+
 std::size_t tridiag_smem(int m, int cpc) {
-  return sizeof(Cx<double>) * (static_cast<std::size_t>(cpc) * m + kTridiagWarps * kMaxCpc + 3 * kMaxCpc + 2) +
-         sizeof(double) * kTridiagWarps;
+  return sizeof(Cx<double>) *
+             (static_cast<std::size_t>(cpc) * tridiag_rows(m) + 2 * kMaxCpc * kTridiagWarps + 2 * kMaxCpc + 3) +
+         sizeof(double) * kTridiagWarps * 32;
 }
 
 constexpr std::size_t kSmemLimit = 227 * 1024;
@@ -1215,16 +1186,16 @@ void hermitian_lowest(cublasHandle_t blas, Cx<double>* a, int m, int wanted, dou
 
   // Layout of the tridiagonal workspace.
   const std::size_t mm = static_cast<std::size_t>(m);
-  const std::size_t bytes = sizeof(double) * 2 * mm + sizeof(Cx<double>) * (mm + mm * mm + 4 * mm + 2 * grid) + 256;
+  const std::size_t bytes = sizeof(double) * 2 * mm + sizeof(Cx<double>) * (mm + mm * mm + 4 * mm + grid) + 256;
   auto* base = static_cast<unsigned char*>(ws.tridiagonal.reserve(bytes));
   auto* arrive = reinterpret_cast<unsigned int*>(base);
   auto* d = reinterpret_cast<double*>(base + 256);
   double* e = d + mm;
   auto* tau = reinterpret_cast<Cx<double>*>(e + mm);
   Cx<double>* reflectors = tau + mm;
-  Cx<double>* colbuf = reflectors + mm * mm;
-  Cx<double>* pbuf = colbuf + 2 * mm;
-  Cx<double>* dotbuf = pbuf + 2 * mm;
+  Cx<double>* abuf = reflectors + mm * mm;
+  Cx<double>* hbuf = abuf + 2 * mm;
+  auto* shares = reinterpret_cast<double*>(hbuf + 2 * mm);
   unsigned int* error_word = arrive + 1;
   SDFT_CUDA(cudaMemsetAsync(arrive, 0, 2 * sizeof(unsigned int), stream));
   // Entries above each reflector's unit element stay zero for the block products.
@@ -1245,7 +1216,8 @@ void hermitian_lowest(cublasHandle_t blas, Cx<double>* a, int m, int wanted, dou
   mark(0);
   const int tail = std::min(m, kClusterOrder), stop = m - tail;  // the cluster kernel's order, the grid kernel's reflectors
   if (stop > 0) {
-    TridiagArgs t{a, m, grid, cpc, stop, d, e, tau, reflectors, colbuf, pbuf, dotbuf, arrive, error_word};
+    TridiagArgs t{a, m, grid, cpc, tridiag_rows(m), stop, d, e, tau, reflectors, abuf, hbuf, shares, arrive,
+                  error_word};
     cooperative_launch(reinterpret_cast<void*>(tridiagonalize_kernel), grid, kTridiagThreads, t, smem, stream);
   }
   const std::size_t corner = static_cast<std::size_t>(stop) * (mm + 1);

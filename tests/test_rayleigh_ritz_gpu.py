@@ -107,6 +107,15 @@ def test_tridiagonalisation_orders(context, n):
     check(context, h, s, 0)
 
 
+@pytest.mark.parametrize("n", [511, 512, 513, 769, 1025])
+def test_grid_reduction_orders(context, n):
+    """Orders around the grid kernel's 256 rows per thread slot, where a column's padding is one row, none or
+    255 rows, and odd column counts per CTA."""
+    rng = np.random.Generator(np.random.PCG64(300 + n))
+    h, s = pencil(n, rng, spectrum=spaced(n, rng))
+    check(context, h, s, n // 3)
+
+
 @pytest.mark.parametrize("n", [5, 130, 300])
 def test_tridiagonalisation_of_decoupled_blocks(context, n):
     """Columns that are already reduced (trivial reflectors) and exact zeros among coupled blocks."""
