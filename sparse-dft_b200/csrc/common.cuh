@@ -51,17 +51,22 @@ void trim_pool();
 // Largest dynamic shared memory a kernel here may take (B200 opt-in limit).
 constexpr std::size_t kMaxDynamicSmem = 227 * 1024;
 
-// Opts a kernel in to all the dynamic shared memory its static shared memory
-// leaves of kMaxDynamicSmem. The attribute is one value per kernel for the
-// whole process, so every call sets the same maximum: solvers on other
-// threads launch the same kernel with other sizes.
+// Dynamic shared memory that `kernel`'s static shared memory leaves of
+// kMaxDynamicSmem on the current device; the first call for a kernel and device
+// opts it in to all of it (device_memory.cu). The attribute is one value per
+// kernel for the whole process: solvers on other threads launch the same
+// kernel with other sizes.
+std::size_t dynamic_smem_limit(const void* kernel);
+
+// CTAs of `kernel` that the current device holds at once (asked once per
+// kernel, block size, shared memory and device).
+long long resident_blocks(const void* kernel, int threads, std::size_t smem);
+
+// Lets a kernel be launched with `bytes` of dynamic shared memory.
 template <typename Kernel>
 void allow_dynamic_smem(Kernel kernel, std::size_t bytes) {
-  cudaFuncAttributes attributes;
-  SDFT_CUDA(cudaFuncGetAttributes(&attributes, kernel));
-  const std::size_t limit = kMaxDynamicSmem - std::min(kMaxDynamicSmem, attributes.sharedSizeBytes);
-  if (bytes > limit) throw InvalidArgument("kernel tile does not fit in shared memory");
-  SDFT_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(limit)));
+  if (bytes > dynamic_smem_limit(reinterpret_cast<const void*>(kernel)))
+    throw InvalidArgument("kernel tile does not fit in shared memory");
 }
 
 // Interleaved complex in precision T (float2/double2 layout).

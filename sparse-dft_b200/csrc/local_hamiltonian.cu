@@ -411,11 +411,7 @@ void allow_smem(Kernel kernel, std::size_t bytes) {
 // CTAs of `kernel` resident on the whole device at once (persistent grids).
 template <typename Kernel>
 long long resident_ctas(Kernel kernel, int threads, std::size_t smem) {
-  int per_sm = 0, device = 0, sms = 0;
-  SDFT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem));
-  SDFT_CUDA(cudaGetDevice(&device));
-  SDFT_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
-  return static_cast<long long>(std::max(per_sm, 1)) * sms;
+  return resident_blocks(reinterpret_cast<const void*>(kernel), threads, smem);
 }
 
 // FP32 plane passes with pair-split lines (fft_pair_dif / fft_pair_dit):
