@@ -340,7 +340,7 @@ SDFT_B200_API sdft_b200_status sdft_b200_rayleigh_ritz(sdft_b200_context* contex
 enum { SDFT_B200_OP_NORMAL = 0, SDFT_B200_OP_ADJOINT = 1 };
 
 /* C(m x n, ldc) = op(A) op(B) (+ C when add), column-major complex with
- * explicit leading dimensions. FP64: FP64 arithmetic (cuBLAS ZGEMM). MIXED:
+ * explicit leading dimensions. FP64: FP64 arithmetic. MIXED:
  * BF16 split products on the tcgen05 tensor cores with FP32 accumulation (an
  * ADJOINT right operand is formed as B^H on the device first). memory applies
  * to a, b and c.

@@ -1,5 +1,6 @@
 // Complex GEMMs and small PAW block products (see gemm.cuh).
 #include <algorithm>
+#include <cstdint>
 
 #include "gemm.cuh"
 
@@ -48,11 +49,13 @@ struct CompensatedSum {
 };
 
 __global__ void block_product_kernel(const int* __restrict__ offsets, const long long* __restrict__ storage,
-                                     const Cx<double>* __restrict__ blocks, const Cx<double>* __restrict__ p,
-                                     long long ldp, int columns, Cx<double>* __restrict__ out, long long ldo) {
+                                     const Cx<double>* __restrict__ blocks, const Cx<double>* __restrict__ second,
+                                     const Cx<double>* __restrict__ p, long long ldp, int columns,
+                                     Cx<double>* __restrict__ out, long long ldo) {
   const int atom = blockIdx.x;
   const int first = offsets[atom], rows = offsets[atom + 1] - first;
-  const Cx<double>* m = blocks + storage[atom];
+  const Cx<double>* m = (blockIdx.z ? second : blocks) + storage[atom];  // z = 1: the second matrix's columns
+  out += static_cast<long long>(blockIdx.z) * columns * ldo;
   const int per_block = blockDim.x / rows;
   if (per_block == 0) return;
   const int local = threadIdx.x % rows;
@@ -140,9 +143,26 @@ unsigned grid_for(long long total, int threads) {
 
 }  // namespace
 
+// Where the library's kernel is ahead of cuBLAS (one B200; own / cuBLAS us):
+// 160 x 20 x 1000 10.3 / 12.7, 64 x 80 x 64 5.4 / 12.5, 160 x 160 x 160 8.5 /
+// 10.6, 64 x 320 x 640 12.3 / 12.8 on one side, 640^3 82 / 71 and 640 x 160 x
+// 23847 805 / 576 on the other. Long K stays with cuBLAS, which shares it
+// between more CTAs.
+bool small_product(int m, int n, int k) {
+  return k <= 4096 && static_cast<double>(m) * n * k <= 1.3e7;
+}
+
 void zgemm(cublasHandle_t handle, Op aop, Op bop, int m, int n, int k, const Cx<double>* a, long long lda,
            const Cx<double>* b, long long ldb, Cx<double>* c, long long ldc, bool add, double alpha) {
   if (m <= 0 || n <= 0 || k <= 0) return;
+  const auto aligned = [](const void* p) { return reinterpret_cast<std::uintptr_t>(p) % sizeof(Cx<double>) == 0; };
+  if (bop == Op::N && small_product(m, n, k) && aligned(a) && aligned(b) && aligned(c)) {
+    cudaStream_t stream = nullptr;
+    check_blas(cublasGetStream(handle, &stream), "cublasGetStream");
+    const ProductOutput out[2] = {product_output(c, ldc, add), {}};
+    zgemm_device(aop == Op::C, m, n, k, a, lda, b, ldb, out, n, alpha, true, stream);
+    return;
+  }
   const cuDoubleComplex one = make_cuDoubleComplex(alpha, 0.0);
   const cuDoubleComplex beta = make_cuDoubleComplex(add ? 1.0 : 0.0, 0.0);
   check_blas(cublasZgemm(handle, aop == Op::N ? CUBLAS_OP_N : CUBLAS_OP_C, bop == Op::N ? CUBLAS_OP_N : CUBLAS_OP_C,
@@ -152,17 +172,31 @@ void zgemm(cublasHandle_t handle, Op aop, Op bop, int m, int n, int k, const Cx<
              "cublasZgemm");
 }
 
-void block_product(int atoms, const int* offsets, const long long* storage, int max_block, const Cx<double>* blocks,
-                   const Cx<double>* p, long long ldp, int columns, Cx<double>* out, long long ldo,
-                   cudaStream_t stream) {
+namespace {
+void launch_block_product(int atoms, const int* offsets, const long long* storage, int max_block,
+                          const Cx<double>* blocks, const Cx<double>* second, const Cx<double>* p, long long ldp,
+                          int columns, Cx<double>* out, long long ldo, cudaStream_t stream) {
   if (atoms <= 0 || columns <= 0) return;
   if (max_block < 1 || max_block > 256) throw InvalidArgument("PAW block size out of range");
   const int threads = 256;
   const int per_block = threads / max_block;
-  const dim3 grid(atoms, static_cast<unsigned>(ceil_div(columns, per_block)));
+  const dim3 grid(atoms, static_cast<unsigned>(ceil_div(columns, per_block)), second ? 2 : 1);
   // Blocks smaller than max_block still map per_block(their size) >= per_block(max) columns per CTA.
-  block_product_kernel<<<grid, threads, 0, stream>>>(offsets, storage, blocks, p, ldp, columns, out, ldo);
+  block_product_kernel<<<grid, threads, 0, stream>>>(offsets, storage, blocks, second, p, ldp, columns, out, ldo);
   SDFT_LAUNCH("block_product_kernel");
+}
+}  // namespace
+
+void block_product(int atoms, const int* offsets, const long long* storage, int max_block, const Cx<double>* blocks,
+                   const Cx<double>* p, long long ldp, int columns, Cx<double>* out, long long ldo,
+                   cudaStream_t stream) {
+  launch_block_product(atoms, offsets, storage, max_block, blocks, nullptr, p, ldp, columns, out, ldo, stream);
+}
+
+void block_product_pair(int atoms, const int* offsets, const long long* storage, int max_block,
+                        const Cx<double>* m_blocks, const Cx<double>* n_blocks, const Cx<double>* p, long long ldp,
+                        int columns, Cx<double>* out, long long ldo, cudaStream_t stream) {
+  launch_block_product(atoms, offsets, storage, max_block, m_blocks, n_blocks, p, ldp, columns, out, ldo, stream);
 }
 
 void shifted_block_product(int atoms, const int* offsets, const long long* storage, int max_block,

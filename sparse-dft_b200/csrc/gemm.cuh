@@ -22,10 +22,31 @@ struct Scratch {
   ~Scratch() { release(); }
 };
 
-// C(m x n, ldc) = alpha op(A) B (+ C if add), all complex FP64 column-major,
-// FP64 arithmetic through cuBLAS ZGEMM (plain library GEMM).
+// C(m x n, ldc) = alpha op(A) op(B) (+ C if add), all complex FP64
+// column-major, FP64 arithmetic, on the handle's stream: the library's kernel
+// (zgemm_device) for small products with B as it lies, cuBLAS ZGEMM otherwise.
 void zgemm(cublasHandle_t handle, Op aop, Op bop, int m, int n, int k, const Cx<double>* a, long long lda,
            const Cx<double>* b, long long ldb, Cx<double>* c, long long ldc, bool add, double alpha = 1.0);
+// Where a product goes: c = prior_scale * prior + alpha op(A) B. prior may be c
+// itself or another matrix; null leaves the term out.
+struct ProductOutput {
+  Cx<double>* c = nullptr;
+  long long ldc = 0;
+  const Cx<double>* prior = nullptr;
+  long long ldp = 0;
+  double prior_scale = 1.0;
+};
+inline ProductOutput product_output(Cx<double>* c, long long ldc, bool add) {
+  return {c, ldc, add ? c : nullptr, ldc, 1.0};
+}
+
+// The library's own kernel (zgemm.cu): op(A) = A or A^H. The product's columns
+// go to out[0] from column 0 and to out[1] from column `second` (n for one
+// output). share_k = false keeps K whole, so that a column's sums do not depend
+// on the width of the product it is part of.
+void zgemm_device(bool adjoint, int m, int n, int k, const Cx<double>* a, long long lda, const Cx<double>* b,
+                  long long ldb, const ProductOutput out[2], int second, double alpha, bool share_k,
+                  cudaStream_t stream);
 
 // Per-atom block-diagonal product out[off_a + i, c] = sum_j M_a(i,j) P[off_a + j, c]
 // with error-free FP64 products and compensated sums (TwoSum + FMA), the
@@ -34,6 +55,11 @@ void zgemm(cublasHandle_t handle, Op aop, Op bop, int m, int n, int k, const Cx<
 void block_product(int atoms, const int* offsets, const long long* storage, int max_block, const Cx<double>* blocks,
                    const Cx<double>* p, long long ldp, int columns, Cx<double>* out, long long ldo,
                    cudaStream_t stream);
+
+// Both of out(:, c) = M_a P(:, c) and out(:, columns + c) = N_a P(:, c), each as block_product.
+void block_product_pair(int atoms, const int* offsets, const long long* storage, int max_block,
+                        const Cx<double>* m_blocks, const Cx<double>* n_blocks, const Cx<double>* p, long long ldp,
+                        int columns, Cx<double>* out, long long ldo, cudaStream_t stream);
 
 // out(:, c) = (M_a - shift[c] N_a) P(:, c) per atom block (shift on the
 // device), both products compensated as in block_product.

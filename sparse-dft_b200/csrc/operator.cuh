@@ -262,8 +262,12 @@ class DeviceOperator {
                      const std::vector<Cx<double>>& q_blocks, const std::vector<int>& offsets,
                      const std::vector<long long>& storage);
   void local_part(const Cx<double>* x, int columns, Cx<double>* y, Precision precision);
-  void paw_add(const Cx<double>* p, int columns, bool overlap, Cx<double>* y, Precision precision);
-  void backproject(const Cx<double>* dp, int columns, Cx<double>* y, Precision precision);
+  void paw_add(const Cx<double>* p, int columns, bool overlap, Cx<double>* y, const Cx<double>* prior,
+               double prior_scale, Precision precision);
+  bool own_backprojection(Precision precision) const;
+  void backproject(const Cx<double>* dp, int columns, const ProductOutput out[2], int second, Precision precision);
+  void add_backprojection(const Cx<double>* dp, int columns, Cx<double>* y, const Cx<double>* prior,
+                          double prior_scale, Precision precision);
 
   Context& ctx_;
   int npw_ = 0, np_ = 0, atoms_ = 0, max_block_ = 0;

@@ -114,13 +114,13 @@ __host__ __device__ constexpr int stages() {
 struct EpilogueArgs {
   int m, n2;                   // rows, real columns (2 x complex columns)
   Cx<float>* partial;          // split-K output [split][n2/2][m] or null
-  Cx<double>* c;               // direct output (when partial is null)
-  long long ldc;
+  ProductOutput out[2];        // direct outputs (when partial is null)
+  int second;                  // first complex column of out[1]
   double alpha;
-  int add;
 };
 
-template <int BN>
+// PAIR: the product's columns go to two outputs.
+template <int BN, bool PAIR>
 __global__ void __launch_bounds__(kThreads, 1)
     umma_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                      int k_blocks_total, int k_blocks_per_split, EpilogueArgs ep) {
@@ -195,15 +195,17 @@ __global__ void __launch_bounds__(kThreads, 1)
   const int row = tile_m + warp * 32 + lane;
   const int n_complex_total = ep.n2 / 2;
   for (int c0 = 0; c0 < BN; c0 += 16) {
-    // The chunk's earlier C values (accumulating products) are requested
-    // before the accumulator read, all eight at once.
+    // The chunk's prior values (accumulating products) are requested before
+    // the accumulator read, all eight at once.
     Cx<double> prior[8];
-    const bool accumulate = !ep.partial && ep.add && row < ep.m;
 #pragma unroll
     for (int q = 0; q < 8; ++q) {
       const int j = (tile_n + c0) / 2 + q;
-      prior[q] = (accumulate && j < n_complex_total) ? ep.c[row + static_cast<long long>(j) * ep.ldc]
-                                                     : Cx<double>{0.0, 0.0};
+      const bool other = PAIR && j >= ep.second;
+      const ProductOutput& o = ep.out[other ? 1 : 0];
+      prior[q] = !ep.partial && o.prior && row < ep.m && j < n_complex_total
+                     ? o.prior[row + static_cast<long long>(other ? j - ep.second : j) * o.ldp]
+                     : Cx<double>{0.0, 0.0};
     }
     std::uint32_t r[16];
     if (have) {
@@ -227,12 +229,12 @@ __global__ void __launch_bounds__(kThreads, 1)
         if (ep.partial) {
           ep.partial[(static_cast<long long>(blockIdx.z) * n_complex_total + j) * ep.m + row] = Cx<float>{re, im};
         } else {
-          double vr = ep.alpha * static_cast<double>(re), vi = ep.alpha * static_cast<double>(im);
-          if (ep.add) {
-            vr += prior[q].re;
-            vi += prior[q].im;
-          }
-          ep.c[row + static_cast<long long>(j) * ep.ldc] = Cx<double>{vr, vi};
+          const bool other = PAIR && j >= ep.second;
+          const ProductOutput& o = ep.out[other ? 1 : 0];
+          const double vr = ep.alpha * static_cast<double>(re), vi = ep.alpha * static_cast<double>(im);
+          o.c[row + static_cast<long long>(other ? j - ep.second : j) * o.ldc] =
+              Cx<double>{__dadd_rn(vr, __dmul_rn(o.prior_scale, prior[q].re)),
+                         __dadd_rn(vi, __dmul_rn(o.prior_scale, prior[q].im))};
         }
       }
     }
@@ -246,10 +248,10 @@ __global__ void __launch_bounds__(kThreads, 1)
   if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS));
 }
 
-// C = alpha * sum_s partial[s] (+ C): one thread per (row i = x, column j = y),
+// alpha * sum_s partial[s] to its output: one thread per (row i = x, column j = y),
 // the splits summed in order with two interleaved accumulators.
 __global__ void reduce_splits_kernel(int m, int n, int splits, const Cx<float>* __restrict__ partial,
-                                     Cx<double>* __restrict__ c, long long ldc, bool add, double alpha) {
+                                     ProductOutput out0, ProductOutput out1, int second, double alpha) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= m) return;
   const long long total = static_cast<long long>(m) * n;
@@ -270,12 +272,14 @@ __global__ void reduce_splits_kernel(int m, int n, int splits, const Cx<float>* 
       im0 += a.im;
     }
     double re = (re0 + re1) * alpha, im = (im0 + im1) * alpha;
-    Cx<double>& out = c[i + static_cast<long long>(j) * ldc];
-    if (add) {
-      re += out.re;
-      im += out.im;
+    const ProductOutput& o = j >= second ? out1 : out0;
+    const long long column = j >= second ? j - second : j;
+    if (o.prior) {
+      const Cx<double> v = o.prior[i + column * o.ldp];
+      re = __dadd_rn(re, __dmul_rn(o.prior_scale, v.re));
+      im = __dadd_rn(im, __dmul_rn(o.prior_scale, v.im));
     }
-    out = Cx<double>{re, im};
+    o.c[i + column * o.ldc] = Cx<double>{re, im};
   }
 }
 
@@ -459,12 +463,13 @@ void launch(const std::uint16_t* a, long long lda, const std::uint16_t* b, long 
             long long kexp, const EpilogueArgs& ep_in, int splits, int k_blocks, int kpb, cudaStream_t stream) {
   constexpr int S = stages<BN>();
   const std::size_t smem = static_cast<std::size_t>(S) * (BM * BK * 2 + BN * BK * 2) + 1024 + 256;
-  allow_dynamic_smem(umma_gemm_kernel<BN>, smem);
+  const auto kernel = ep_in.second < n2 / 2 && !ep_in.partial ? umma_gemm_kernel<BN, true> : umma_gemm_kernel<BN, false>;
+  allow_dynamic_smem(kernel, smem);
   const CUtensorMap map_a = kmajor_map(a, m, kexp, lda, BM);
   const CUtensorMap map_b = kmajor_map(b, n2, kexp, ldb, BN);
   if (ceil_div(m, BM) > 65535) throw InvalidArgument("tensor-core GEMM has more than 65535 row tiles");
   const dim3 grid(static_cast<unsigned>(ceil_div(n2, BN)), static_cast<unsigned>(ceil_div(m, BM)), splits);
-  umma_gemm_kernel<BN><<<grid, kThreads, smem, stream>>>(map_a, map_b, k_blocks, kpb, ep_in);
+  kernel<<<grid, kThreads, smem, stream>>>(map_a, map_b, k_blocks, kpb, ep_in);
   SDFT_LAUNCH("umma_gemm_kernel");
 }
 
@@ -569,13 +574,13 @@ int model_splits(int m, int n2, int k_blocks, int bn) {
 
 // One product with the given tile width and split count.
 void run_config(const std::uint16_t* a, long long lda, const std::uint16_t* b, long long ldb, int m, int n,
-                long long kexp, Cx<double>* c, long long ldc, bool add, double alpha, int bn, int splits,
+                long long kexp, const ProductOutput out[2], int second, double alpha, int bn, int splits,
                 Scratch& workspace, cudaStream_t stream) {
   const int n2 = 2 * n;
   const int k_blocks = static_cast<int>(kexp / BK);
   const int kpb = static_cast<int>(ceil_div(k_blocks, splits));
   splits = static_cast<int>(ceil_div(k_blocks, kpb));
-  EpilogueArgs ep{m, n2, nullptr, c, ldc, alpha, add ? 1 : 0};
+  EpilogueArgs ep{m, n2, nullptr, {out[0], out[1]}, second, alpha};
   if (splits > 1)
     ep.partial = static_cast<Cx<float>*>(workspace.reserve(sizeof(Cx<float>) * static_cast<std::size_t>(m) * n * splits));
   if (bn == 256) launch<256>(a, lda, b, ldb, m, n2, kexp, ep, splits, k_blocks, kpb, stream);
@@ -584,7 +589,7 @@ void run_config(const std::uint16_t* a, long long lda, const std::uint16_t* b, l
   if (splits > 1) {
     reduce_splits_kernel<<<dim3(static_cast<unsigned>(ceil_div(m, 256)), static_cast<unsigned>(std::min(n, kMaxGridY))),
                            256, 0, stream>>>(
-        m, n, splits, ep.partial, c, ldc, add, alpha);
+        m, n, splits, ep.partial, out[0], out[1], second, alpha);
     SDFT_LAUNCH("reduce_splits_kernel");
   }
 }
@@ -602,8 +607,10 @@ void run_config(const std::uint16_t* a, long long lda, const std::uint16_t* b, l
 // summation order. SDFT_B200_GEMM_AUTOTUNE=0 uses the cost model alone.
 struct ShapeClass {
   int row_tiles, column_units, k_blocks;
+  bool share_k;  // whether K may be split
   bool operator<(const ShapeClass& o) const {
-    return std::tie(row_tiles, column_units, k_blocks) < std::tie(o.row_tiles, o.column_units, o.k_blocks);
+    return std::tie(row_tiles, column_units, k_blocks, share_k) <
+           std::tie(o.row_tiles, o.column_units, o.k_blocks, o.share_k);
   }
 };
 struct TileChoice {
@@ -624,19 +631,20 @@ bool autotune_enabled() {
 }
 
 TileChoice tuned_choice(const std::uint16_t* a, long long lda, const std::uint16_t* b, long long ldb, int m, int n,
-                        long long kexp, Scratch& workspace, cudaStream_t stream) {
+                        long long kexp, bool share_k, cudaStream_t stream) {
   const int n2 = 2 * n;
   const int k_blocks = static_cast<int>(kexp / BK);
   int k_class = 1;
   for (int j = 1; k_class < k_blocks; ++j) k_class = static_cast<int>(std::ceil(std::exp2(j / 8.0)));
-  const ShapeClass key{static_cast<int>(ceil_div(m, BM)), static_cast<int>(ceil_div(n2, 32)), k_class};
+  const ShapeClass key{static_cast<int>(ceil_div(m, BM)), static_cast<int>(ceil_div(n2, 32)), k_class,
+                       share_k};
   std::lock_guard<std::mutex> lock(g_tune_mutex);
   auto found = g_tuned.find(key);
   if (found != g_tuned.end()) return found->second;
   std::vector<std::pair<int, int>> candidates;
   for (int bn : {128, 160, 256}) {
-    const int s = model_splits(m, n2, k_blocks, bn);
-    for (int split : {1, s, std::min(max_splits_for(k_blocks), 2 * s)})
+    const int s = share_k ? model_splits(m, n2, k_blocks, bn) : 1;
+    for (int split : {1, s, share_k ? std::min(max_splits_for(k_blocks), 2 * s) : 1})
       if (std::find(candidates.begin(), candidates.end(), std::make_pair(bn, split)) == candidates.end())
         candidates.emplace_back(bn, split);
   }
@@ -646,12 +654,13 @@ TileChoice tuned_choice(const std::uint16_t* a, long long lda, const std::uint16
   SDFT_CUDA(cudaEventCreate(&start));
   SDFT_CUDA(cudaEventCreate(&stop));
   TileChoice best{model_width(n2), 0, -1.0f};
-  best.splits = model_splits(m, n2, k_blocks, best.bn);
+  best.splits = share_k ? model_splits(m, n2, k_blocks, best.bn) : 1;
+  const ProductOutput scratch[2] = {product_output(c, m, false), {}};
   try {
     for (const auto& [bn, splits] : candidates) {
-      run_config(a, lda, b, ldb, m, n, kexp, c, m, false, 1.0, bn, splits, partials, stream);
+      run_config(a, lda, b, ldb, m, n, kexp, scratch, n, 1.0, bn, splits, partials, stream);
       SDFT_CUDA(cudaEventRecord(start, stream));
-      run_config(a, lda, b, ldb, m, n, kexp, c, m, false, 1.0, bn, splits, partials, stream);
+      run_config(a, lda, b, ldb, m, n, kexp, scratch, n, 1.0, bn, splits, partials, stream);
       SDFT_CUDA(cudaEventRecord(stop, stream));
       SDFT_CUDA(cudaEventSynchronize(stop));
       float ms = 0;
@@ -671,21 +680,30 @@ TileChoice tuned_choice(const std::uint16_t* a, long long lda, const std::uint16
 
 }  // namespace
 
-void umma_complex_gemm(const std::uint16_t* a, long long lda, const std::uint16_t* b, long long ldb, int m, int n,
-                       long long kexp, Cx<double>* c, long long ldc, bool add, double alpha, Scratch& workspace,
-                       cudaStream_t stream) {
+namespace {
+void product(const std::uint16_t* a, long long lda, const std::uint16_t* b, long long ldb, int m, int n,
+             long long kexp, const ProductOutput out[2], int second, double alpha, bool share_k, Scratch& workspace,
+             cudaStream_t stream) {
   if (m <= 0 || n <= 0 || kexp <= 0) return;
   if (kexp % BK != 0) throw InvalidArgument("expanded K must be a multiple of 64");
   int bn, splits;
   if (autotune_enabled()) {
-    const TileChoice choice = tuned_choice(a, lda, b, ldb, m, n, kexp, workspace, stream);
+    const TileChoice choice = tuned_choice(a, lda, b, ldb, m, n, kexp, share_k, stream);
     bn = choice.bn;
     splits = choice.splits;
   } else {
     bn = model_width(2 * n);
-    splits = model_splits(m, 2 * n, static_cast<int>(kexp / BK), bn);
+    splits = share_k ? model_splits(m, 2 * n, static_cast<int>(kexp / BK), bn) : 1;
   }
-  run_config(a, lda, b, ldb, m, n, kexp, c, ldc, add, alpha, bn, splits, workspace, stream);
+  run_config(a, lda, b, ldb, m, n, kexp, out, second, alpha, bn, splits, workspace, stream);
+}
+}  // namespace
+
+void umma_complex_gemm(const std::uint16_t* a, long long lda, const std::uint16_t* b, long long ldb, int m, int n,
+                       long long kexp, Cx<double>* c, long long ldc, bool add, double alpha, Scratch& workspace,
+                       cudaStream_t stream) {
+  const ProductOutput out[2] = {product_output(c, ldc, add), {}};
+  product(a, lda, b, ldb, m, n, kexp, out, n, alpha, true, workspace, stream);
 }
 
 std::size_t gemm_tuned_classes(std::size_t capacity, int* rows) {
@@ -753,6 +771,15 @@ void gemm_tc(Op aop, int m, int n, int k, const Cx<double>* a, long long lda, co
   auto* pb = static_cast<std::uint16_t*>(ws.b.reserve(sizeof(std::uint16_t) * static_cast<std::size_t>(kexp) * 2 * n));
   pack_b(b, ldb, k, n, split, pb, kexp, stream);
   umma_complex_gemm(pa, lda_p, pb, kexp, m, n, kexp, c, ldc, add, alpha, ws.partial, stream);
+}
+
+void gemm_tc_packed(const PackedA& packed, int n, const Cx<double>* b, long long ldb, const ProductOutput out[2],
+                    int second, TensorCoreWorkspace& ws, cudaStream_t stream) {
+  if (packed.rows <= 0 || n <= 0 || packed.k <= 0) return;
+  const long long kexp = expanded_k(packed.k, packed.split);
+  auto* pb = static_cast<std::uint16_t*>(ws.b.reserve(sizeof(std::uint16_t) * static_cast<std::size_t>(kexp) * 2 * n));
+  pack_b(b, ldb, packed.k, n, packed.split, pb, kexp, stream);
+  product(packed.data, packed.ld, pb, kexp, packed.rows, n, kexp, out, second, 1.0, false, ws.partial, stream);
 }
 
 unsigned int umma_error_flag() {

@@ -94,6 +94,11 @@ void gemm_tc(Op aop, int m, int n, int k, const Cx<double>* a, long long lda, co
              const Cx<double>* b, long long ldb, Cx<double>* c, long long ldc, bool add, double alpha, Split split,
              TensorCoreWorkspace& ws, cudaStream_t stream);
 
+// op(A) B of a packed A (K whole: a column's sums do not depend on n), columns
+// below `second` to out[0], the others to out[1].
+void gemm_tc_packed(const PackedA& packed, int n, const Cx<double>* b, long long ldb, const ProductOutput out[2],
+                    int second, TensorCoreWorkspace& ws, cudaStream_t stream);
+
 // Reads the device word set when a tensor-core kernel's bounded wait ran out
 // (0 = no failure). The word is never cleared: concurrent solvers share it,
 // and after a failure every later tensor-core product winds down and reports

@@ -151,3 +151,18 @@ def test_autotuner_records_each_shape_class_once(context):
     again = complex_gemm(context, a, b, precision="mixed")
     assert np.array_equal(first, again)
     assert len(C.gemm_tuned_classes()) == len(table)
+
+
+@pytest.mark.parametrize("m,n,k", [(1, 1, 1), (7, 9, 3), (8, 8, 4), (64, 64, 8), (65, 8, 9), (63, 65, 31), (128, 24, 33),
+                                   (20, 20, 1000), (160, 41, 700), (100, 13, 4096), (200, 70, 257)])
+@pytest.mark.parametrize("adjoint", [False, True])
+def test_small_fp64_products(context, m, n, k, adjoint):
+    """The library's FP64 product at the edges of its tiles (64 rows, 8 to 64 columns, K stages of 8) and of its
+    K shares: two sums of k rounded products differ by at most 4 k eps |A||B| per entry, sqrt(k) eps in norm for
+    independent roundings (1.4e-14 at k = 4096)."""
+    rng = np.random.default_rng(m + 131 * n + 17 * k)
+    a = random(rng, (k, m) if adjoint else (m, k))
+    b, c = random(rng, (k, n)), random(rng, (m, n))
+    ref = (a.conj().T if adjoint else a) @ b
+    assert relative_error(complex_gemm(context, a, b, adjoint_a=adjoint), ref) < 1.5e-14
+    assert relative_error(complex_gemm(context, a, b, adjoint_a=adjoint, c=c), ref + c) < 1.5e-14
