@@ -317,11 +317,11 @@ void DavidsonSolver::update_projected(const Cx<double>* applied, Cx<double>* cac
     auto& ctx = op_.context();
     const long long kexp = expanded_k(n_, split_);
     umma_complex_gemm(static_cast<std::uint16_t*>(pack_vc_.ptr), ld_rows_, packed_applied + 2LL * first * ld_rows_,
-                      ld_rows_, size_, columns, kexp, cached + static_cast<long long>(first) * capacity_, capacity_,
+                      ld_rows_, size_, columns, kexp, split_, cached + static_cast<long long>(first) * capacity_, capacity_,
                       false, 1.0, ctx.tc.partial, ctx.stream);
     if (first)
       umma_complex_gemm(static_cast<std::uint16_t*>(pack_vc_.ptr) + first * ld_rows_, ld_rows_, packed_applied,
-                        ld_rows_, columns, first, kexp, cached + first, capacity_, false, 1.0, ctx.tc.partial,
+                        ld_rows_, columns, first, kexp, split_, cached + first, capacity_, false, 1.0, ctx.tc.partial,
                         ctx.stream);
     return;
   }

@@ -117,6 +117,7 @@ struct EpilogueArgs {
   ProductOutput out[2];        // direct outputs (when partial is null)
   int second;                  // first complex column of out[1]
   double alpha;
+  bool shared_terms;           // BF16x3 blocks: term 0 in elements 0-31, term 1 in 32-63
 };
 
 // PAIR: the product's columns go to two outputs.
@@ -181,9 +182,17 @@ __global__ void __launch_bounds__(kThreads, 1)
       if (!mbar_wait(&full[s], (i / S) & 1)) break;
       tc_fence_after();
       const std::uint32_t a_addr = smem_u32(smem + s * STAGE), b_addr = a_addr + A_BYTES;
+      if (ep.shared_terms) {
+        // Products (0,0), (0,1), (1,0) of the block's terms, two K = 16 steps each (byte offsets in a 128-byte row).
 #pragma unroll
-      for (int kk = 0; kk < BK / 16; ++kk)
-        umma_bf16(tmem, smem_desc(a_addr + kk * 32), smem_desc(b_addr + kk * 32), idesc, (i | kk) != 0);
+        for (int kk = 0; kk < 6; ++kk)
+          umma_bf16(tmem, smem_desc(a_addr + (kk >= 4 ? 64 : 0) + (kk & 1) * 32),
+                    smem_desc(b_addr + (kk == 2 || kk == 3 ? 64 : 0) + (kk & 1) * 32), idesc, (i | kk) != 0);
+      } else {
+#pragma unroll
+        for (int kk = 0; kk < BK / 16; ++kk)
+          umma_bf16(tmem, smem_desc(a_addr + kk * 32), smem_desc(b_addr + kk * 32), idesc, (i | kk) != 0);
+      }
       umma_commit(&empty[s]);
     }
     umma_commit(accum);
@@ -285,8 +294,8 @@ __global__ void reduce_splits_kernel(int m, int n, int splits, const Cx<float>* 
 
 // ---- packing (FP64 complex -> BF16 split terms) ---------------------------
 
-// Split-term index of product p on the A and B side: BF16x3 pairs (0,0) (0,1)
-// (1,0); BF16x6 adds (0,2) (1,1) (2,0).
+// Split-term index of BF16x6 product p on the A and B side: (0,0) (0,1) (1,0)
+// (0,2) (1,1) (2,0).
 __host__ __device__ constexpr int term_a(int p) { return p == 2 || p == 4 ? 1 : p == 5 ? 2 : 0; }
 __host__ __device__ constexpr int term_b(int p) { return p == 1 || p == 4 ? 1 : p == 3 ? 2 : 0; }
 
@@ -301,36 +310,46 @@ __device__ __forceinline__ void split3(double x, std::uint16_t t[3]) {
   t[2] = __bfloat16_as_ushort(h2);
 }
 
-// Stores P (lo, hi) uint16 pairs at dst with 8-byte stores when P is even
-// (dst is then 8-byte aligned: rows are 128-byte aligned and each value
-// takes 4P bytes), else 4-byte stores.
-template <int P>
-__device__ __forceinline__ void store_pairs(std::uint16_t* dst, const std::uint32_t (&pairs)[P]) {
-  if constexpr (P % 2 == 0) {
-    auto* d = reinterpret_cast<uint2*>(dst);
-#pragma unroll
-    for (int q = 0; q < P / 2; ++q) d[q] = make_uint2(pairs[2 * q], pairs[2 * q + 1]);
-  } else {
-    auto* d = reinterpret_cast<std::uint32_t*>(dst);
-#pragma unroll
-    for (int q = 0; q < P; ++q) d[q] = pairs[q];
-  }
-}
-
 __device__ __forceinline__ std::uint32_t pair(std::uint16_t lo, std::uint16_t hi) {
   return static_cast<std::uint32_t>(lo) | (static_cast<std::uint32_t>(hi) << 16);
 }
 
-// Writes the 2P A-side entries of one complex value.
-template <int P>
-__device__ __forceinline__ void write_a(std::uint16_t* dst, Cx<double> v) {
-  std::uint16_t re[3], im[3];
-  split3(v.re, re);
-  split3(v.im, im);
-  std::uint32_t pairs[P];
+// Writes the entries of complex k in an expanded row: terms of (x, y) as pairs.
+// BF16x3 rows hold each of the two terms once, BF16x6 rows the six product terms.
+template <int P, bool SIDE_B>
+__device__ __forceinline__ void write_entry(std::uint16_t* row, long long k, double x, double y, std::uint32_t sign) {
+  std::uint16_t u[3], v[3];
+  split3(x, u);
+  split3(y, v);
+  if constexpr (P == 3) {
+    auto* d = reinterpret_cast<std::uint32_t*>(row + (k / kSharedBlock) * 64 + (k % kSharedBlock) * 2);
+    d[0] = pair(u[0], v[0]) ^ sign;
+    d[kSharedBlock] = pair(u[1], v[1]) ^ sign;
+  } else {
+    auto* d = reinterpret_cast<uint2*>(row + k * 2 * P);  // 24 bytes an entry in 128-byte rows: 8-byte aligned
 #pragma unroll
-  for (int p = 0; p < P; ++p) pairs[p] = pair(re[term_a(p)], im[term_a(p)]);
-  store_pairs<P>(dst, pairs);
+    for (int p = 0; p < P; p += 2) {
+      const int t0 = SIDE_B ? term_b(p) : term_a(p), t1 = SIDE_B ? term_b(p + 1) : term_a(p + 1);
+      d[p / 2] = make_uint2(pair(u[t0], v[t0]) ^ sign, pair(u[t1], v[t1]) ^ sign);
+    }
+  }
+}
+template <int P>
+__device__ __forceinline__ void write_a(std::uint16_t* row, long long k, Cx<double> v) {
+  write_entry<P, false>(row, k, v.re, v.im, 0u);
+}
+
+// Zeros the entries k..end of an expanded row of kexp elements, thread `first` of `count`.
+template <int P>
+__device__ __forceinline__ void zero_tail(std::uint16_t* row, int k, long long kexp, int first, int count) {
+  if constexpr (P == 3) {
+    for (long long q = k + first; q < kexp / 64 * kSharedBlock; q += count) {
+      auto* d = reinterpret_cast<std::uint32_t*>(row + (q / kSharedBlock) * 64 + (q % kSharedBlock) * 2);
+      d[0] = d[kSharedBlock] = 0u;
+    }
+  } else {
+    for (long long q = 2LL * P * k + first; q < kexp; q += count) row[q] = 0;
+  }
 }
 
 // One row i of A per blockIdx.y; threads stride over k.
@@ -345,19 +364,18 @@ __global__ void pack_a_direct_kernel(const Cx<double>* __restrict__ src, long lo
     for (int kk = blockIdx.x * blockDim.x + threadIdx.x; kk < k; kk += gridDim.x * blockDim.x) {
       Cx<double> v = in[kk];
       if (CONJ_T) v.im = -v.im;
-      write_a<P>(row + static_cast<long long>(kk) * 2 * P, v);
+      write_a<P>(row, kk, v);
     }
-    // zero padding [2Pk, kexp) of the row
-    for (long long q = 2LL * P * k + blockIdx.x * blockDim.x + threadIdx.x; q < kexp;
-         q += static_cast<long long>(gridDim.x) * blockDim.x)
-      row[q] = 0;
+    zero_tail<P>(row, k, kexp, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
   }
 }
 
 // A[i,k] = src[i + k*lds] (rows contiguous): 32x32 shared-memory transpose.
+// kexp > 0: the rows end there, and the last blocks zero what follows entry k.
 template <int P>
 __global__ void pack_a_transpose_kernel(const Cx<double>* __restrict__ src, long long lds, int rows, int k,
-                                        std::uint16_t* __restrict__ out, long long ldo, long long out_k_offset) {
+                                        std::uint16_t* __restrict__ out, long long ldo, long long out_k_offset,
+                                        long long kexp) {
   __shared__ Cx<double> tile[32][33];
   const int i0 = blockIdx.x * 32, k0 = blockIdx.y * 32;
   const int tx = threadIdx.x, ty = threadIdx.y;  // 32 x 8
@@ -368,17 +386,11 @@ __global__ void pack_a_transpose_kernel(const Cx<double>* __restrict__ src, long
   __syncthreads();
   for (int r = ty; r < 32; r += 8) {
     const int i = i0 + r, kk = k0 + tx;
-    if (i < rows && kk < k) write_a<P>(out + static_cast<long long>(i) * ldo + (out_k_offset + kk) * 2 * P, tile[tx][r]);
+    if (i < rows && kk < k) write_a<P>(out + static_cast<long long>(i) * ldo, out_k_offset + kk, tile[tx][r]);
   }
-}
-
-template <int P>
-__global__ void zero_pad_kernel(std::uint16_t* __restrict__ out, long long ldo, int rows, long long from, long long to) {
-  const long long pad = to - from;
-  const long long total = static_cast<long long>(rows) * pad;
-  for (long long idx = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; idx < total;
-       idx += static_cast<long long>(gridDim.x) * blockDim.x)
-    out[(idx / pad) * ldo + from + idx % pad] = 0;
+  if (kexp > 0 && blockIdx.y == gridDim.y - 1)
+    for (int r = ty; r < 32 && i0 + r < rows; r += 8)
+      zero_tail<P>(out + static_cast<long long>(i0 + r) * ldo, k, kexp, tx, 32);
 }
 
 // Source columns j = blockIdx.y, blockIdx.y + gridDim.y, ... (two expanded
@@ -392,24 +404,11 @@ __global__ void pack_b_kernel(const Cx<double>* __restrict__ src, long long ldb,
     std::uint16_t* row1 = row0 + ldo;
     for (int kk = blockIdx.x * blockDim.x + threadIdx.x; kk < k; kk += gridDim.x * blockDim.x) {
       const Cx<double> v = in[kk];
-      std::uint16_t re[3], im[3];
-      split3(v.re, re);
-      split3(v.im, im);
-      std::uint32_t p0[P], p1[P];
-#pragma unroll
-      for (int p = 0; p < P; ++p) {
-        const int t = term_b(p);
-        p0[p] = pair(re[t], im[t] ^ 0x8000u);  // [Re, -Im] (sign flip is exact)
-        p1[p] = pair(im[t], re[t]);            // [Im, Re]
-      }
-      store_pairs<P>(row0 + static_cast<long long>(kk) * 2 * P, p0);
-      store_pairs<P>(row1 + static_cast<long long>(kk) * 2 * P, p1);
+      write_entry<P, true>(row0, kk, v.re, v.im, 0x80000000u);  // [Re, -Im] (sign flip is exact)
+      write_entry<P, true>(row1, kk, v.im, v.re, 0u);           // [Im, Re]
     }
-    for (long long q = 2LL * P * k + blockIdx.x * blockDim.x + threadIdx.x; q < kexp;
-         q += static_cast<long long>(gridDim.x) * blockDim.x) {
-      row0[q] = 0;
-      row1[q] = 0;
-    }
+    zero_tail<P>(row0, k, kexp, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
+    zero_tail<P>(row1, k, kexp, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
   }
 }
 
@@ -421,10 +420,6 @@ constexpr int kMaxGridY = 65535;
 unsigned row_blocks(long long length, int rows) {
   const long long per_row = std::max<long long>(1, (148LL * 16 + rows - 1) / rows);
   return static_cast<unsigned>(std::max<long long>(1, std::min<long long>(per_row, (length + 255) / 256)));
-}
-
-unsigned grid_for(long long total) {
-  return static_cast<unsigned>(std::min<long long>(std::max<long long>(1, (total + 255) / 256), 148LL * 16));
 }
 
 // ---- tensor maps -----------------------------------------------------------
@@ -486,7 +481,7 @@ void pack_a(Op aop, const Cx<double>* src, long long lds, int rows, int k, Split
             long long ldo, cudaStream_t stream) {
   const long long kexp = expanded_k(k, split);
   if (aop == Op::C) {
-    const dim3 grid(row_blocks(std::max<long long>(k, kexp - 2LL * split_terms(split) * k), rows),
+    const dim3 grid(row_blocks(k, rows),
                     static_cast<unsigned>(std::min(rows, kMaxGridY)));
     if (split == Split::BF16x3)
       pack_a_direct_kernel<3, true><<<grid, 256, 0, stream>>>(src, lds, rows, k, out, ldo, kexp);
@@ -497,16 +492,10 @@ void pack_a(Op aop, const Cx<double>* src, long long lds, int rows, int k, Split
   }
   const dim3 grid(static_cast<unsigned>(ceil_div(rows, 32)), static_cast<unsigned>(ceil_div(k, 32)));
   if (split == Split::BF16x3)
-    pack_a_transpose_kernel<3><<<grid, dim3(32, 8), 0, stream>>>(src, lds, rows, k, out, ldo, 0);
+    pack_a_transpose_kernel<3><<<grid, dim3(32, 8), 0, stream>>>(src, lds, rows, k, out, ldo, 0, kexp);
   else
-    pack_a_transpose_kernel<6><<<grid, dim3(32, 8), 0, stream>>>(src, lds, rows, k, out, ldo, 0);
+    pack_a_transpose_kernel<6><<<grid, dim3(32, 8), 0, stream>>>(src, lds, rows, k, out, ldo, 0, kexp);
   SDFT_LAUNCH("pack_a_transpose_kernel");
-  const long long from = 2LL * split_terms(split) * k;
-  if (kexp > from) {
-    zero_pad_kernel<3><<<grid_for(static_cast<long long>(rows) * (kexp - from)), 256, 0, stream>>>(out, ldo, rows,
-                                                                                                  from, kexp);
-    SDFT_LAUNCH("zero_pad_kernel");
-  }
 }
 
 void pack_a_columns(const Cx<double>* src, long long lds, int rows, int first, int count, Split split,
@@ -515,16 +504,16 @@ void pack_a_columns(const Cx<double>* src, long long lds, int rows, int first, i
   const dim3 grid(static_cast<unsigned>(ceil_div(rows, 32)), static_cast<unsigned>(ceil_div(count, 32)));
   const Cx<double>* s = src + static_cast<long long>(first) * lds;
   if (split == Split::BF16x3)
-    pack_a_transpose_kernel<3><<<grid, dim3(32, 8), 0, stream>>>(s, lds, rows, count, out, ldo, first);
+    pack_a_transpose_kernel<3><<<grid, dim3(32, 8), 0, stream>>>(s, lds, rows, count, out, ldo, first, 0);
   else
-    pack_a_transpose_kernel<6><<<grid, dim3(32, 8), 0, stream>>>(s, lds, rows, count, out, ldo, first);
+    pack_a_transpose_kernel<6><<<grid, dim3(32, 8), 0, stream>>>(s, lds, rows, count, out, ldo, first, 0);
   SDFT_LAUNCH("pack_a_transpose_kernel");
 }
 
 void pack_b(const Cx<double>* src, long long ldb, int k, int n, Split split, std::uint16_t* out, long long ldo,
             cudaStream_t stream) {
   const long long kexp = expanded_k(k, split);
-  const dim3 grid(row_blocks(std::max<long long>(k, kexp - 2LL * split_terms(split) * k), n),
+  const dim3 grid(row_blocks(k, n),
                   static_cast<unsigned>(std::min(n, kMaxGridY)));
   if (split == Split::BF16x3) pack_b_kernel<3><<<grid, 256, 0, stream>>>(src, ldb, k, n, out, ldo, kexp);
   else pack_b_kernel<6><<<grid, 256, 0, stream>>>(src, ldb, k, n, out, ldo, kexp);
@@ -574,13 +563,13 @@ int model_splits(int m, int n2, int k_blocks, int bn) {
 
 // One product with the given tile width and split count.
 void run_config(const std::uint16_t* a, long long lda, const std::uint16_t* b, long long ldb, int m, int n,
-                long long kexp, const ProductOutput out[2], int second, double alpha, int bn, int splits,
+                long long kexp, Split split, const ProductOutput out[2], int second, double alpha, int bn, int splits,
                 Scratch& workspace, cudaStream_t stream) {
   const int n2 = 2 * n;
   const int k_blocks = static_cast<int>(kexp / BK);
   const int kpb = static_cast<int>(ceil_div(k_blocks, splits));
   splits = static_cast<int>(ceil_div(k_blocks, kpb));
-  EpilogueArgs ep{m, n2, nullptr, {out[0], out[1]}, second, alpha};
+  EpilogueArgs ep{m, n2, nullptr, {out[0], out[1]}, second, alpha, split == Split::BF16x3};
   if (splits > 1)
     ep.partial = static_cast<Cx<float>*>(workspace.reserve(sizeof(Cx<float>) * static_cast<std::size_t>(m) * n * splits));
   if (bn == 256) launch<256>(a, lda, b, ldb, m, n2, kexp, ep, splits, k_blocks, kpb, stream);
@@ -608,9 +597,10 @@ void run_config(const std::uint16_t* a, long long lda, const std::uint16_t* b, l
 struct ShapeClass {
   int row_tiles, column_units, k_blocks;
   bool share_k;  // whether K may be split
+  Split split;
   bool operator<(const ShapeClass& o) const {
-    return std::tie(row_tiles, column_units, k_blocks, share_k) <
-           std::tie(o.row_tiles, o.column_units, o.k_blocks, o.share_k);
+    return std::tie(row_tiles, column_units, k_blocks, share_k, split) <
+           std::tie(o.row_tiles, o.column_units, o.k_blocks, o.share_k, o.split);
   }
 };
 struct TileChoice {
@@ -631,22 +621,22 @@ bool autotune_enabled() {
 }
 
 TileChoice tuned_choice(const std::uint16_t* a, long long lda, const std::uint16_t* b, long long ldb, int m, int n,
-                        long long kexp, bool share_k, cudaStream_t stream) {
+                        long long kexp, Split split, bool share_k, cudaStream_t stream) {
   const int n2 = 2 * n;
   const int k_blocks = static_cast<int>(kexp / BK);
   int k_class = 1;
   for (int j = 1; k_class < k_blocks; ++j) k_class = static_cast<int>(std::ceil(std::exp2(j / 8.0)));
   const ShapeClass key{static_cast<int>(ceil_div(m, BM)), static_cast<int>(ceil_div(n2, 32)), k_class,
-                       share_k};
+                       share_k, split};
   std::lock_guard<std::mutex> lock(g_tune_mutex);
   auto found = g_tuned.find(key);
   if (found != g_tuned.end()) return found->second;
   std::vector<std::pair<int, int>> candidates;
   for (int bn : {128, 160, 256}) {
     const int s = share_k ? model_splits(m, n2, k_blocks, bn) : 1;
-    for (int split : {1, s, share_k ? std::min(max_splits_for(k_blocks), 2 * s) : 1})
-      if (std::find(candidates.begin(), candidates.end(), std::make_pair(bn, split)) == candidates.end())
-        candidates.emplace_back(bn, split);
+    for (int count : {1, s, share_k ? std::min(max_splits_for(k_blocks), 2 * s) : 1})
+      if (std::find(candidates.begin(), candidates.end(), std::make_pair(bn, count)) == candidates.end())
+        candidates.emplace_back(bn, count);
   }
   static thread_local Scratch output, partials;
   auto* c = static_cast<Cx<double>*>(output.reserve(sizeof(Cx<double>) * static_cast<std::size_t>(m) * n));
@@ -658,9 +648,9 @@ TileChoice tuned_choice(const std::uint16_t* a, long long lda, const std::uint16
   const ProductOutput scratch[2] = {product_output(c, m, false), {}};
   try {
     for (const auto& [bn, splits] : candidates) {
-      run_config(a, lda, b, ldb, m, n, kexp, scratch, n, 1.0, bn, splits, partials, stream);
+      run_config(a, lda, b, ldb, m, n, kexp, split, scratch, n, 1.0, bn, splits, partials, stream);
       SDFT_CUDA(cudaEventRecord(start, stream));
-      run_config(a, lda, b, ldb, m, n, kexp, scratch, n, 1.0, bn, splits, partials, stream);
+      run_config(a, lda, b, ldb, m, n, kexp, split, scratch, n, 1.0, bn, splits, partials, stream);
       SDFT_CUDA(cudaEventRecord(stop, stream));
       SDFT_CUDA(cudaEventSynchronize(stop));
       float ms = 0;
@@ -682,28 +672,30 @@ TileChoice tuned_choice(const std::uint16_t* a, long long lda, const std::uint16
 
 namespace {
 void product(const std::uint16_t* a, long long lda, const std::uint16_t* b, long long ldb, int m, int n,
-             long long kexp, const ProductOutput out[2], int second, double alpha, bool share_k, Scratch& workspace,
+             long long kexp, Split split, const ProductOutput out[2], int second, double alpha, bool share_k,
+             Scratch& workspace,
              cudaStream_t stream) {
   if (m <= 0 || n <= 0 || kexp <= 0) return;
   if (kexp % BK != 0) throw InvalidArgument("expanded K must be a multiple of 64");
   int bn, splits;
   if (autotune_enabled()) {
-    const TileChoice choice = tuned_choice(a, lda, b, ldb, m, n, kexp, share_k, stream);
+    const TileChoice choice = tuned_choice(a, lda, b, ldb, m, n, kexp, split, share_k, stream);
     bn = choice.bn;
     splits = choice.splits;
   } else {
     bn = model_width(2 * n);
     splits = share_k ? model_splits(m, 2 * n, static_cast<int>(kexp / BK), bn) : 1;
   }
-  run_config(a, lda, b, ldb, m, n, kexp, out, second, alpha, bn, splits, workspace, stream);
+  run_config(a, lda, b, ldb, m, n, kexp, split, out, second, alpha, bn, splits, workspace, stream);
 }
 }  // namespace
 
 void umma_complex_gemm(const std::uint16_t* a, long long lda, const std::uint16_t* b, long long ldb, int m, int n,
-                       long long kexp, Cx<double>* c, long long ldc, bool add, double alpha, Scratch& workspace,
+                       long long kexp, Split split, Cx<double>* c, long long ldc, bool add, double alpha,
+                       Scratch& workspace,
                        cudaStream_t stream) {
   const ProductOutput out[2] = {product_output(c, ldc, add), {}};
-  product(a, lda, b, ldb, m, n, kexp, out, n, alpha, true, workspace, stream);
+  product(a, lda, b, ldb, m, n, kexp, split, out, n, alpha, true, workspace, stream);
 }
 
 std::size_t gemm_tuned_classes(std::size_t capacity, int* rows) {
@@ -770,7 +762,7 @@ void gemm_tc(Op aop, int m, int n, int k, const Cx<double>* a, long long lda, co
   }
   auto* pb = static_cast<std::uint16_t*>(ws.b.reserve(sizeof(std::uint16_t) * static_cast<std::size_t>(kexp) * 2 * n));
   pack_b(b, ldb, k, n, split, pb, kexp, stream);
-  umma_complex_gemm(pa, lda_p, pb, kexp, m, n, kexp, c, ldc, add, alpha, ws.partial, stream);
+  umma_complex_gemm(pa, lda_p, pb, kexp, m, n, kexp, split, c, ldc, add, alpha, ws.partial, stream);
 }
 
 void gemm_tc_packed(const PackedA& packed, int n, const Cx<double>* b, long long ldb, const ProductOutput out[2],
@@ -779,7 +771,7 @@ void gemm_tc_packed(const PackedA& packed, int n, const Cx<double>* b, long long
   const long long kexp = expanded_k(packed.k, packed.split);
   auto* pb = static_cast<std::uint16_t*>(ws.b.reserve(sizeof(std::uint16_t) * static_cast<std::size_t>(kexp) * 2 * n));
   pack_b(b, ldb, packed.k, n, packed.split, pb, kexp, stream);
-  product(packed.data, packed.ld, pb, kexp, packed.rows, n, kexp, out, second, 1.0, false, ws.partial, stream);
+  product(packed.data, packed.ld, pb, kexp, packed.rows, n, kexp, packed.split, out, second, 1.0, false, ws.partial, stream);
 }
 
 unsigned int umma_error_flag() {

@@ -1,14 +1,22 @@
 // Tensor-core (tcgen05 / TMEM / TMA) complex GEMM with BF16 split products.
 //
-// A complex product C = op(A) B is evaluated as one real BF16 GEMM over an
-// expanded K axis. Every complex k contributes P split-product terms
-// (x ~ x0 + x1 + x2 in BF16, products a_i b_j for the pairs of the chosen
-// pattern) and, for each term, the pair (re, im):
-//   Ahat[i, (k*P+p)*2 + 0] = A_{ia(p)}(Re A[i,k]),  Ahat[i, (k*P+p)*2 + 1] = A_{ia(p)}(Im A[i,k])
-//   Bhat[2j,   (k*P+p)*2 + {0,1}] = ( B_{ib(p)}(Re B[k,j]), -B_{ib(p)}(Im B[k,j]) )
-//   Bhat[2j+1, (k*P+p)*2 + {0,1}] = ( B_{ib(p)}(Im B[k,j]),  B_{ib(p)}(Re B[k,j]) )
+// A complex product C = op(A) B is evaluated as one real BF16 GEMM whose K axis
+// holds, for every complex k, the pair (re, im) of the split terms x ~ x0 + x1
+// (+ x2):
+//   Ahat[i, .]    = ( A_t(Re A[i,k]),  A_t(Im A[i,k]) )
+//   Bhat[2j, .]   = ( B_t(Re B[k,j]), -B_t(Im B[k,j]) )
+//   Bhat[2j+1, .] = ( B_t(Im B[k,j]),  B_t(Re B[k,j]) )
 // so that (Ahat Bhat^T)[i, 2j] = Re C[i,j] and [i, 2j+1] = Im C[i,j], with the
-// FP32 accumulator held in tensor memory. Both operands are K-major BF16 rows.
+// FP32 accumulator held in tensor memory. Both operands are K-major BF16 rows
+// of 64-element (128-byte) blocks.
+//   BF16x3: a block holds 16 complex k, term 0 of all of them and then term 1
+//   (32 elements each), every term once; the kernel forms the products (0,0),
+//   (0,1), (1,0) of a block from the same staged data. (With every product's
+//   operands stored, a k-th of the row was 6 elements instead of 4 and the
+//   tensor cores waited for shared-memory fills: 55 -> 42 us for B x of 160
+//   columns at 512 x 23847, 14 -> 11.5 us for its packing.)
+//   BF16x6: 6 product terms p per k, elements (k*6 + p)*2 + {0, 1}: A holds
+//   term ia(p), B term ib(p), and the product is a plain one.
 #pragma once
 #include <cstdint>
 
@@ -23,11 +31,13 @@ enum class Split : int { BF16x3 = 3, BF16x6 = 6 };
 
 inline int split_terms(Split s) { return static_cast<int>(s); }
 
-// Expanded-K length (bf16 elements) of a K-long complex contraction, padded to
-// the 64-element tensor-core K block.
+constexpr int kSharedBlock = 16;  // complex k of a BF16x3 block
+
+// Expanded-K length (bf16 elements) of a K-long complex contraction, whole
+// 64-element tensor-core K blocks.
 inline long long expanded_k(int k, Split s) {
-  const long long raw = 2LL * split_terms(s) * k;
-  return (raw + 63) / 64 * 64;
+  if (s == Split::BF16x3) return (static_cast<long long>(k) + kSharedBlock - 1) / kSharedBlock * 64;
+  return (2LL * split_terms(s) * k + 63) / 64 * 64;
 }
 
 // A side: out[i][kexp] for i < rows (row stride ldo bf16 elements), from the
@@ -42,7 +52,7 @@ void pack_b(const Cx<double>* src, long long ldb, int k, int n, Split split, std
 
 // Same, but writes the A-side layout for `count` new K entries of an
 // existing packed row block: columns [first, first+count) of the complex
-// source (ld lds, rows rows) become expanded-K entries first*2P.. of each row
+// source (ld lds, rows rows) become complex entries first.. of each row
 // (used to extend a packed transposed basis without repacking it).
 void pack_a_columns(const Cx<double>* src, long long lds, int rows, int first, int count, Split split,
                     std::uint16_t* out, long long ldo, cudaStream_t stream);
@@ -51,7 +61,7 @@ void pack_a_columns(const Cx<double>* src, long long lds, int rows, int first, i
 // Ahat is m x kexp and Bhat is 2n x kexp (BF16, K-major, leading dims lda/ldb
 // in elements, 16-byte multiples). kexp = expanded_k(k, split).
 void umma_complex_gemm(const std::uint16_t* a, long long lda, const std::uint16_t* b, long long ldb, int m, int n,
-                       long long kexp, Cx<double>* c, long long ldc, bool add, double alpha, Scratch& workspace,
+                       long long kexp, Split split, Cx<double>* c, long long ldc, bool add, double alpha, Scratch& workspace,
                        cudaStream_t stream);
 
 // The tile autotuner's table so far: per shape class (rows rounded up to

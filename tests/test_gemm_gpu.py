@@ -166,3 +166,16 @@ def test_small_fp64_products(context, m, n, k, adjoint):
     ref = (a.conj().T if adjoint else a) @ b
     assert relative_error(complex_gemm(context, a, b, adjoint_a=adjoint), ref) < 1.5e-14
     assert relative_error(complex_gemm(context, a, b, adjoint_a=adjoint, c=c), ref + c) < 1.5e-14
+
+
+@pytest.mark.parametrize("k", [1, 15, 16, 17, 31, 33, 100])
+@pytest.mark.parametrize("adjoint", [False, True])
+def test_mixed_products_at_block_edges(context, k, adjoint):
+    """K around the 16 complex entries of a packed block: the padding entries are zero on both sides. Dropped
+    split products are below 3 * 2^-17 of |A||B| entry by entry (2.3e-5), and average out in norm."""
+    rng = np.random.default_rng(700 + k)
+    a = random(rng, (k, 130) if adjoint else (130, k))
+    b, c = random(rng, (k, 41)), random(rng, (130, 41))
+    ref = (a.conj().T if adjoint else a) @ b
+    assert relative_error(complex_gemm(context, a, b, adjoint_a=adjoint, precision="mixed"), ref) < 2e-5
+    assert relative_error(complex_gemm(context, a, b, adjoint_a=adjoint, precision="mixed", c=c), ref + c) < 2e-5
