@@ -759,14 +759,13 @@ void DeviceOperator::project(const Cx<double>* x, int columns, Cx<double>* p, Pr
 }
 
 // Whether the back-projection is the library's joint product, which saves
-// launches and reads B^H once: FP64 where B^H is small (one B200, 64 x 936 and
-// 20 columns 4.9 us against cuBLAS's 6.9), mixed up to 3e6 entries of B (both
-// images of 80 columns at 8564 x 256: 221 -> 210 us; at 17137 x 512 with 160
-// columns two products and a copy are the faster, 625 against 641 us). A rule on
-// B alone, and K (the projectors) never shared between CTAs: the joint
-// application's sums are those of the separate ones, bit for bit.
+// launches and reads B^H once: mixed always (H and S of 10 columns at 1067 plane
+// waves 75 -> 55 us, of 160 at 17137 627 -> 546), FP64 where B^H is small (one
+// B200, 64 x 936 and 20 columns 4.9 us against cuBLAS's 6.9). A rule on B alone,
+// and K (the projectors) never shared between CTAs: the joint application's sums
+// are those of the separate ones, bit for bit.
 bool DeviceOperator::own_backprojection(Precision precision) const {
-  return static_cast<double>(npw_) * np_ <= (precision == Precision::FP64 ? 262144.0 : 3e6);
+  return precision != Precision::FP64 || static_cast<double>(npw_) * np_ <= 262144.0;
 }
 
 // out[0] from the first `second` of dp's columns, out[1] from the rest.
@@ -787,11 +786,7 @@ void DeviceOperator::add_backprojection(const Cx<double>* dp, int columns, Cx<do
     return;
   }
   if (prior != y) scale_copy(prior, npw_, y, npw_, npw_, columns, prior_scale, ctx_.stream);
-  if (precision == Precision::FP64)
-    zgemm(ctx_.blas, Op::C, Op::N, npw_, columns, np_, b_, np_, dp, np_, y, npw_, true);
-  else
-    gemm_tc(Op::C, npw_, columns, np_, b_, np_, &bh_packed_, dp, np_, y, npw_, true, 1.0, bh_packed_.split, ctx_.tc,
-            ctx_.stream);
+  zgemm(ctx_.blas, Op::C, Op::N, npw_, columns, np_, b_, np_, dp, np_, y, npw_, true);
 }
 
 // y = prior_scale prior + B^H M P, M the D or Q blocks.

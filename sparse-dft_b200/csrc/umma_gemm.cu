@@ -1,14 +1,23 @@
 // tcgen05 / TMEM / TMA BF16 GEMM for the mixed-precision complex products.
 //
-// One CTA computes a 128 x BN FP32 tile of Ahat Bhat^T over a range of 64-wide
-// K blocks (split-K across CTAs). Warp 0 lane 0 streams A and B tiles with TMA
-// (128-byte swizzle, no multicast) into a STAGES-deep shared-memory ring;
-// warp 1 lane 0 issues tcgen05.mma (M=128, N=BN, K=16 per instruction) into a
-// tensor-memory accumulator and releases ring slots with tcgen05.commit; then
-// all four warps drain the accumulator with tcgen05.ld (warp w owns TMEM lanes
-// 32w..32w+31) and write either FP32 split-K partials or the final FP64
-// complex result. Every mbarrier wait is bounded; a wait that runs out sets a
-// device error word and the CTA winds down (the host turns it into an error).
+// One CTA per SM walks over 128 x BN FP32 tiles of Ahat Bhat^T, each over a
+// range of 64-wide K blocks (split-K across tiles). Warp 0 lane 0 streams A and
+// B tiles with TMA (128-byte swizzle, no multicast) into a STAGES-deep
+// shared-memory ring; warp 1 lane 0 issues tcgen05.mma (M=128, N=BN, K=16 per
+// instruction) into one of two tensor-memory accumulators and releases ring
+// slots with tcgen05.commit; eight more warps drain the other accumulator with
+// tcgen05.ld (warp w may read TMEM lanes 32 (w % 4) and up; two warps share
+// each quarter's columns) and write either FP32 split-K partials or the final
+// FP64 complex result, while the next tile's products run. Every mbarrier wait
+// is bounded; a wait that runs out sets a device error word and the CTA winds
+// down (the host turns it into an error).
+// Tall products are bound by their FP64 results (and the values they add to),
+// not by the tensor cores: with one tile per CTA, four warps reading a chunk's
+// prior values only once they came to it and nothing running meanwhile, the
+// joint back-projection of 160 columns at 23847 x 512 took 197 us; with the
+// epilogue's loads a chunk ahead and beside the next tile's products 113 us
+// (245 MB of results and priors, 38 us at copy rate). B x of the same block,
+// bound by shared-memory fills, stays at 42-44 us.
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cudaTypedefs.h>
@@ -28,7 +37,9 @@ namespace sdft_b200 {
 
 namespace {
 
-constexpr int BM = 128, BK = 64, kThreads = 128;
+constexpr int BM = 128, BK = 64;
+constexpr int kEpilogueWarps = 8;  // warps 2..9
+constexpr int kThreads = 32 * (2 + kEpilogueWarps);
 constexpr unsigned long long kWaitLimitNs = 2000000000ULL;  // 2 s per wait
 
 __device__ unsigned int g_umma_error = 0;
@@ -46,6 +57,9 @@ __device__ __forceinline__ void mbar_init(std::uint64_t* bar, std::uint32_t coun
 }
 __device__ __forceinline__ void mbar_arrive_expect_tx(std::uint64_t* bar, std::uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void mbar_arrive(std::uint64_t* bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 __device__ __forceinline__ bool mbar_try_wait(std::uint64_t* bar, std::uint32_t parity) {
   std::uint32_t ok;
@@ -111,6 +125,21 @@ __host__ __device__ constexpr int stages() {
   return BN >= 256 ? 4 : 6;
 }
 
+// The tiles of a product: columns fastest, so that the CTAs sharing an A tile
+// work on it together and all but the first read it from L2; then rows, then
+// shares of K.
+struct WorkTile {
+  int row, column, split;
+};
+struct TileGrid {
+  int columns, rows;
+  long long count;
+  __device__ WorkTile at(long long w) const {
+    const long long strip = w / columns;
+    return {static_cast<int>(strip % rows), static_cast<int>(w % columns), static_cast<int>(strip / rows)};
+  }
+};
+
 struct EpilogueArgs {
   int m, n2;                   // rows, real columns (2 x complex columns)
   Cx<float>* partial;          // split-K output [split][n2/2][m] or null
@@ -124,31 +153,29 @@ struct EpilogueArgs {
 template <int BN, bool PAIR>
 __global__ void __launch_bounds__(kThreads, 1)
     umma_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
-                     int k_blocks_total, int k_blocks_per_split, EpilogueArgs ep) {
+                     int k_blocks_total, int k_blocks_per_split, TileGrid tiles, EpilogueArgs ep) {
   constexpr int S = stages<BN>();
   constexpr int A_BYTES = BM * BK * 2, B_BYTES = BN * BK * 2, STAGE = A_BYTES + B_BYTES;
-  constexpr std::uint32_t TMEM_COLS = BN <= 32 ? 32 : BN <= 64 ? 64 : BN <= 128 ? 128 : 256;
+  constexpr std::uint32_t TMEM_COLS = BN <= 128 ? 256 : 512;  // two accumulators
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>(
       (reinterpret_cast<std::uintptr_t>(smem_raw) + 1023) & ~static_cast<std::uintptr_t>(1023));
   std::uint64_t* full = reinterpret_cast<std::uint64_t*>(smem + S * STAGE);
   std::uint64_t* empty = full + S;
-  std::uint64_t* accum = empty + S;
-  std::uint32_t* tmem_holder = reinterpret_cast<std::uint32_t*>(accum + 1);
+  std::uint64_t* acc_full = empty + S;
+  std::uint64_t* acc_empty = acc_full + 2;
+  std::uint32_t* tmem_holder = reinterpret_cast<std::uint32_t*>(acc_empty + 2);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  // Column tiles run fastest, so the CTAs sharing an A tile are resident
-  // together and all but the first read it from L2.
-  const int tile_n = blockIdx.x * BN, tile_m = blockIdx.y * BM;
-  const int kb0 = blockIdx.z * k_blocks_per_split;
-  const int nkb = max(0, min(k_blocks_total, kb0 + k_blocks_per_split) - kb0);
-
   if (threadIdx.x == 0) {
     for (int s = 0; s < S; ++s) {
       mbar_init(&full[s], 1);
       mbar_init(&empty[s], 1);
     }
-    mbar_init(accum, 1);
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(&acc_full[b], 1);
+      mbar_init(&acc_empty[b], kEpilogueWarps);
+    }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
@@ -165,93 +192,124 @@ __global__ void __launch_bounds__(kThreads, 1)
   int issued = 0;
   if (warp == 0 && lane == 0) {
     // TMA producer
-    for (int i = 0; i < nkb; ++i) {
-      const int s = i % S;
-      if (i >= S && !mbar_wait(&empty[s], ((i / S) - 1) & 1)) break;
-      mbar_arrive_expect_tx(&full[s], STAGE);
-      const int kc = (kb0 + i) * BK;
-      tma_load_2d(smem + s * STAGE, &map_a, kc, tile_m, &full[s]);
-      tma_load_2d(smem + s * STAGE + A_BYTES, &map_b, kc, tile_n, &full[s]);
-      issued = i + 1;
+    for (long long w = blockIdx.x; w < tiles.count; w += gridDim.x) {
+      const WorkTile t = tiles.at(w);
+      const int kb0 = t.split * k_blocks_per_split, kb1 = min(k_blocks_total, kb0 + k_blocks_per_split);
+      bool alive = true;
+      for (int kb = kb0; kb < kb1 && alive; ++kb) {
+        const int s = issued % S;
+        alive = issued < S || mbar_wait(&empty[s], ((issued / S) - 1) & 1);
+        if (!alive) break;
+        mbar_arrive_expect_tx(&full[s], STAGE);
+        tma_load_2d(smem + s * STAGE, &map_a, kb * BK, t.row * BM, &full[s]);
+        tma_load_2d(smem + s * STAGE + A_BYTES, &map_b, kb * BK, t.column * BN, &full[s]);
+        ++issued;
+      }
+      if (!alive) break;
     }
   } else if (warp == 1 && lane == 0) {
     // tcgen05.mma issuer
     constexpr std::uint32_t idesc = instr_desc<BN>();
-    for (int i = 0; i < nkb; ++i) {
-      const int s = i % S;
-      if (!mbar_wait(&full[s], (i / S) & 1)) break;
+    int i = 0, n = 0;
+    for (long long w = blockIdx.x; w < tiles.count; w += gridDim.x, ++n) {
+      const int kb0 = tiles.at(w).split * k_blocks_per_split, kb1 = min(k_blocks_total, kb0 + k_blocks_per_split);
+      const std::uint32_t acc = tmem + (n & 1) * (TMEM_COLS / 2);
+      bool alive = n < 2 || mbar_wait(&acc_empty[n & 1], ((n / 2) - 1) & 1);
       tc_fence_after();
-      const std::uint32_t a_addr = smem_u32(smem + s * STAGE), b_addr = a_addr + A_BYTES;
-      if (ep.shared_terms) {
-        // Products (0,0), (0,1), (1,0) of the block's terms, two K = 16 steps each (byte offsets in a 128-byte row).
+      for (int kb = kb0; kb < kb1 && alive; ++kb, ++i) {
+        const int s = i % S;
+        alive = mbar_wait(&full[s], (i / S) & 1);
+        if (!alive) break;
+        tc_fence_after();
+        const std::uint32_t a_addr = smem_u32(smem + s * STAGE), b_addr = a_addr + A_BYTES;
+        if (ep.shared_terms) {
+          // Products (0,0), (0,1), (1,0) of the block's terms, two K = 16 steps each (byte offsets in a 128-byte row).
 #pragma unroll
-        for (int kk = 0; kk < 6; ++kk)
-          umma_bf16(tmem, smem_desc(a_addr + (kk >= 4 ? 64 : 0) + (kk & 1) * 32),
-                    smem_desc(b_addr + (kk == 2 || kk == 3 ? 64 : 0) + (kk & 1) * 32), idesc, (i | kk) != 0);
-      } else {
+          for (int kk = 0; kk < 6; ++kk)
+            umma_bf16(acc, smem_desc(a_addr + (kk >= 4 ? 64 : 0) + (kk & 1) * 32),
+                      smem_desc(b_addr + (kk == 2 || kk == 3 ? 64 : 0) + (kk & 1) * 32), idesc, kb != kb0 || kk != 0);
+        } else {
 #pragma unroll
-        for (int kk = 0; kk < BK / 16; ++kk)
-          umma_bf16(tmem, smem_desc(a_addr + kk * 32), smem_desc(b_addr + kk * 32), idesc, (i | kk) != 0);
+          for (int kk = 0; kk < BK / 16; ++kk)
+            umma_bf16(acc, smem_desc(a_addr + kk * 32), smem_desc(b_addr + kk * 32), idesc, kb != kb0 || kk != 0);
+        }
+        umma_commit(&empty[s]);
       }
-      umma_commit(&empty[s]);
+      if (!alive) break;
+      umma_commit(&acc_full[n & 1]);
     }
-    umma_commit(accum);
+  } else if (warp >= 2) {
+    // Epilogue: this warp's quarter of the rows, every second 16-column chunk.
+    const int quarter = warp & 3, half = (warp - 2) >> 2;
+    const int n_complex_total = ep.n2 / 2;
+    int n = 0;
+    for (long long w = blockIdx.x; w < tiles.count; w += gridDim.x, ++n) {
+      const WorkTile t = tiles.at(w);
+      const int row = t.row * BM + quarter * 32 + lane, first = t.column * (BN / 2);
+      const bool in_rows = row < ep.m;
+      // A chunk's prior values (accumulating products) are requested one chunk
+      // ahead, the first chunk's before the accumulator is complete.
+      auto load_prior = [&](int c0, Cx<double>(&prior)[8]) {
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+          const int j = first + c0 / 2 + q;
+          const bool other = PAIR && j >= ep.second;
+          const Cx<double>* from = other ? ep.out[1].prior : ep.out[0].prior;
+          const long long at = other ? (j - ep.second) * ep.out[1].ldp : j * ep.out[0].ldp;
+          prior[q] = !ep.partial && from && in_rows && c0 < BN && j < n_complex_total ? from[row + at]
+                                                                                       : Cx<double>{0.0, 0.0};
+        }
+      };
+      Cx<double> prior[8];
+      load_prior(16 * half, prior);
+      if (!__all_sync(0xffffffffu, mbar_wait(&acc_full[n & 1], (n / 2) & 1))) break;
+      tc_fence_after();
+      const std::uint32_t acc = tmem + (n & 1) * (TMEM_COLS / 2) + (static_cast<std::uint32_t>(quarter * 32) << 16);
+      for (int c0 = 16 * half; c0 < BN; c0 += 32) {
+        std::uint32_t r[16];
+        asm volatile(
+            "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+            : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+              "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+            : "r"(acc + static_cast<std::uint32_t>(c0)));
+        Cx<double> next[8];
+        load_prior(c0 + 32, next);
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        if (c0 + 32 >= BN) {  // the accumulator is free once every warp has read its last chunk
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&acc_empty[n & 1]);
+        }
+        if (in_rows) {
+#pragma unroll
+          for (int q = 0; q < 8; ++q) {
+            const int j = first + c0 / 2 + q;
+            if (j >= n_complex_total) break;
+            const float re = __uint_as_float(r[2 * q]), im = __uint_as_float(r[2 * q + 1]);
+            if (ep.partial) {
+              ep.partial[(static_cast<long long>(t.split) * n_complex_total + j) * ep.m + row] = Cx<float>{re, im};
+            } else {
+              const bool other = PAIR && j >= ep.second;
+              Cx<double>* to = other ? ep.out[1].c : ep.out[0].c;
+              const long long at = other ? (j - ep.second) * ep.out[1].ldc : j * ep.out[0].ldc;
+              const double scale = other ? ep.out[1].prior_scale : ep.out[0].prior_scale;
+              const double vr = ep.alpha * static_cast<double>(re), vi = ep.alpha * static_cast<double>(im);
+              to[row + at] = Cx<double>{__dadd_rn(vr, __dmul_rn(scale, prior[q].re)),
+                                        __dadd_rn(vi, __dmul_rn(scale, prior[q].im))};
+            }
+          }
+        }
+#pragma unroll
+        for (int q = 0; q < 8; ++q) prior[q] = next[q];
+      }
+    }
   }
   __syncwarp();
-  // Epilogue: warp w reads TMEM lanes 32w..32w+31 (tile rows).
-  const bool have = __all_sync(0xffffffffu, nkb > 0 && mbar_wait(accum, 0));
-  tc_fence_after();
-  const int row = tile_m + warp * 32 + lane;
-  const int n_complex_total = ep.n2 / 2;
-  for (int c0 = 0; c0 < BN; c0 += 16) {
-    // The chunk's prior values (accumulating products) are requested before
-    // the accumulator read, all eight at once.
-    Cx<double> prior[8];
-#pragma unroll
-    for (int q = 0; q < 8; ++q) {
-      const int j = (tile_n + c0) / 2 + q;
-      const bool other = PAIR && j >= ep.second;
-      const ProductOutput& o = ep.out[other ? 1 : 0];
-      prior[q] = !ep.partial && o.prior && row < ep.m && j < n_complex_total
-                     ? o.prior[row + static_cast<long long>(other ? j - ep.second : j) * o.ldp]
-                     : Cx<double>{0.0, 0.0};
-    }
-    std::uint32_t r[16];
-    if (have) {
-      const std::uint32_t taddr = tmem + (static_cast<std::uint32_t>(warp * 32) << 16) + static_cast<std::uint32_t>(c0);
-      asm volatile(
-          "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-          : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-            "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-          : "r"(taddr));
-      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-    } else {
-#pragma unroll
-      for (int q = 0; q < 16; ++q) r[q] = 0u;
-    }
-    if (row < ep.m) {
-#pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        const int j = (tile_n + c0) / 2 + q;
-        if (j >= n_complex_total) break;
-        const float re = __uint_as_float(r[2 * q]), im = __uint_as_float(r[2 * q + 1]);
-        if (ep.partial) {
-          ep.partial[(static_cast<long long>(blockIdx.z) * n_complex_total + j) * ep.m + row] = Cx<float>{re, im};
-        } else {
-          const bool other = PAIR && j >= ep.second;
-          const ProductOutput& o = ep.out[other ? 1 : 0];
-          const double vr = ep.alpha * static_cast<double>(re), vi = ep.alpha * static_cast<double>(im);
-          o.c[row + static_cast<long long>(other ? j - ep.second : j) * o.ldc] =
-              Cx<double>{__dadd_rn(vr, __dmul_rn(o.prior_scale, prior[q].re)),
-                         __dadd_rn(vi, __dmul_rn(o.prior_scale, prior[q].im))};
-        }
-      }
-    }
-  }
   // Wind-down: drain TMA copies still in flight on the error path, free TMEM.
   if (warp == 0 && lane == 0 && *reinterpret_cast<volatile unsigned int*>(&g_umma_error) != 0u) {
     for (int i = max(0, issued - S); i < issued; ++i) mbar_wait(&full[i % S], (i / S) & 1);
   }
+  __syncwarp();
   tc_fence_before();
   __syncthreads();
   if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS));
@@ -462,9 +520,10 @@ void launch(const std::uint16_t* a, long long lda, const std::uint16_t* b, long 
   allow_dynamic_smem(kernel, smem);
   const CUtensorMap map_a = kmajor_map(a, m, kexp, lda, BM);
   const CUtensorMap map_b = kmajor_map(b, n2, kexp, ldb, BN);
-  if (ceil_div(m, BM) > 65535) throw InvalidArgument("tensor-core GEMM has more than 65535 row tiles");
-  const dim3 grid(static_cast<unsigned>(ceil_div(n2, BN)), static_cast<unsigned>(ceil_div(m, BM)), splits);
-  kernel<<<grid, kThreads, smem, stream>>>(map_a, map_b, k_blocks, kpb, ep_in);
+  TileGrid tiles{static_cast<int>(ceil_div(n2, BN)), static_cast<int>(ceil_div(m, BM)), 0};
+  tiles.count = static_cast<long long>(tiles.columns) * tiles.rows * splits;
+  const unsigned grid = static_cast<unsigned>(std::min<long long>(tiles.count, kSmCount));
+  kernel<<<grid, kThreads, smem, stream>>>(map_a, map_b, k_blocks, kpb, tiles, ep_in);
   SDFT_LAUNCH("umma_gemm_kernel");
 }
 

@@ -179,3 +179,14 @@ def test_mixed_products_at_block_edges(context, k, adjoint):
     ref = (a.conj().T if adjoint else a) @ b
     assert relative_error(complex_gemm(context, a, b, adjoint_a=adjoint, precision="mixed"), ref) < 2e-5
     assert relative_error(complex_gemm(context, a, b, adjoint_a=adjoint, precision="mixed", c=c), ref + c) < 2e-5
+
+
+@pytest.mark.parametrize("m,n,k", [(1, 1, 20), (128, 64, 64), (19001, 65, 40), (9473, 200, 130), (300, 700, 4000)])
+def test_mixed_products_over_many_tiles(context, m, n, k):
+    """One tile, one tile just filled, and more tiles (or K shares) than SMs, so that a CTA's two accumulators are
+    reused; the accumulating form adds every entry once. Tolerance as above."""
+    rng = np.random.default_rng(800 + m)
+    a, b, c = random(rng, (m, k)), random(rng, (k, n)), random(rng, (m, n))
+    ref = a @ b
+    assert relative_error(complex_gemm(context, a, b, precision="mixed"), ref) < 2e-5
+    assert relative_error(complex_gemm(context, a, b, precision="mixed", c=c), ref + c) < 2e-5
