@@ -520,6 +520,7 @@ void launch(const std::uint16_t* a, long long lda, const std::uint16_t* b, long 
   allow_dynamic_smem(kernel, smem);
   const CUtensorMap map_a = kmajor_map(a, m, kexp, lda, BM);
   const CUtensorMap map_b = kmajor_map(b, n2, kexp, ldb, BN);
+  if (ceil_div(m, BM) > 65535) throw InvalidArgument("tensor-core GEMM has more than 65535 row tiles");
   TileGrid tiles{static_cast<int>(ceil_div(n2, BN)), static_cast<int>(ceil_div(m, BM)), 0};
   tiles.count = static_cast<long long>(tiles.columns) * tiles.rows * splits;
   const unsigned grid = static_cast<unsigned>(std::min<long long>(tiles.count, kSmCount));
