@@ -145,6 +145,94 @@ __device__ __forceinline__ void copy_async_commit() { asm volatile("cp.async.com
 // Waits until at most one committed group of this thread is still pending.
 __device__ __forceinline__ void copy_async_wait_all_but_one() { asm volatile("cp.async.wait_group 1;\n" ::: "memory"); }
 
+// FP32 pencil pass for even n0 whose slab rows all differ mod n0/2 (the sphere
+// spans at most half the rows, as on every grid that holds the product of two
+// wave functions): the radix-2 step next to the sphere is then no sum but a
+// selection, and the two half-length spectra are worked off one after the
+// other. Row r's value, times conj(W^r) for the second half, is entry r mod
+// n0/2 of half q, whose backward transform gives the grid points 2m + q; V(r)
+// and the forward transform return its part of row r, the second half's times
+// W^r. A thread holds half a line: between the halves its results change places
+// with the staged rows, so nothing else is kept, and one copy of the transforms
+// serves both. Persistent over units of 128 lines and `groups` columns as the
+// one-thread form above, with V(r) of the line block staged once for the CTA's
+// columns; the threads of a group meet only where the line block changes.
+// Bound by instruction issue and the latency of 16 warps an SM (128 registers;
+// the one-thread form holds a whole line, 8 warps): 231 -> 188 us for 160 columns
+// at 70 points (440 MB of slab traffic, 2.3 TB/s). Small
+// lengths gain less (54 points and 80 columns: level; 48 and 64-point cells
+// 2-6 % of the whole application). Longer even lengths keep the lane-pair form,
+// which a half line would spill in.
+constexpr int kHalfPencilLines = 128;
+constexpr int kHalfPencilGroups = 2;
+constexpr int kHalfPencilBlocks = 2;
+
+template <int N0>
+struct PencilHalfArgs {
+  RegTwiddles<float, N0 / 2> tw;
+  Cx<float> w[N0 / 2];  // exp(-2 pi i r / n0) of the row r with r mod n0/2 = entry
+  int slot[N0 / 2];     // its slab slot, or -1
+};
+
+template <int N0>
+__global__ void __launch_bounds__(kHalfPencilLines* kHalfPencilGroups, kHalfPencilBlocks) pencil_half_kernel(
+    Cx<float>* __restrict__ slab, long long n12, int slots, int columns, long long units,
+    const float* __restrict__ potential, const __grid_constant__ PencilHalfArgs<N0> p) {
+  constexpr int H = N0 / 2, TL = kHalfPencilLines;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int t = threadIdx.x % TL, group = threadIdx.x / TL, groups = blockDim.x / TL;
+  const int sets = (columns + groups - 1) / groups;  // units of a line block
+  Cx<float>* mine = reinterpret_cast<Cx<float>*>(smem_raw) + group * slots * TL + t;  // per group [slots][TL]
+  float* staged_v = reinterpret_cast<float*>(reinterpret_cast<Cx<float>*>(smem_raw) + groups * slots * TL) + t;  // [N0][TL]
+  const long long begin = units * blockIdx.x / gridDim.x, end = units * (blockIdx.x + 1) / gridDim.x;
+  long long block = -1;
+  for (long long u = begin; u < end; ++u) {
+    const long long b = u / sets, kl = b * TL + t;
+    const int c = static_cast<int>(u % sets) * groups + group;
+    const bool live = kl < n12 && c < columns, fresh = b != block;
+    Cx<float>* rows = slab + static_cast<long long>(c) * slots * n12 + kl;
+    if (live)
+      for (int s = 0; s < slots; ++s) copy_async<8>(mine + s * TL, rows + s * n12);
+    if (fresh) {  // V(r) of the new line block, a share of its rows per group
+      block = b;
+      __syncthreads();
+      if (kl < n12)
+        for (int i = group; i < N0; i += groups) copy_async<4>(staged_v + i * TL, potential + i * n12 + kl);
+    }
+    copy_async_commit();
+    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+    if (fresh) __syncthreads();
+    Cx<float> v[H];
+#pragma unroll
+    for (int j = 0; j < H; ++j) v[j] = p.slot[j] >= 0 ? mine[p.slot[j] * TL] : Cx<float>{0.0f, 0.0f};
+#pragma unroll 1
+    for (int q = 0; q < 2; ++q) {
+      fft_line_registers<float, true, H>(v, p.tw.w);
+#pragma unroll
+      for (int m = 0; m < H; ++m) v[m] = cscale(v[m], staged_v[(2 * m + q) * TL]);
+      fft_line_registers<float, false, H>(v, p.tw.w);
+      if (q == 0) {
+#pragma unroll
+        for (int j = 0; j < H; ++j) {
+          Cx<float> x{0.0f, 0.0f};
+          if (p.slot[j] >= 0) {
+            x = mine[p.slot[j] * TL];
+            mine[p.slot[j] * TL] = v[j];
+          }
+          v[j] = cmul(x, Cx<float>{p.w[j].re, -p.w[j].im});
+        }
+      } else if (live) {
+#pragma unroll
+        for (int j = 0; j < H; ++j)
+          if (p.slot[j] >= 0) {
+            const Cx<float> even = mine[p.slot[j] * TL], odd = cmul(v[j], p.w[j]);
+            rows[p.slot[j] * n12] = Cx<float>{even.re + odd.re, even.im + odd.im};
+          }
+      }
+    }
+  }
+}
+
 template <int N0>
 __global__ void __launch_bounds__(kRegisterPencilThreads) pencil_registers_kernel(
     Cx<float>* __restrict__ slab, long long n12, int slots, int columns, long long units,
@@ -646,6 +734,27 @@ bool launch_pencil_registers(const SpherePlan& plan, int columns, const T* poten
                             columns;
     auto go = [&](auto length) {
       constexpr int N0 = decltype(length)::value;
+      if constexpr (N0 % 2 == 0 && N0 <= kRegisterPencilMax) {
+        if (plan.half_rows) {
+          PencilHalfArgs<N0> p;
+          for (int j = 0; j < N0 / 2; ++j) {
+            p.tw.w[j] = plan.twiddles_host[0][2 * j];
+            const int r = plan.slot_of_row_host[j] >= 0 ? j : j + N0 / 2;
+            p.w[j] = plan.twiddles_host[0][r];
+            p.slot[j] = plan.slot_of_row_host[r];
+          }
+          const int groups = std::min(columns, kHalfPencilGroups), threads = groups * kHalfPencilLines;
+          const std::size_t smem = (sizeof(Cx<float>) * groups * plan.slots + sizeof(float) * N0) * kHalfPencilLines;
+          allow_smem(pencil_half_kernel<N0>, smem);
+          const long long half_units = static_cast<long long>(ceil_div(static_cast<std::size_t>(n12), kHalfPencilLines) *
+                                                              ceil_div(static_cast<std::size_t>(columns), groups));
+          const long long grid = std::min<long long>(half_units, resident_ctas(pencil_half_kernel<N0>, threads, smem));
+          pencil_half_kernel<N0><<<static_cast<unsigned>(grid), threads, smem, stream>>>(slab, n12, plan.slots, columns,
+                                                                                         half_units, potential, p);
+          SDFT_LAUNCH("pencil_half_kernel");
+          return true;
+        }
+      }
       if constexpr (N0 > kRegisterPencilMax) {
         const long long pair_units =
             static_cast<long long>(ceil_div(static_cast<std::size_t>(n12), kPairPencilLines)) * columns;
@@ -954,6 +1063,8 @@ void SpherePlan::build(const int shape[3], const std::vector<std::uint64_t>& ind
   slots = static_cast<int>(h_slot_row.size());
   for (int s = 0; s < slots; ++s) slot_of_row[h_slot_row[s]] = s;
   slot_of_row_host = slot_of_row;
+  half_rows = n[0] % 2 == 0;
+  for (int r = 0; half_rows && r < n[0] / 2; ++r) half_rows = slot_of_row[r] < 0 || slot_of_row[r + n[0] / 2] < 0;
   krow_host.assign(rows1.begin(), rows1.end());
   for (int a = 0; a < 3; ++a) {
     twiddles_host[a].resize(n[a]);

@@ -26,6 +26,7 @@ struct SpherePlan {
   int* krow = nullptr;          // [krows]
   LinePlan line[3];
   std::vector<int> slot_of_row_host;       // [n0] slot of grid row i0, or -1
+  bool half_rows = false;                  // n0 is even and the slots' rows differ mod n0/2
   std::vector<int> krow_host;              // [krows] the active i1 rows
   std::vector<Cx<float>> twiddles_host[3]; // [n[a]] FP32 twiddles, passed as kernel parameters
 

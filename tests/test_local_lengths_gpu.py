@@ -106,3 +106,23 @@ def test_local_apply_on_unequal_axes(context, cell):
         assert relative_error(op.local_apply(x, precision="mixed"), expected) < 2e-5
     finally:
         op.close()
+
+
+@pytest.mark.parametrize("n", [40, 42, 54, 70, 72])
+@pytest.mark.parametrize("columns", [1, 2, 5])
+def test_half_line_pencils_at_column_counts(context, n, columns):
+    """Even lengths whose pencils are worked off in two half-length spectra, two columns to a CTA: one column, one
+    pair, and an odd count whose last pair has one. Bar as above (FP32 against FP64, per column)."""
+    import torch
+    ecut, k = CELLS[n]
+    op = PlaneWaveOperator(context, synthetic.tiny(ecut_ha=ecut, kpoint=(k, k, k), roots=4))
+    try:
+        assert op.shape == (n, n, n) and 2 * op.active_rows <= n
+        xd = torch.from_numpy(np.ascontiguousarray(probe_block(op.npw, columns, 300 + n).T)).cuda().T
+        y64 = op.local_apply(xd, precision="fp64")
+        y32 = op.local_apply(xd, precision="mixed")
+        context.synchronize()
+        for c in range(columns):
+            assert relative_error(y32.T[c].cpu().numpy(), y64.T[c].cpu().numpy()) < 2e-5
+    finally:
+        op.close()
