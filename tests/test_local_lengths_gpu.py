@@ -118,7 +118,9 @@ def test_half_line_pencils_at_column_counts(context, n, columns):
     op = PlaneWaveOperator(context, synthetic.tiny(ecut_ha=ecut, kpoint=(k, k, k), roots=4))
     try:
         assert op.shape == (n, n, n) and 2 * op.active_rows <= n
-        xd = torch.from_numpy(np.ascontiguousarray(probe_block(op.npw, columns, 300 + n).T)).cuda().T
+        # strides given outright: torch does not keep them for a single column
+        xd = torch.empty_strided((op.npw, columns), (1, op.npw), dtype=torch.complex128, device="cuda")
+        xd.copy_(torch.from_numpy(probe_block(op.npw, columns, 300 + n)))
         y64 = op.local_apply(xd, precision="fp64")
         y32 = op.local_apply(xd, precision="mixed")
         context.synchronize()
