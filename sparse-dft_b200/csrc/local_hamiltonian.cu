@@ -118,7 +118,7 @@ __global__ void __launch_bounds__(kThreads) pencil_kernel(Cx<T>* __restrict__ sl
   }
 }
 
-// FP32 pencil pass with one thread per (i1, i2) line: the line's n0 values
+// FP32 pencil pass of the odd lengths, one thread per (i1, i2) line: the line's n0 values
 // live in registers through both transforms (fft_line_registers), so no
 // transform stage touches shared memory. The kernel is persistent: CTA k
 // walks a contiguous range of units (block of 128 lines, column), column
@@ -735,27 +735,25 @@ bool launch_pencil_registers(const SpherePlan& plan, int columns, const T* poten
     auto go = [&](auto length) {
       constexpr int N0 = decltype(length)::value;
       if constexpr (N0 % 2 == 0 && N0 <= kRegisterPencilMax) {
-        if (plan.half_rows) {
-          PencilHalfArgs<N0> p;
-          for (int j = 0; j < N0 / 2; ++j) {
-            p.tw.w[j] = plan.twiddles_host[0][2 * j];
-            const int r = plan.slot_of_row_host[j] >= 0 ? j : j + N0 / 2;
-            p.w[j] = plan.twiddles_host[0][r];
-            p.slot[j] = plan.slot_of_row_host[r];
-          }
-          const int groups = std::min(columns, kHalfPencilGroups), threads = groups * kHalfPencilLines;
-          const std::size_t smem = (sizeof(Cx<float>) * groups * plan.slots + sizeof(float) * N0) * kHalfPencilLines;
-          allow_smem(pencil_half_kernel<N0>, smem);
-          const long long half_units = static_cast<long long>(ceil_div(static_cast<std::size_t>(n12), kHalfPencilLines) *
-                                                              ceil_div(static_cast<std::size_t>(columns), groups));
-          const long long grid = std::min<long long>(half_units, resident_ctas(pencil_half_kernel<N0>, threads, smem));
-          pencil_half_kernel<N0><<<static_cast<unsigned>(grid), threads, smem, stream>>>(slab, n12, plan.slots, columns,
-                                                                                         half_units, potential, p);
-          SDFT_LAUNCH("pencil_half_kernel");
-          return true;
+        // Grids of 2 (span of the basis) + 1 or more points always have it.
+        if (!plan.half_rows) return false;
+        PencilHalfArgs<N0> p;
+        for (int j = 0; j < N0 / 2; ++j) {
+          p.tw.w[j] = plan.twiddles_host[0][2 * j];
+          const int r = plan.slot_of_row_host[j] >= 0 ? j : j + N0 / 2;
+          p.w[j] = plan.twiddles_host[0][r];
+          p.slot[j] = plan.slot_of_row_host[r];
         }
-      }
-      if constexpr (N0 > kRegisterPencilMax) {
+        const int groups = std::min(columns, kHalfPencilGroups), threads = groups * kHalfPencilLines;
+        const std::size_t smem = (sizeof(Cx<float>) * groups * plan.slots + sizeof(float) * N0) * kHalfPencilLines;
+        allow_smem(pencil_half_kernel<N0>, smem);
+        const long long half_units = static_cast<long long>(ceil_div(static_cast<std::size_t>(n12), kHalfPencilLines) *
+                                                            ceil_div(static_cast<std::size_t>(columns), groups));
+        const long long grid = std::min<long long>(half_units, resident_ctas(pencil_half_kernel<N0>, threads, smem));
+        pencil_half_kernel<N0><<<static_cast<unsigned>(grid), threads, smem, stream>>>(slab, n12, plan.slots, columns,
+                                                                                       half_units, potential, p);
+        SDFT_LAUNCH("pencil_half_kernel");
+      } else if constexpr (N0 > kRegisterPencilMax) {
         const long long pair_units =
             static_cast<long long>(ceil_div(static_cast<std::size_t>(n12), kPairPencilLines)) * columns;
         PencilPairArgs<N0> p;
