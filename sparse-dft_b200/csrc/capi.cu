@@ -716,7 +716,7 @@ sdft_b200_status sdft_b200_rayleigh_ritz(sdft_b200_context* context, size_t n, s
     sdft_b200::hermitian_from_lower(hin, m, hw, m, m, ctx.stream);
     sdft_b200::hermitian_from_lower(sin, m, sw, m, m, ctx.stream);
     sdft_b200::generalized_lowest(ctx.blas, ctx.solver, hw, sw, m, count, dvalues, hw, ctx.eigen, sdft_b200::rr_mode(),
-                                  ctx.stream);
+                                  ctx.stream, 1e-5, 1e-8, sdft_b200::Reduction::Columns);
     if (memory == SDFT_B200_MEMORY_HOST) {
       SDFT_CUDA(cudaMemcpyAsync(values, dvalues, sizeof(double) * count, cudaMemcpyDeviceToHost, ctx.stream));
       SDFT_CUDA(cudaMemcpyAsync(vectors, hw, sizeof(C) * n * count, cudaMemcpyDeviceToHost, ctx.stream));

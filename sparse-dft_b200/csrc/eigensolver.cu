@@ -12,8 +12,10 @@
 //    and publishes it with the next head row. Exchange buffers are
 //    double-buffered by step parity. The barrier is a counting barrier with a
 //    time limit: on expiry an error word is set and every CTA returns.
-// 2. bisect_kernel: one warp per wanted eigenvalue, 64-point multisection on
-//    division-free Sturm counts of the tridiagonal matrix.
+//    tridiagonalize_columns_kernel: the form of Reduction::Columns.
+// 2. bisect_kernel: one warp per wanted eigenvalue, multisection with 64 points
+//    (128 for Reduction::Columns) on division-free Sturm counts of the
+//    tridiagonal matrix.
 // 3. inverse_iteration_kernel: one thread per wanted eigenvalue, factors in
 //    shared memory; LU with partial pivoting of T - lambda I, two solves from
 //    a start vector of its own; then cluster_orthonormalize_kernel, one CTA
@@ -704,6 +706,288 @@ __global__ void __cluster_dims__(kClusterCtas, 1, 1) __launch_bounds__(kClusterT
   cluster_barrier();
 }
 
+struct ColumnArgs {
+  const Cx<double>* a;
+  int m, grid, cpc;
+  double* d;
+  double* e;
+  Cx<double>* tau;
+  Cx<double>* reflectors;  // m x m, column j holds v_j in rows j+1..m-1
+  Cx<double>* colbuf;      // 2 x m
+  Cx<double>* pbuf;        // 2 x m
+  Cx<double>* dotbuf;      // 2 x grid
+  unsigned int* arrive;
+  unsigned int* error;  // set when a barrier wait runs out; every CTA then returns
+};
+
+// Reflector scalars of one step, formed redundantly by every thread from the
+// same shared inputs (so every thread holds equal values).
+struct ColumnReflector {
+  Cx<double> tau, scale;
+  double beta;
+  bool trivial;
+};
+
+__device__ __forceinline__ ColumnReflector make_column_reflector(Cx<double> alpha, double xnorm2) {
+  ColumnReflector h;
+  if (xnorm2 == 0.0 && alpha.im == 0.0) {
+    h.trivial = true;
+    h.tau = Cx<double>{0.0, 0.0};
+    h.beta = alpha.re;
+    h.scale = Cx<double>{0.0, 0.0};
+  } else {
+    const double beta = -copysign(sqrt(alpha.re * alpha.re + alpha.im * alpha.im + xnorm2), alpha.re);
+    h.trivial = false;
+    h.tau = Cx<double>{(beta - alpha.re) / beta, -alpha.im / beta};
+    h.beta = beta;
+    // 1 / (alpha - beta)
+    const double dr = alpha.re - beta, di = alpha.im, den = dr * dr + di * di;
+    h.scale = Cx<double>{dr / den, -di / den};
+  }
+  return h;
+}
+
+// The reduction of Reduction::Columns, any order up to kRowsPerThread *
+// kTridiagThreads in one cooperative launch: rows r = tid + kTridiagThreads k of
+// the reflector and rank-2 vectors in registers, own columns c = cta + G s in
+// shared memory. Step j+1's reflector is formed from the published column
+// before step j's rank-2 update, so the update of each own column and its
+// product with the next reflector share one pass; a step publishes p = tau A v
+// and the column after next. Per step: one CTA barrier for the next column's
+// norm, one for the column products, and the grid barrier: 7.3 to 9.3 us, the
+// norm, the square root and the divisions behind the grid barrier.
+__global__ void __launch_bounds__(kTridiagThreads, 1) tridiagonalize_columns_kernel(ColumnArgs t) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  constexpr int R = kRowsPerThread;
+  const int m = t.m, G = t.grid, cpc = t.cpc, cta = blockIdx.x, tid = threadIdx.x;
+  const int lane = tid & 31, warp = tid >> 5;
+  Cx<double>* cols = reinterpret_cast<Cx<double>*>(smem_raw);
+  Cx<double>* red = cols + static_cast<long long>(cpc) * m;  // kTridiagWarps x kMaxCpc column-product partials
+  Cx<double>* colv = red + kTridiagWarps * kMaxCpc;                  // 2 x kMaxCpc: v at own columns, by step parity
+  Cx<double>* colw = colv + 2 * kMaxCpc;                      // kMaxCpc: w at own columns
+  Cx<double>* pick = colw + kMaxCpc;                          // alpha (row jc+1), diagonal (row jc)
+  double* nrm = reinterpret_cast<double*>(pick + 2);          // kTridiagWarps norm partials
+  __shared__ int ok;
+
+  int slot_of_row[R];
+#pragma unroll
+  for (int k = 0; k < R; ++k) {
+    const int r = tid + k * kTridiagThreads;
+    slot_of_row[k] = (r < m && r >= cta && (r - cta) % G == 0) ? (r - cta) / G : -1;
+  }
+  for (int s = 0; s < cpc; ++s) {
+    const int c = cta + s * G;
+    if (c < m)
+      for (int r = tid; r < m; r += kTridiagThreads) cols[static_cast<long long>(s) * m + r] = t.a[r + static_cast<long long>(c) * m];
+  }
+
+  Cx<double> v[R], w[R], vn[R], col[R];
+  ColumnReflector cur, next;
+
+  // Reflector of column jc from col[] (rows >= jc): vn[] for rows >= jc+1,
+  // v at own columns into colv[jc & 1], and CTA 0's outputs. Contains the
+  // step's first CTA barrier (after which colw, written before it, is visible).
+  auto reflect = [&](int jc) -> ColumnReflector {
+    double part = 0.0;
+#pragma unroll
+    for (int k = 0; k < R; ++k) {
+      const int r = tid + k * kTridiagThreads;
+      if (r < m && r >= jc + 2) part += col[k].re * col[k].re + col[k].im * col[k].im;
+      if (r == jc + 1) pick[0] = col[k];
+      if (r == jc) pick[1] = col[k];
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
+    if (lane == 0) nrm[warp] = part;
+    __syncthreads();
+    double xnorm2 = 0.0;
+#pragma unroll
+    for (int q = 0; q < kTridiagWarps; ++q) xnorm2 += nrm[q];
+    const ColumnReflector h = make_column_reflector(pick[0], xnorm2);
+    if (cta == 0 && tid == 0) {
+      t.d[jc] = pick[1].re;
+      t.e[jc] = h.beta;
+      t.tau[jc] = h.tau;
+    }
+    Cx<double>* cv = colv + (jc & 1) * kMaxCpc;
+#pragma unroll
+    for (int k = 0; k < R; ++k) {
+      const int r = tid + k * kTridiagThreads;
+      Cx<double> vr{0.0, 0.0};
+      if (r == jc + 1) vr = Cx<double>{1.0, 0.0};
+      else if (r > jc + 1 && r < m && !h.trivial) vr = cmulz(col[k], h.scale);
+      vn[k] = vr;
+      if (cta == 0 && r > jc && r < m) t.reflectors[r + static_cast<long long>(jc) * m] = vr;
+      if (slot_of_row[k] >= 0) cv[slot_of_row[k]] = vr;
+    }
+    return h;
+  };
+
+  // Column products conj(A(:,c)) . vn over the CTA (acc), then p = tau A v at
+  // own columns c > jc, the CTA share of p^H v, and column jc+1 published.
+  auto publish = [&](int jc, const ColumnReflector& h, Cx<double> (&acc)[kMaxCpc]) {
+#pragma unroll
+    for (int q = 0; q < kMaxCpc; ++q) {
+      if (q < cpc) {
+        double re = acc[q].re, im = acc[q].im;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+          re += __shfl_xor_sync(0xffffffffu, re, o);
+          im += __shfl_xor_sync(0xffffffffu, im, o);
+        }
+        if (lane == 0) red[warp * kMaxCpc + q] = Cx<double>{re, im};
+      }
+    }
+    __syncthreads();
+    if (warp == 0) {
+      Cx<double> dot{0.0, 0.0};
+      const int c = cta + lane * G;
+      if (lane < cpc && c > jc && c < m) {
+        Cx<double> s{0.0, 0.0};
+        for (int q = 0; q < kTridiagWarps; ++q) s = cadd(s, red[q * kMaxCpc + lane]);
+        const Cx<double> p = cmulz(h.tau, s);
+        t.pbuf[static_cast<long long>(jc & 1) * m + c] = p;
+        dot = cdot1(p, colv[(jc & 1) * kMaxCpc + lane]);
+      }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        dot.re += __shfl_xor_sync(0xffffffffu, dot.re, o);
+        dot.im += __shfl_xor_sync(0xffffffffu, dot.im, o);
+      }
+      if (lane == 0) t.dotbuf[static_cast<long long>(jc & 1) * G + cta] = dot;
+    }
+    // Column jc+1 (updates 0..jc-1 applied) for step jc+1.
+    if (jc + 1 < m && (jc + 1) % G == cta) {
+      const long long slot = (jc + 1) / G;
+      Cx<double>* dst = t.colbuf + static_cast<long long>((jc + 1) & 1) * m;
+      for (int r = jc + 1 + tid; r < m; r += kTridiagThreads) dst[r] = cols[slot * m + r];
+    }
+  };
+
+  // Step 0: reflector of column 0, p_0 over own columns, column 1 published.
+#pragma unroll
+  for (int k = 0; k < R; ++k) {
+    const int r = tid + k * kTridiagThreads;
+    col[k] = r < m ? t.a[r] : Cx<double>{0.0, 0.0};
+  }
+  __syncthreads();  // own columns in shared memory
+  cur = reflect(0);
+#pragma unroll
+  for (int k = 0; k < R; ++k) v[k] = vn[k];
+  {
+    Cx<double> acc[kMaxCpc];
+#pragma unroll
+    for (int q = 0; q < kMaxCpc; ++q) {
+      acc[q] = Cx<double>{0.0, 0.0};
+      const int c = cta + q * G;
+      if (q >= cpc || c < 1 || c >= m) continue;
+      const Cx<double>* a = cols + static_cast<long long>(q) * m;
+#pragma unroll
+      for (int k = 0; k < R; ++k) {
+        const int r = tid + k * kTridiagThreads;
+        if (r >= 1 && r < m) acc[q] = cadd(acc[q], cdot1(a[r], v[k]));
+      }
+    }
+    publish(0, cur, acc);
+  }
+  __syncthreads();  // the published column comes from every warp
+  if (!grid_barrier(t.arrive, t.error, static_cast<unsigned int>(G), &ok)) return;
+
+  for (int j = 0; j < m - 1; ++j) {
+    const bool last = j == m - 2;
+    // All of this step's global reads first (one round of L2 latency): p on
+    // own rows, column j+1, p at own columns and at row j+1, the CTA shares
+    // of p^H v (every warp sums them in the same order).
+    const double2* pb = reinterpret_cast<const double2*>(t.pbuf + static_cast<long long>(j & 1) * m);
+    const double2* cb = reinterpret_cast<const double2*>(t.colbuf + static_cast<long long>((j + 1) & 1) * m);
+    const double2* db = reinterpret_cast<const double2*>(t.dotbuf + static_cast<long long>(j & 1) * G);
+    const double2 zero2 = make_double2(0.0, 0.0);
+    double2 pq[R], cq[R], shares[kMaxShares];
+#pragma unroll
+    for (int k = 0; k < R; ++k) {
+      const int r = tid + k * kTridiagThreads;
+      const bool row = r > j && r < m;
+      pq[k] = (row && !cur.trivial) ? __ldcg(pb + r) : zero2;
+      cq[k] = (row && !last) ? __ldcg(cb + r) : zero2;
+    }
+    const int own_c = cta + tid * G;
+    const bool own_w = !cur.trivial && tid < cpc && own_c > j && own_c < m;
+    const double2 pc = own_w ? __ldcg(pb + own_c) : zero2;
+    const double2 ph = cur.trivial ? zero2 : __ldcg(pb + j + 1);
+#pragma unroll
+    for (int i = 0; i < kMaxShares; ++i) {
+      const int g = lane + 32 * i;
+      shares[i] = (!cur.trivial && g < G) ? __ldcg(db + g) : zero2;
+    }
+    Cx<double> sum{0.0, 0.0};
+#pragma unroll
+    for (int i = 0; i < kMaxShares; ++i) sum = cadd(sum, Cx<double>{shares[i].x, shares[i].y});
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      sum.re += __shfl_xor_sync(0xffffffffu, sum.re, o);
+      sum.im += __shfl_xor_sync(0xffffffffu, sum.im, o);
+    }
+    const Cx<double> alpha = cmulz(Cx<double>{-0.5 * cur.tau.re, -0.5 * cur.tau.im}, sum);
+    // w = p + alpha v on own rows; w at own columns for the update; w[j+1] (v[j+1] = 1).
+#pragma unroll
+    for (int k = 0; k < R; ++k) {
+      const int r = tid + k * kTridiagThreads;
+      w[k] = (r > j && r < m && !cur.trivial) ? cadd(Cx<double>{pq[k].x, pq[k].y}, cmulz(alpha, v[k]))
+                                               : Cx<double>{0.0, 0.0};
+      col[k] = Cx<double>{cq[k].x, cq[k].y};
+    }
+    const Cx<double> head_w = cur.trivial ? Cx<double>{0.0, 0.0} : cadd(Cx<double>{ph.x, ph.y}, alpha);
+    if (own_w) colw[tid] = cadd(Cx<double>{pc.x, pc.y}, cmulz(alpha, colv[(j & 1) * kMaxCpc + tid]));
+
+    // Step j+1's reflector from column j+1 with update j applied.
+    if (!last) {
+      const Cx<double> hw = cconj(head_w);
+#pragma unroll
+      for (int k = 0; k < R; ++k) {
+        const int r = tid + k * kTridiagThreads;
+        if (r > j && r < m) col[k] = csub(col[k], cadd(cmulz(v[k], hw), w[k]));
+      }
+      next = reflect(j + 1);
+    } else {
+      __syncthreads();  // colw visible
+    }
+
+    // Update j on own columns c > j; p_{j+1} partial sums over rows/columns > j+1.
+    Cx<double> acc[kMaxCpc];
+#pragma unroll
+    for (int q = 0; q < kMaxCpc; ++q) {
+      acc[q] = Cx<double>{0.0, 0.0};
+      const int c = cta + q * G;
+      if (q >= cpc || c <= j || c >= m) continue;
+      const Cx<double> wc = cconj(colw[q]), vc = cconj(colv[(j & 1) * kMaxCpc + q]);
+      Cx<double>* a = cols + static_cast<long long>(q) * m;
+      const bool dot_column = !last && c > j + 1;
+#pragma unroll
+      for (int k = 0; k < R; ++k) {
+        const int r = tid + k * kTridiagThreads;
+        if (r > j && r < m) {
+          Cx<double> x = a[r];
+          if (!cur.trivial) {
+            x = csub(x, cadd(cmulz(v[k], wc), cmulz(w[k], vc)));
+            a[r] = x;
+          }
+          if (dot_column && r > j + 1) acc[q] = cadd(acc[q], cdot1(x, vn[k]));
+        }
+      }
+    }
+    if (last) break;
+    publish(j + 1, next, acc);
+    __syncthreads();
+    if (!grid_barrier(t.arrive, t.error, static_cast<unsigned int>(G) * static_cast<unsigned int>(j + 2), &ok))
+      return;
+    cur = next;
+#pragma unroll
+    for (int k = 0; k < R; ++k) v[k] = vn[k];
+  }
+  __syncthreads();
+  if ((m - 1) % G == cta && tid == 0) t.d[m - 1] = cols[static_cast<long long>((m - 1) / G) * m + m - 1].re;
+}
+
 // Number of eigenvalues of the tridiagonal (d, e) below x: sign changes of
 // the Sturm sequence p_0 = 1, p_1 = d_0 - x, p_i = (d_{i-1} - x) p_{i-1} -
 // e_{i-2}^2 p_{i-2}, kept in range by exact power-of-two rescaling. A p_i
@@ -746,6 +1030,7 @@ __device__ void sturm_counts(const double* d, const double* e2, int m, const dou
 }
 
 // One warp per wanted eigenvalue; 32 x P points per round (P per lane).
+template <int P>
 __global__ void bisect_kernel(const double* __restrict__ d, const double* __restrict__ e, int m, int wanted,
                               double* __restrict__ values) {
   extern __shared__ double sm[];
@@ -783,8 +1068,8 @@ __global__ void bisect_kernel(const double* __restrict__ d, const double* __rest
   const double atol = DBL_EPSILON * tnorm;
   // P points per lane trade rounds (53 bits / log2(32 P + 1)) for the length of
   // a Sturm step's chain: 0.252 ms at order 640 with 320 values and 0.496 at
-  // 1280 with P = 2, 0.332 and 0.654 with P = 4.
-  constexpr int P = 2;
+  // 1280 with P = 2, 0.332 and 0.654 with P = 4 (Reduction::Columns). The
+  // interval that is left, and with it the eigenvalue's last bits, depends on P.
   for (int round = 0; round < 64; ++round) {
     const double width = hi - lo;
     if (width <= 2.0 * DBL_EPSILON * fmax(fabs(lo), fabs(hi)) || width <= atol || width <= pivmin) break;
@@ -1094,6 +1379,11 @@ std::size_t tridiag_smem(int m, int cpc) {
          sizeof(double) * kTridiagWarps * 32;
 }
 
+std::size_t columns_smem(int m, int cpc) {
+  return sizeof(Cx<double>) * (static_cast<std::size_t>(cpc) * m + kTridiagWarps * kMaxCpc + 3 * kMaxCpc + 2) +
+         sizeof(double) * kTridiagWarps;
+}
+
 constexpr std::size_t kSmemLimit = 227 * 1024;
 
 std::size_t invit_smem(int m) { return static_cast<std::size_t>(kInvitThreads) * (5 * sizeof(double) + 1) * m; }
@@ -1120,7 +1410,13 @@ CooperativeLane& cooperative_lane(int device) {
   return lanes[device];
 }
 
-void cooperative_launch(void* kernel, int grid, int threads, TridiagArgs& args, std::size_t smem, cudaStream_t stream) {
+template <typename Args>
+void cooperative_launch(void (*kernel)(Args), int grid, int threads, Args& args, std::size_t smem,
+                        cudaStream_t stream) {
+  allow_dynamic_smem(kernel, smem);
+  int per_sm = 0;
+  SDFT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem));
+  if (per_sm < 1) throw InvalidArgument("tridiagonalization kernel cannot be resident");
   int device = 0;
   SDFT_CUDA(cudaGetDevice(&device));
   CooperativeLane& lane = cooperative_lane(device);
@@ -1133,8 +1429,8 @@ void cooperative_launch(void* kernel, int grid, int threads, TridiagArgs& args, 
     SDFT_CUDA(cudaEventRecord(ready, stream));
     SDFT_CUDA(cudaStreamWaitEvent(lane.stream, ready, 0));
     void* params[] = {&args};
-    SDFT_CUDA(cudaLaunchCooperativeKernel(kernel, dim3(grid), dim3(threads), params, smem, lane.stream));
-    SDFT_LAUNCH("tridiagonalize_kernel");
+    SDFT_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<void*>(kernel), dim3(grid), dim3(threads), params, smem, lane.stream));
+    SDFT_LAUNCH("cooperative tridiagonalization kernel");
     SDFT_CUDA(cudaEventRecord(done, lane.stream));
     SDFT_CUDA(cudaStreamWaitEvent(stream, done, 0));
   } catch (...) {
@@ -1145,6 +1441,7 @@ void cooperative_launch(void* kernel, int grid, int threads, TridiagArgs& args, 
   cudaEventDestroy(ready);  // released once the recorded work completes
   cudaEventDestroy(done);
 }
+
 template <int RT, int CT>
 void launch_cluster(const ClusterArgs& t, cudaStream_t stream) {
   const auto kernel = tridiagonalize_cluster_kernel<RT, CT>;
@@ -1177,7 +1474,7 @@ int hermitian_eigen_max_order() {
 }
 
 void hermitian_lowest(cublasHandle_t blas, Cx<double>* a, int m, int wanted, double* values, Cx<double>* vectors,
-                      EigenWorkspace& ws, cudaStream_t stream) {
+                      EigenWorkspace& ws, cudaStream_t stream, Reduction reduction) {
   if (m < 2 || wanted < 1 || wanted > m) throw InvalidArgument("invalid Hermitian eigenproblem size");
   const int grid = std::min({sm_count(), m, 32 * kMaxShares});
   const int cpc = (m + grid - 1) / grid;
@@ -1186,25 +1483,20 @@ void hermitian_lowest(cublasHandle_t blas, Cx<double>* a, int m, int wanted, dou
 
   // Layout of the tridiagonal workspace.
   const std::size_t mm = static_cast<std::size_t>(m);
-  const std::size_t bytes = sizeof(double) * 2 * mm + sizeof(Cx<double>) * (mm + mm * mm + 4 * mm + grid) + 256;
+  const std::size_t bytes = sizeof(double) * 2 * mm + sizeof(Cx<double>) * (mm + mm * mm + 4 * mm + 2 * grid) + 256;
   auto* base = static_cast<unsigned char*>(ws.tridiagonal.reserve(bytes));
   auto* arrive = reinterpret_cast<unsigned int*>(base);
   auto* d = reinterpret_cast<double*>(base + 256);
   double* e = d + mm;
   auto* tau = reinterpret_cast<Cx<double>*>(e + mm);
   Cx<double>* reflectors = tau + mm;
-  Cx<double>* abuf = reflectors + mm * mm;
-  Cx<double>* hbuf = abuf + 2 * mm;
-  auto* shares = reinterpret_cast<double*>(hbuf + 2 * mm);
+  Cx<double>* exchange[2] = {reflectors + mm * mm, reflectors + mm * mm + 2 * mm};  // 2 x m each
+  Cx<double>* shares = exchange[1] + 2 * mm;                                         // 2 x grid
   unsigned int* error_word = arrive + 1;
   SDFT_CUDA(cudaMemsetAsync(arrive, 0, 2 * sizeof(unsigned int), stream));
   // Entries above each reflector's unit element stay zero for the block products.
   SDFT_CUDA(cudaMemsetAsync(reflectors, 0, sizeof(Cx<double>) * mm * mm, stream));
 
-  allow_dynamic_smem(tridiagonalize_kernel, smem);
-  int per_sm = 0;
-  SDFT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, tridiagonalize_kernel, kTridiagThreads, smem));
-  if (per_sm < 1) throw InvalidArgument("tridiagonalization kernel cannot be resident");
   // SDFT_B200_TRACE: device times of the stages, printed after the final synchronisation.
   static const bool trace = std::getenv("SDFT_B200_TRACE") != nullptr;
   cudaEvent_t marks[6] = {};
@@ -1214,23 +1506,29 @@ void hermitian_lowest(cublasHandle_t blas, Cx<double>* a, int m, int wanted, dou
     if (trace) SDFT_CUDA(cudaEventRecord(marks[i], stream));
   };
   mark(0);
-  const int tail = std::min(m, kClusterOrder), stop = m - tail;  // the cluster kernel's order, the grid kernel's reflectors
-  if (stop > 0) {
-    TridiagArgs t{a, m, grid, cpc, tridiag_rows(m), stop, d, e, tau, reflectors, abuf, hbuf, shares, arrive,
-                  error_word};
-    cooperative_launch(reinterpret_cast<void*>(tridiagonalize_kernel), grid, kTridiagThreads, t, smem, stream);
+  if (reduction == Reduction::Columns) {
+    ColumnArgs t{a, m, grid, cpc, d, e, tau, reflectors, exchange[0], exchange[1], shares, arrive, error_word};
+    cooperative_launch(tridiagonalize_columns_kernel, grid, kTridiagThreads, t, columns_smem(m, cpc), stream);
+  } else {
+    const int tail = std::min(m, kClusterOrder), stop = m - tail;  // the cluster kernel's order, the grid kernel's reflectors
+    if (stop > 0) {
+      TridiagArgs t{a, m, grid, cpc, tridiag_rows(m), stop, d, e, tau, reflectors, exchange[0], exchange[1],
+                    reinterpret_cast<double*>(shares), arrive, error_word};
+      cooperative_launch(tridiagonalize_kernel, grid, kTridiagThreads, t, smem, stream);
+    }
+    const std::size_t corner = static_cast<std::size_t>(stop) * (mm + 1);
+    cluster_tridiagonalize(ClusterArgs{a + corner, m, tail, d + stop, e + stop, tau + stop, reflectors + corner,
+                                       error_word},
+                           stream);
   }
-  const std::size_t corner = static_cast<std::size_t>(stop) * (mm + 1);
-  cluster_tridiagonalize(ClusterArgs{a + corner, m, tail, d + stop, e + stop, tau + stop, reflectors + corner,
-                                     error_word},
-                         stream);
   mark(1);
 
   const int warps_per_block = 4;
   const std::size_t bisect_smem = sizeof(double) * 2 * mm;
-  allow_dynamic_smem(bisect_kernel, bisect_smem);
-  bisect_kernel<<<static_cast<unsigned>(ceil_div(wanted, warps_per_block)), 32 * warps_per_block, bisect_smem,
-                  stream>>>(d, e, m, wanted, values);
+  const auto bisect = reduction == Reduction::Columns ? bisect_kernel<4> : bisect_kernel<2>;
+  allow_dynamic_smem(bisect, bisect_smem);
+  bisect<<<static_cast<unsigned>(ceil_div(wanted, warps_per_block)), 32 * warps_per_block, bisect_smem, stream>>>(
+      d, e, m, wanted, values);
   SDFT_LAUNCH("bisect_kernel");
   mark(2);
 
@@ -1364,7 +1662,7 @@ void check_solver(cusolverStatus_t status, const char* what) {
 
 void generalized_lowest(cublasHandle_t blas, cusolverDnHandle_t solver, Cx<double>* h, Cx<double>* s, int m,
                         int wanted, double* values, Cx<double>* vectors, EigenWorkspace& ws, RitzSolver mode,
-                        cudaStream_t st, double max_deviation, double first_order_limit) {
+                        cudaStream_t st, double max_deviation, double first_order_limit, Reduction reduction) {
   if (m < 1 || wanted < 1 || wanted > m) throw InvalidArgument("invalid Rayleigh-Ritz dimensions");
   const std::size_t mm = static_cast<std::size_t>(m);
   if (mode == RitzSolver::Device && m >= 2 && m <= hermitian_eigen_max_order()) {
@@ -1383,7 +1681,7 @@ void generalized_lowest(cublasHandle_t blas, cusolverDnHandle_t solver, Cx<doubl
         zgemm(blas, Op::N, Op::N, m, m, m, s, m, h, m, f, m, false);
         lowdin_combine(h, f, m, st);
       }
-      hermitian_lowest(blas, h, m, wanted, values, vectors, ws, st);
+      hermitian_lowest(blas, h, m, wanted, values, vectors, ws, st, reduction);
       if (correct) {
         zgemm(blas, Op::N, Op::N, m, wanted, m, s, m, vectors, m, f, m, false, -0.5);
         add_block(f, m, vectors, m, m, wanted, st);
@@ -1398,7 +1696,7 @@ void generalized_lowest(cublasHandle_t blas, cusolverDnHandle_t solver, Cx<doubl
       lowdin_second_order(s, c, m, st);
       zgemm(blas, Op::N, Op::N, m, m, m, c, m, h, m, f, m, false);
       zgemm(blas, Op::N, Op::N, m, m, m, f, m, c, m, h, m, false);
-      hermitian_lowest(blas, h, m, wanted, values, vectors, ws, st);
+      hermitian_lowest(blas, h, m, wanted, values, vectors, ws, st, reduction);
       zgemm(blas, Op::N, Op::N, m, wanted, m, c, m, vectors, m, f, m, false);
       copy_block(f, m, vectors, m, m, wanted, st);
       return;

@@ -3,12 +3,16 @@ src/pw_core.cpp:56-136) against the dense FP64 oracle: eigenvalues, residuals
 ||H y - e S y|| and S-orthonormality, on the paths the Davidson solve takes
 (S = I exactly, S within 1e-6 of I, S far from I), with degenerate spectra and
 at the largest Davidson subspace (160 roots: 1280)."""
+import pathlib
+
 import numpy as np
 import pytest
 
 from oracle import sdft_oracle
 
 pytestmark = pytest.mark.gpu
+
+GOLDEN = pathlib.Path(__file__).resolve().parent / "golden"
 
 
 def random_unitary(n, rng):
@@ -125,3 +129,30 @@ def test_tridiagonalisation_of_decoupled_blocks(context, n):
     h = np.diag(lam).astype(complex)
     h[half:, half:], _ = pencil(n - half, rng, spectrum=np.sort(lam[half:]))
     check(context, h, np.eye(n), 0)
+
+
+def paired_pencil(n):
+    """Hermitian matrix whose eigenvalues come in pairs about 1e-6 apart: a random matrix of order n / 2 times the
+    2 x 2 identity, plus 2^-20 of another. Every entry is an integer over a power of two, so the matrix is the same
+    on any machine."""
+    rng = np.random.Generator(np.random.PCG64(400 + n))
+
+    def hermitian(m):
+        a = rng.integers(-2**9, 2**9, (m, m)) + 1j * rng.integers(-2**9, 2**9, (m, m))
+        return (np.tril(a) + np.tril(a, -1).conj().T - 1j * np.diag(np.diag(a).imag)) / 2.0**8
+
+    return np.kron(hermitian(n // 2), np.eye(2)) + hermitian(n) / 2.0**20
+
+
+@pytest.mark.parametrize("n", [96, 300, 700])
+def test_vectors_of_near_pairs_are_the_recorded_ones(context, n):
+    """The weights |y|^2 of pairs 1e-6 apart turn the reduction's rounding into eps ||T|| / gap (1e-9 to 1e-8 here), so the
+    call is held to the results that it gave before solves got a reduction of their own, as recorded on a B200
+    (148 SMs) at commit 2fc5f5b. With the same tridiagonal matrix and eigenvalues only the back-transformation's
+    rounding is left, sqrt(n) eps per vector (6e-15)."""
+    from sdft_b200.operator import rayleigh_ritz
+    recorded = np.load(GOLDEN / "ritz_pairs.npz")
+    values, vectors = rayleigh_ritz(context, paired_pencil(n), np.eye(n), 12)
+    weights = vectors.real ** 2 + vectors.imag ** 2
+    assert np.array_equal(values, recorded[f"values_{n}"])
+    assert np.linalg.norm(weights - recorded[f"weights_{n}"]) < 1e-13 * np.linalg.norm(recorded[f"weights_{n}"])
