@@ -1,5 +1,6 @@
 // Device eigensolver for the Davidson Rayleigh-Ritz step (lowest `wanted`
-// eigenpairs of an m x m Hermitian matrix, m up to ~1290).
+// eigenpairs of an m x m Hermitian matrix, m up to kRowsPerThread * kTridiagThreads
+// = 1280).
 //
 // 1. Householder reduction (LAPACK zhetd2, lower, H_j = I - tau v v^H with
 //    v[j+1] = 1): tridiagonalize_cluster_kernel for orders up to 256 and for
@@ -1460,17 +1461,18 @@ void cluster_tridiagonalize(const ClusterArgs& t, cudaStream_t stream) {
 }  // namespace
 
 int hermitian_eigen_max_order() {
-  const int g = sm_count();
-  int best = 0;
-  for (int m = 2; m <= 4096; ++m) {
-    const int grid = std::min({g, m, 32 * kMaxShares});
-    const int cpc = (m + grid - 1) / grid;
-    if (cpc > kMaxCpc || tridiag_smem(m, cpc) > kSmemLimit || m > kRowsPerThread * kTridiagThreads ||
-        invit_smem(m) > kSmemLimit)
-      break;
-    best = m;
-  }
-  return best;
+  static const int order = [] {
+    const int g = sm_count();
+    int best = 0;
+    for (int m = 2; m <= kRowsPerThread * kTridiagThreads; ++m) {
+      const int grid = std::min({g, m, 32 * kMaxShares});
+      const int cpc = (m + grid - 1) / grid;
+      if (cpc > kMaxCpc || tridiag_smem(m, cpc) > kSmemLimit || invit_smem(m) > kSmemLimit) break;
+      best = m;
+    }
+    return best;
+  }();
+  return order;
 }
 
 void hermitian_lowest(cublasHandle_t blas, Cx<double>* a, int m, int wanted, double* values, Cx<double>* vectors,
@@ -1479,7 +1481,7 @@ void hermitian_lowest(cublasHandle_t blas, Cx<double>* a, int m, int wanted, dou
   const int grid = std::min({sm_count(), m, 32 * kMaxShares});
   const int cpc = (m + grid - 1) / grid;
   const std::size_t smem = tridiag_smem(m, cpc);
-  if (cpc > kMaxCpc || smem > kSmemLimit) throw InvalidArgument("Hermitian eigenproblem too large for the device solver");
+  if (m > hermitian_eigen_max_order()) throw InvalidArgument("Hermitian eigenproblem too large for the device solver");
 
   // Layout of the tridiagonal workspace.
   const std::size_t mm = static_cast<std::size_t>(m);

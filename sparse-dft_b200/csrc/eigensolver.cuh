@@ -27,7 +27,8 @@ enum class RitzSolver : int { Device = 0, Subset = 1, Full = 2 };
 // SDFT_B200_RR: device (default), subset (cuSOLVER zhegvdx) or full (zhegvd).
 RitzSolver rr_mode();
 
-// Largest matrix order the tridiagonalization kernel holds in shared memory.
+// Largest matrix order the tridiagonalization kernels hold in shared memory and
+// in their threads' row registers (1280 on a B200).
 int hermitian_eigen_max_order();
 
 // How a matrix is reduced to tridiagonal form and its eigenvalues are searched.

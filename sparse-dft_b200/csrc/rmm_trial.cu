@@ -199,7 +199,13 @@ bool RmmTrial::full_rank(const Images& v) {
   auto& ctx = op_.context();
   zgemm(ctx.blas, Op::C, Op::N, k_, k_, n_, v.x, n_, v.s, n_, ss_, k_, false);
   hermitian_part(ss_, k_, hs_, k_, k_, ctx.stream);
-  hermitian_lowest(ctx.blas, hs_, k_, k_, values_, hs_, eigen_, ctx.stream);
+  if (k_ <= hermitian_eigen_max_order()) {
+    hermitian_lowest(ctx.blas, hs_, k_, k_, values_, hs_, eigen_, ctx.stream);
+  } else {  // the pencil of G and the identity, by cuSOLVER
+    SDFT_CUDA(cudaMemsetAsync(ss_, 0, sizeof(Cx<double>) * static_cast<std::size_t>(k_) * k_, ctx.stream));
+    add_identity(ss_, k_, ctx.stream);
+    generalized_lowest(ctx.blas, ctx.solver, hs_, ss_, k_, k_, values_, hs_, eigen_, rr_mode(), ctx.stream);
+  }
   std::vector<double> values(k_);
   SDFT_CUDA(cudaMemcpyAsync(values.data(), values_, sizeof(double) * k_, cudaMemcpyDeviceToHost, ctx.stream));
   ctx.synchronize();

@@ -75,3 +75,27 @@ def test_rmm_trial_with_one_iteration_budget_falls_back(context, warm):
     op = PlaneWaveOperator(context, base)
     got = op.rmm_trial(base.roots, solved["eigenvectors"], 1, 1e-6)
     assert not got["trial_manifold"] and got["iterations"] == 1
+
+
+def test_rmm_trial_beyond_the_device_eigensolver(context):
+    """1290 roots, past the 1280 rows that the tridiagonalisation holds: the rank check of the block goes to
+    cuSOLVER. A rotated block of exact eigenvectors passes it and is accepted in one step; the same block with its
+    last column (a row past 1280) a copy of the first does not, and goes to the Davidson solve."""
+    import scipy.linalg
+    inputs = synthetic.tiny(ecut_ha=19.0, roots=4)
+    h, s = sdft_oracle.Operator(inputs).dense()
+    roots, tolerance = 1290, 1e-6
+    values, exact = scipy.linalg.eigh(h, s, subset_by_index=(0, roots - 1))
+    rng = np.random.Generator(np.random.PCG64(1290))
+    mix = rng.standard_normal((roots, roots)) + 1j * rng.standard_normal((roots, roots))
+    block = exact @ (np.eye(roots) + 0.1 / np.sqrt(roots) * mix)
+    op = PlaneWaveOperator(context, inputs)
+    try:
+        got = op.rmm_trial(roots, np.ascontiguousarray(block.T), 2, tolerance)
+        assert got["trial_manifold"] and got["iterations"] == 1
+        assert np.max(np.abs(got["eigenvalues"] - values)) < 1e-8
+        block[:, -1] = block[:, 0]
+        got = op.rmm_trial(roots, np.ascontiguousarray(block.T), 2, tolerance)
+        assert not got["trial_manifold"]
+    finally:
+        op.close()
