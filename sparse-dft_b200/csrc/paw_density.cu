@@ -19,6 +19,7 @@
 // keys, 64 atoms), both directions: 781 -> 398 us a pair of calls, errors 1.3e-15
 // -> 6.9e-16; FP64 and load issue bound it.
 #include <algorithm>
+#include <array>
 #include <cmath>
 #include <cstring>
 #include <limits>
@@ -487,6 +488,28 @@ V3 combine(const V3 basis[3], double u, double v, double w) {
   return add(add(scaled(basis[0], u), scaled(basis[1], v)), scaled(basis[2], w));
 }
 
+// order: the keys' caller indices in lexicographic order, ties in the caller's.
+// opposite: per key in that order the caller's index of -G (the adjoint samples
+// V(-G)), -1 when absent, the last of repeated keys: -G walks the order
+// backwards as G walks it forwards. pack orders as (h, k, l) do, for every key
+// and its opposite.
+template <typename Pack>
+void sort_keys(const int* hkl, std::vector<int>& order, std::vector<int>& opposite, Pack pack) {
+  using Packed = decltype(pack(0LL, 0LL, 0LL));
+  std::vector<std::pair<Packed, int>> sorted(order.size());
+  for (std::size_t g = 0; g < sorted.size(); ++g)
+    sorted[g] = {pack(hkl[3 * g], hkl[3 * g + 1], hkl[3 * g + 2]), static_cast<int>(g)};
+  std::sort(sorted.begin(), sorted.end());
+  for (std::size_t i = 0, j = sorted.size(); i < sorted.size(); ++i) {
+    order[i] = sorted[i].second;
+    const int* key = hkl + 3 * static_cast<std::size_t>(order[i]);
+    const Packed target = pack(-static_cast<long long>(key[0]), -static_cast<long long>(key[1]),
+                               -static_cast<long long>(key[2]));
+    while (j > 0 && sorted[j - 1].first > target) --j;
+    opposite[i] = j > 0 && sorted[j - 1].first == target ? sorted[j - 1].second : -1;
+  }
+}
+
 }  // namespace
 
 CompensationCharge::CompensationCharge(Context& ctx, const CompensationInput& in) : ctx_(ctx) {
@@ -514,29 +537,27 @@ CompensationCharge::CompensationCharge(Context& ctx, const CompensationInput& in
   const double scale = 2.0 * kPi / signed_volume;
   const V3 b[3] = {scaled(cross(a[1], a[2]), scale), scaled(cross(a[2], a[0]), scale),
                    scaled(cross(a[0], a[1]), scale)};
-  // Keys in lexicographic order (ties in the caller's order); the arrays below
-  // follow it, order_ leads back.
-  auto packed = [](int h, int k, int l) {
-    const auto b = [](int v) { return static_cast<std::uint64_t>(static_cast<std::int64_t>(v) + (1LL << 20)) & 0x1FFFFF; };
-    return (b(h) << 42) | (b(k) << 21) | b(l);
-  };
-  std::vector<std::pair<std::uint64_t, int>> sorted(count_);
-  for (std::size_t g = 0; g < count_; ++g)
-    sorted[g] = {packed(in.keys[3 * g], in.keys[3 * g + 1], in.keys[3 * g + 2]), static_cast<int>(g)};
-  std::sort(sorted.begin(), sorted.end());
+  // The arrays below follow the keys' order, order_ leads back. Components below
+  // 2^20 pack into one word; further ones would wrap there and break the order.
+  long long m[3] = {0, 0, 0};
+  for (std::size_t i = 0; i < 3 * count_; ++i)
+    m[i % 3] = std::max(m[i % 3], std::llabs(static_cast<long long>(in.keys[i])));
   std::vector<int> order(count_), keys(3 * count_), opposite(count_);
+  if (std::max({m[0], m[1], m[2]}) < 1LL << 20)
+    sort_keys(in.keys, order, opposite, [](long long h, long long k, long long l) {
+      const auto biased = [](long long v) { return static_cast<std::uint64_t>(v + (1LL << 20)); };
+      return biased(h) << 42 | biased(k) << 21 | biased(l);
+    });
+  else
+    sort_keys(in.keys, order, opposite,
+              [](long long h, long long k, long long l) { return std::array<long long, 3>{h, k, l}; });
   std::vector<double> q(3 * count_);
   std::vector<int> shell(count_);
   std::unordered_map<double, int> shells;
   std::vector<double> radii;
-  long long m[3] = {0, 0, 0};
   for (std::size_t i = 0; i < count_; ++i) {
-    const std::size_t g = static_cast<std::size_t>(sorted[i].second);
-    order[i] = sorted[i].second;
-    for (int c = 0; c < 3; ++c) {
-      keys[3 * i + c] = in.keys[3 * g + c];
-      m[c] = std::max(m[c], std::llabs(in.keys[3 * g + c]));
-    }
+    const std::size_t g = static_cast<std::size_t>(order[i]);
+    for (int c = 0; c < 3; ++c) keys[3 * i + c] = in.keys[3 * g + c];
     const V3 v = combine(b, static_cast<double>(in.keys[3 * g]), static_cast<double>(in.keys[3 * g + 1]),
                          static_cast<double>(in.keys[3 * g + 2]));
     q[3 * i] = v.x;
@@ -557,13 +578,6 @@ CompensationCharge::CompensationCharge(Context& ctx, const CompensationInput& in
   SDFT_CUDA(cudaMalloc(&form_, sizeof(double) * lms_ * count_));
   SDFT_CUDA(cudaMalloc(&moments_, sizeof(Cx<double>) * lms_ * atoms_));
   SDFT_CUDA(cudaMalloc(&flags_, sizeof(unsigned int)));
-  // The caller's index of -G (the adjoint samples V(-G)), -1 when absent, the
-  // last of repeated keys: -G walks the order backwards as G walks it forwards.
-  for (std::size_t i = 0, j = count_; i < count_; ++i) {
-    const std::uint64_t target = packed(-keys[3 * i], -keys[3 * i + 1], -keys[3 * i + 2]);
-    while (j > 0 && sorted[j - 1].first > target) --j;
-    opposite[i] = j > 0 && sorted[j - 1].first == target ? sorted[j - 1].second : -1;
-  }
   opposite_ = upload(opposite.data(), opposite.size());
   // Phase tables while they stay small: a support's box is far smaller than its key count.
   constexpr long long kTableEntries = 3 * 4096, kTableBytes = 256LL << 20;

@@ -347,3 +347,28 @@ def test_compensation_small_supports_match_oracle(context, atoms, max_l, count, 
         assert np.array_equal(charge.project(potential), projected)
     finally:
         charge.close()
+
+
+@pytest.mark.parametrize("edge", [2**20 - 1, 2**20, 2**21 + 1])
+def test_compensation_keys_past_the_packed_range(context, edge):
+    """Keys at and past 2^20, where a component no longer fits the packed order, keep every other key's opposite,
+    and are matched by value (2^21 + 1 is not 1). Their own terms are left out of the comparison: the oracle's phase
+    carries eps times 2 pi h."""
+    from sdft_b200 import density, synthetic
+    rng = np.random.Generator(np.random.PCG64(edge))
+    aug = synthetic.augmentation(max_l=2)
+    every = np.stack(np.meshgrid(*[np.arange(-2, 3)] * 3, indexing="ij"), axis=-1).reshape(-1, 3)
+    near = every[rng.permutation(len(every))].astype(np.int32)
+    keys = np.concatenate([near[:60], [[edge, 0, 0], [1, -edge, 0], [0, 0, edge], [0, 2, -edge]], near[60:]]).astype(np.int32)
+    potential = rng.standard_normal(len(keys)) + 1j * rng.standard_normal(len(keys))
+    lattice, fractional = np.diag([10.0, 11.0, 12.0]), rng.uniform(0.0, 1.0, size=(3, 3))
+    transform = rng.standard_normal((9, 16)) + 1j * rng.standard_normal((9, 16))
+    charge = density.CompensationCharge(context, lattice, fractional, keys, aug, transform)
+    try:
+        got = charge.project(potential)
+    finally:
+        charge.close()
+    # The far keys have no opposite: the adjoint is that of the near ones.
+    isnear = np.abs(keys).max(axis=1) < 100
+    expected = sdft_oracle.compensation_project(lattice, fractional, keys[isnear], aug, transform, potential[isnear])
+    assert np.max(np.abs(got - expected)) <= 1e-12 * np.max(np.abs(expected))
