@@ -10,9 +10,10 @@
 //            backward FFT along i0 and accumulate f_b/Omega |.|^2 in registers
 //            in band order; the density line is written once.
 //
-// Axis lengths without a split into two transforms of at most 16 points (125),
-// and planes beyond shared memory, take rows (i2 transforms of the active rows
-// through HBM), columns (i1) and pencils kernels on radix stages in shared memory.
+// Axis lengths without a split into two transforms of at most 16 points (125,
+// 147, 162, 175, 189, 200, 216, 243, 245, 250, 252 and all above 256), and planes
+// beyond shared memory, take rows (i2 transforms of the active rows through HBM),
+// columns (i1) and pencils kernels on radix stages in shared memory.
 //
 // The density grid is then transformed forward in place (unnormalised) and
 // the support keys gathered and divided by N (src/density_functionals.cpp:269-284).

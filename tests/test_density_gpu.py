@@ -5,6 +5,7 @@ import numpy as np
 import pytest
 
 from oracle import sdft_oracle
+from sdft_b200 import _capi as C
 
 pytestmark = pytest.mark.gpu
 
@@ -372,3 +373,37 @@ def test_compensation_keys_past_the_packed_range(context, edge):
     isnear = np.abs(keys).max(axis=1) < 100
     expected = sdft_oracle.compensation_project(lattice, fractional, keys[isnear], aug, transform, potential[isnear])
     assert np.max(np.abs(got - expected)) <= 1e-12 * np.max(np.abs(expected))
+
+
+# Grids whose axes split into two short transforms or not (125, 147, 162, 250 and everything above 256 do not):
+# rows, columns and pencils kernels on radix stages; split planes under those pencils; those planes under split
+# pencils, in either order; every tile width (32, 16 and 8 lines).
+UNSPLIT = [(125, 125, 125), (147, 9, 12), (12, 125, 9), (9, 12, 125), (250, 9, 125), (14, 162, 147), (512, 3, 5),
+           (5, 320, 5), (5, 5, 360)]
+
+
+@pytest.mark.parametrize("shape", UNSPLIT, ids=lambda s: "x".join(map(str, s)))
+def test_band_density_on_axes_without_a_split(context, monkeypatch, shape):
+    """Random plane waves and support keys that reach the grid's corners. Both sides sum fewer than 130 rounded terms
+    of 1.1e-16 a transform and square the field: 4e-14 bounds their relative difference. Bands one at a time add up
+    in the same order."""
+    from conftest import relative_error
+    from sdft_b200 import density
+    rng = np.random.Generator(np.random.PCG64(sum(shape)))
+    extent = (np.array(shape) - 1) // 2
+    hkl = np.unique(np.concatenate([rng.integers(-(extent // 2), extent // 2 + 1, size=(300, 3)),
+                                    np.diag(extent // 2), -np.diag(extent // 2)]), axis=0).astype(np.int32)
+    support = np.unique(np.concatenate([rng.integers(-extent, extent + 1, size=(500, 3)), np.diag(extent),
+                                        -np.diag(extent), np.zeros((1, 3), int)]), axis=0).astype(np.int32)
+    hkl = hkl[rng.permutation(len(hkl))]
+    psi = rng.standard_normal((5, len(hkl))) + 1j * rng.standard_normal((5, len(hkl)))
+    occupations = np.array([2.0, 0.0, 0.7, 1.3, 2.0])
+    assert sdft_oracle.density_grid_shape(hkl, support, True) == shape
+    got = density.band_density(context, hkl, psi, occupations, 700.0, support)
+    expected = sdft_oracle.plane_wave_density(hkl, psi, occupations, 700.0, support, fast=True)
+    assert relative_error(got, expected) < 4e-14
+    monkeypatch.setenv("SDFT_B200_DENSITY_SLAB_BYTES", "1")
+    assert np.array_equal(density.band_density(context, hkl, psi, occupations, 700.0, support), got)
+    psi[2, -1] = np.nan
+    with pytest.raises(C.InvalidArgument, match="nonfinite wavefunction"):
+        density.band_density(context, hkl, psi, occupations, 700.0, support)
