@@ -1,21 +1,25 @@
 """The fused local H~psi at every grid length its register-resident kernels
-are compiled for (the one-thread pencil up to 72 points, the pair-split
-pencil above, the pair-split plane passes for even lengths, and the plane
-passes through the slab in global memory where two shared-memory planes do
-not fit), on small cubic cells whose alias-free grid rule
-(src/plane_wave_operator.cpp:445-457) lands on that length; a k-point of
-(k, k, k) makes the span odd where needed.
+are compiled for (FP32: the half-line pencils of even lengths up to 72 points,
+the one-thread pencils of odd ones, the pair-split pencils above, and the
+pair-split plane passes of even lengths) and lengths that take the four-step
+planes and pencils (all of them in FP64), on small cubic cells whose alias-free
+grid rule (src/plane_wave_operator.cpp:445-457) lands on that length; a k-point
+of (k, k, k) makes the span odd where needed. Lengths without a split (125) and
+plane waves outside the grid rule follow on callers' grids.
 
 Bars: the FP32 local apply (mixed form) within 2e-5 relative of the FP64
 one (the mixed bar of tests/native/plane_wave_operator_smoke.cpp), per column
 and for the block; the FP64 apply within 1e-12 of the numpy oracle's local
 term; the mixed full H~x / S~x pair bit-identical to separate applies.
 """
+import ctypes
+
 import numpy as np
 import pytest
 
 from conftest import probe_block, relative_error
 from oracle import sdft_oracle
+from sdft_b200 import _capi as C
 from sdft_b200 import synthetic
 from sdft_b200.operator import PlaneWaveOperator
 
@@ -27,9 +31,8 @@ CELLS = {35: (26.0, 0.0), 40: (33.0, 0.0), 42: (40.5, 0.0), 45: (45.0, 0.5), 48:
          75: (131.0, 0.0), 80: (145.5, 0.0), 81: (161.5, 0.0), 84: (169.5, 0.5), 90: (178.0, 0.0),
          96: (204.5, 0.5), 98: (232.5, 0.0), 100: (242.5, 0.5), 112: (294.0, 0.0), 120: (316.0, 0.0),
          128: (400.0, 0.5)}
-# Lengths checked against the numpy oracle as well: small ones, and ones whose
-# plane passes run through the slab in global memory because two shared-memory
-# planes do not fit (the FP64 form from 98 points on, FP32 from 120).
+# Lengths checked against the numpy oracle as well: small ones, and the four-step
+# transforms of 7 x 14, 8 x 14, 10 x 12 and 8 x 16 points (radices above 10).
 ORACLE_LENGTHS = {35, 40, 45, 49, 98, 112, 120, 128}
 COLUMNS = 6
 
@@ -128,3 +131,51 @@ def test_half_line_pencils_at_column_counts(context, n, columns):
             assert relative_error(y32.T[c].cpu().numpy(), y64.T[c].cpu().numpy()) < 2e-5
     finally:
         op.close()
+
+
+def accelerated_local(context, shape, indices, potential, kinetic, x, precision):
+    """T x + V(r) x through the accelerator's entry, which takes any grid and plane waves. x: (npw, columns)."""
+    n, columns = x.shape
+    xin, out = np.ascontiguousarray(x.T), np.zeros((columns, n), dtype=np.complex128)
+    dims = np.array(shape, dtype=np.int32)
+    C.check(C.library().sdft_b200_local_hamiltonian(
+        context.handle, dims.ctypes.data_as(C.I32), indices.ctypes.data_as(C.U64), n, kinetic.ctypes.data_as(C.D),
+        potential.ctypes.data_as(C.D), ctypes.c_void_p(xin.ctypes.data), columns, ctypes.c_void_p(out.ctypes.data),
+        C.FP64 if precision == "fp64" else C.MIXED, 0))
+    return out.T
+
+
+# Grid and the rows that plane waves take along each axis (None: all).
+GRIDS = {
+    # an axis of 125 points (no split): the two-buffer plane kernels, the radix-stage pencils, planes through the slab
+    "n1=125": ((12, 125, 20), (6, 60, 10)), "n2=125": ((14, 20, 125), (7, 9, 63)), "n0=125": ((125, 10, 12), (62, 5, 6)),
+    "planes=125": ((8, 125, 125), (4, 50, 61)), "planes=125x45": ((10, 125, 45), (5, 60, 20)),
+    # even FP32 lengths whose rows do not differ mod n0 / 2: four-step pencils instead of two half-length spectra
+    "all rows of 40": ((40, 8, 9), (None, 4, 5)), "all rows of 70": ((70, 15, 14), (None, 7, 7)),
+    "36 rows of 70": ((70, 15, 14), (36, 7, 7)), "all rows of 72": ((72, 72, 72), (None, None, None)),
+    # and rows that do, on planes smaller than a block of 128 lines and a little larger
+    "35 rows of 70": ((70, 6, 5), (35, 3, 3)), "21 rows of 42": ((42, 10, 14), (21, 5, 7)),
+}
+
+
+@pytest.mark.parametrize("grid", list(GRIDS))
+def test_local_apply_on_callers_grids(context, grid):
+    """FP64 within 130 rounded terms of 1.1e-16 of numpy's transforms, as above; the mixed form at its bar."""
+    shape, rows = GRIDS[grid]
+    rng = np.random.Generator(np.random.PCG64(sum(shape)))
+    axes = [np.arange(n) if r is None else np.arange(-((r - 1) // 2), r // 2 + 1) % n for n, r in zip(shape, rows)]
+    box = (axes[0][:, None, None] * shape[1] + axes[1][None, :, None]) * shape[2] + axes[2][None, None, :]
+    # one plane wave at least on every row of the first axis
+    indices = np.unique(np.concatenate([rng.permutation(box.ravel())[:2000], box[:, 0, 0]])).astype(np.uint64)
+    indices = np.ascontiguousarray(rng.permutation(indices))
+    assert len(np.unique(indices // np.uint64(shape[1] * shape[2]))) == (rows[0] or shape[0])
+    potential = rng.standard_normal(shape)
+    kinetic = rng.uniform(0.0, 10.0, len(indices))
+    x = probe_block(len(indices), 3, 11)
+    field = np.zeros((3, int(np.prod(shape))), dtype=np.complex128)
+    field[:, indices.astype(np.int64)] = x.T
+    field = np.fft.ifftn(field.reshape(3, *shape), axes=(1, 2, 3)) * potential
+    field = np.fft.fftn(field, axes=(1, 2, 3)).reshape(3, -1)
+    expected = field[:, indices.astype(np.int64)].T + kinetic[:, None] * x
+    assert relative_error(accelerated_local(context, shape, indices, potential, kinetic, x, "fp64"), expected) < 1.5e-14
+    assert relative_error(accelerated_local(context, shape, indices, potential, kinetic, x, "mixed"), expected) < 2e-5
