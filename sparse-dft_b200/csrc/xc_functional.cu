@@ -31,6 +31,7 @@
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
+#include <functional>
 #include <limits>
 #include <map>
 #include <string>
@@ -638,6 +639,18 @@ void write_support(const FunctionalSupport& s, std::int32_t* hkl) {
   }
 }
 
+// The same while the device works; where the output is one of the input arrays,
+// once its (asynchronous) upload is through.
+void write_support(Context& ctx, const FunctionalSupport& s, std::int32_t* hkl) {
+  const std::less<const std::int32_t*> before;
+  for (int f = 0; f < s.fields; ++f)
+    if (before(hkl, s.field[f].hkl + 3 * s.field[f].count) && before(s.field[f].hkl, hkl + 3 * s.count)) {
+      ctx.synchronize();
+      break;
+    }
+  write_support(s, hkl);
+}
+
 void density_functionals(Context& ctx, const FunctionalSupport& s, std::int32_t* support_hkl, Cx<double>* potential,
                          Cx<double>* xc_potential, FunctionalResult& result) {
   SDFT_CUDA(cudaSetDevice(ctx.device));
@@ -680,7 +693,7 @@ void density_functionals(Context& ctx, const FunctionalSupport& s, std::int32_t*
   xc_merge_kernel<<<1, kTileThreads, 0, ctx.stream>>>(key_partials, key_blocks, kKeySums, nullptr, nullptr,
                                                       merged + 2 * kSums + 2);
   SDFT_LAUNCH("xc_merge_kernel keys");
-  write_support(s, support_hkl);  // while the device works
+  write_support(ctx, s, support_hkl);
   std::vector<double> scalars(2 * (kSums + kKeySums) + 4);
   SDFT_CUDA(cudaMemcpyAsync(scalars.data(), merged, sizeof(double) * scalars.size(), cudaMemcpyDeviceToHost,
                             ctx.stream));
@@ -977,6 +990,11 @@ void collinear_functionals(Context& ctx, const FunctionalSupport& s, std::int32_
   const int count = static_cast<int>(s.count);
   const std::size_t n = s.count;
   const long long points = s.points;
+  double electrons[2] = {0.0, 0.0};  // taken before any output is written: the caller's arrays may be both
+  for (int c = 0; c < 2; ++c)
+    for (std::size_t u = 0; u < s.field[c].count; ++u)
+      if (!s.field[c].hkl[3 * u] && !s.field[c].hkl[3 * u + 1] && !s.field[c].hkl[3 * u + 2])
+        electrons[c] = s.volume * s.field[c].values[2 * u];
   const DeviceSupport support = upload_support(ctx, s);
   const KeyData keys = support.keys;
   const Cx<double>* down = support.down;
@@ -1025,7 +1043,7 @@ void collinear_functionals(Context& ctx, const FunctionalSupport& s, std::int32_
   xc_merge_kernel<<<1, kTileThreads, 0, ctx.stream>>>(key_partials, key_blocks, kSpinKeySums, nullptr, nullptr,
                                                       merged + 2 * stride);
   SDFT_LAUNCH("xc_merge_kernel spin keys");
-  write_support(s, support_hkl);  // while the device works
+  write_support(ctx, s, support_hkl);
   std::vector<double> scalars(3 * stride);
   unsigned int bad = 0;
   SDFT_CUDA(cudaMemcpyAsync(scalars.data(), merged, sizeof(double) * scalars.size(), cudaMemcpyDeviceToHost,
@@ -1060,10 +1078,7 @@ void collinear_functionals(Context& ctx, const FunctionalSupport& s, std::int32_
     r.vxc_density = key_total(10 + c);
     r.grid_points = static_cast<std::uint64_t>(points);
     for (int a = 0; a < 3; ++a) r.grid[a] = s.shape[a];
-    r.sampled_electrons = 0.0;
-    for (std::size_t u = 0; u < s.field[c].count; ++u)
-      if (!s.field[c].hkl[3 * u] && !s.field[c].hkl[3 * u + 1] && !s.field[c].hkl[3 * u + 2])
-        r.sampled_electrons = s.volume * s.field[c].values[2 * u];
+    r.sampled_electrons = electrons[c];
   }
 }
 

@@ -16,6 +16,7 @@ import numpy as np
 import pytest
 
 from conftest import relative_error
+from sdft_b200 import _capi as C
 from sdft_b200 import density, synthetic
 from test_oracle_pins import COLLINEAR_POTENTIAL_TOL, check_collinear, collinear_inputs
 
@@ -58,3 +59,54 @@ def test_collinear_host_checks(context):
     bad[0] = np.nan
     with pytest.raises(ValueError, match="nonfinite spin density"):
         density.collinear_functionals(context, c["lattice"], c["up_keys"], bad, c["down_keys"], c["down"])
+
+
+@pytest.mark.parametrize("pinned", [False, True])
+def test_outputs_may_be_the_input_arrays(context, pinned):
+    """Both forms through the C entry with the support, the potentials and the densities in the same (pageable or
+    page-locked) arrays, the keys in random order: the same results, bit for bit, as with arrays of their own."""
+    import ctypes
+
+    import torch
+    rng = np.random.Generator(np.random.PCG64(31))
+    every = np.stack(np.meshgrid(*[np.arange(-9, 10)] * 3, indexing="ij"), axis=-1).reshape(-1, 3)
+    hkl = np.ascontiguousarray(every[rng.permutation(len(every))], dtype=np.int32)
+    decay = np.exp(-0.5 * (hkl.astype(float) ** 2).sum(axis=1))
+    values = [f * decay * np.exp(-2j * np.pi * (hkl @ rng.uniform(size=3))) for f in (0.02, 0.013)]
+    lattice = np.ascontiguousarray(np.diag([9.0, 10.0, 11.0]).reshape(9))
+    lib, n, count = C.library(), len(hkl), ctypes.c_size_t()
+
+    def array(source):
+        t = torch.from_numpy(np.ascontiguousarray(source).copy())
+        return t.pin_memory().numpy() if pinned else t.numpy()
+
+    def fields(a):
+        return a.ctypes.data_as(C.D)
+
+    def collinear(inplace):
+        keys, up, down = array(hkl), array(values[0]), array(values[1])
+        support, pu, pd = (keys, up, down) if inplace else (array(hkl * 0), array(up * 0), array(down * 0))
+        xu, xd = array(up * 0), array(down * 0)
+        result = (C.Functionals * 2)()
+        C.check(lib.sdft_b200_collinear_functionals(
+            context.handle, fields(lattice), n, keys.ctypes.data_as(C.I32), fields(up), n, keys.ctypes.data_as(C.I32),
+            fields(down), 0, None, None, 0, support.ctypes.data_as(C.I32), fields(pu), fields(pd), fields(xu),
+            fields(xd), n, ctypes.byref(count), result))
+        return [support, pu, pd, xu, xd], [r.as_dict() for r in result]
+
+    def unpolarised(inplace):
+        keys, density = array(hkl), array(values[0])
+        support, potential = (keys, density) if inplace else (array(hkl * 0), array(density * 0))
+        xc, result = array(density * 0), C.Functionals()
+        C.check(lib.sdft_b200_density_functionals(
+            context.handle, fields(lattice), n, keys.ctypes.data_as(C.I32), fields(density), 0, None, None, 0,
+            support.ctypes.data_as(C.I32), fields(potential), fields(xc), n, ctypes.byref(count), ctypes.byref(result)))
+        return [support, potential, xc], [result.as_dict()]
+
+    for form in (collinear, unpolarised):
+        (own, own_scalars), (same, same_scalars) = form(False), form(True)
+        assert count.value == n
+        for a, b in zip(own, same):
+            assert np.array_equal(a, b)
+        for a, b in zip(own_scalars, same_scalars):
+            assert all(np.array_equal(a[key], b[key]) for key in a)
