@@ -190,6 +190,12 @@ def run_reference(args):
     world, rank, _ = distributed()
     if rank != 0:
         return
+    from oracle import ref_oracle
+    if not ref_oracle.available():
+        print(json.dumps({"impl": "reference",
+                          "unavailable": "the reference's library (oracle/_ref) is not built: its sources are not here"}),
+              flush=True)
+        return
     threads = os.cpu_count() or 1
     os.environ.setdefault("OMP_NUM_THREADS", str(threads))
     os.environ.setdefault("OPENBLAS_NUM_THREADS", "1")

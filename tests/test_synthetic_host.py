@@ -67,3 +67,16 @@ def test_serving_request_reuses_the_cell_potential():
                                      kpoint=tuple(request[1].kpoint), seed=4242 * 1000 + 3,
                                      sites=(first.positions, first.species), q_scaling="linear")
     assert np.array_equal(fresh.v_values, request[1].v_values) and np.array_equal(fresh.q, request[1].q)
+
+
+def test_bench_reference_arm_without_the_reference(monkeypatch, capsys):
+    """Where the reference's library is not built the arm says so in one line instead of failing."""
+    import argparse
+    import json
+
+    import bench
+    from oracle import ref_oracle
+    monkeypatch.setattr(ref_oracle, "available", lambda: False)
+    bench.run_reference(argparse.Namespace(gpus=1, steps=1, warmup=0))
+    line = json.loads(capsys.readouterr().out)
+    assert line["impl"] == "reference" and line["unavailable"]
