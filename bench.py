@@ -427,7 +427,7 @@ def fused_local_roofline(op, inputs, stream):
     # DRAM bytes (read + write) of plane_in + pencil + plane_out for one
     # 160-column launch, from one ncu capture of `bench.py --case local
     # --columns 160` (profiles/fused_local_h_si64_160cols.md).
-    traffic = 956_765_952 if cols == 160 and (n0, n1, n2) == (70, 70, 70) else None
+    traffic = 953_614_336 if cols == 160 and (n0, n1, n2) == (70, 70, 70) else None
     return {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
             "traffic": traffic, "kernel": "fused local H~psi (plane_in + pencil + plane_out), FP32, 160 columns",
             "ms_per_launch": ms, "algorithmic_bytes": algorithmic,
@@ -512,7 +512,7 @@ def density_side(ctx, inputs, stream, peak):
                   "achieved_gbs": points * 64 / (ms * 1e-3) / 1e9}
     # Hartree + PBE functional, spin-unpolarised and collinear, of the Si64
     # f = 4 Gaussian densities with a frozen core (142^3 grid, prime-71 axes):
-    # wall time of the host call, the host key sort and union included.
+    # wall time of the host call, key union and copies included.
     case = synthetic.functional_case("si64")
     args = (case["lattice"], case["keys"], case["values"], case["core_keys"], case["core_values"])
     spin = synthetic.collinear_case("si64")
@@ -527,7 +527,7 @@ def density_side(ctx, inputs, stream, peak):
     end = time.perf_counter()
     out["functional"] = {"grid": list(result["grid"]), "keys": int(result["hkl"].shape[0]),
                          "ms": (middle - start) * 1e3, "collinear_ms": (end - middle) * 1e3,
-                         "timing": "wall clock of the host call (host key sort and union included)"}
+                         "timing": "wall clock of the host call (key union and copies included)"}
     return out
 
 

@@ -55,10 +55,10 @@ void trim_pool() {
   SDFT_CUDA(cudaMemPoolTrimTo(current_pool(), 0));
 }
 
-// The attribute calls take a lock of the driver that every launch in the process
-// waits for: made with each launch, four solves on four threads queued behind
-// one another (four 8-atom k-points 102 ms; 62 ms with the calls made once per
-// kernel and device). A single thread's launches cost the same either way.
+// The attribute and occupancy calls take a lock of the driver that every launch in
+// the process waits for: with the shared-memory attribute set at each launch, four
+// solves on four threads queued behind one another (four 8-atom k-points 102 ms; 62
+// ms with that call made once per kernel and device). A single thread's launches cost the same either way.
 std::size_t dynamic_smem_limit(const void* kernel) {
   static std::shared_mutex mutex;
   static std::map<std::pair<int, const void*>, std::size_t> limits;

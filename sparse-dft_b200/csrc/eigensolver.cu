@@ -384,7 +384,8 @@ __global__ void __launch_bounds__(kTridiagThreads, 1) tridiagonalize_kernel(Trid
 // step is bound by its serial chain of instructions, not by a pipe or memory.
 // It reduces whole matrices up to kClusterOrder and the trailing kClusterOrder
 // rows of larger ones; a solve below kClusterOrder needs no cooperative
-// launch, so solves on other streams do not queue behind it.
+// launch, so solves on other streams do not queue behind it (its cluster-size
+// attribute is still set with each launch).
 //
 // Reflector j has head row h = j + 1 and v = e_h + scale x, x the part of
 // column j below h. Step j starts with x, and A x and row h of the trailing

@@ -157,8 +157,9 @@ __device__ __forceinline__ void copy_async_wait_all_but_one() { asm volatile("cp
 // serves both. Persistent over units of 128 lines and `groups` columns as the
 // one-thread form above, with V(r) of the line block staged once for the CTA's
 // columns; the threads of a group meet only where the line block changes.
-// Bound by instruction issue and the latency of 16 warps an SM (128 registers;
-// the one-thread form holds a whole line, 8 warps): 231 -> 188 us for 160 columns
+// Bound by instruction issue (63 % of the slots; instruction fetches and the other
+// warps' turns are the largest waits) at 16 warps an SM (128 registers; the
+// one-thread form holds a whole line, 8 warps): 231 -> 188 us for 160 columns
 // at 70 points (440 MB of slab traffic, 2.3 TB/s). Small
 // lengths gain less (54 points and 80 columns: level; 48 and 64-point cells
 // 2-6 % of the whole application). The FP32 error of the local term against FP64

@@ -17,7 +17,9 @@
 // LM), then one thread per two G sums exp(-i G.tau_a) (F(G) . M_a) / Omega over
 // the atoms in order (src/paw_compensation.cpp:508-520). Si64, f = 8 (542 369
 // keys, 64 atoms), both directions: 781 -> 398 us a pair of calls, errors 1.3e-15
-// -> 6.9e-16; FP64 and load issue bound it.
+// -> 6.9e-16. The density sum (187 us) waits for its table
+// reads: 16 of 17 cycles between issues, at 31 % warps, FP64 pipe 32 %; the
+// adjoint (175 us), its keys staged, is nearer the FP64 pipe (41 %, issue 52 %).
 #include <algorithm>
 #include <array>
 #include <cmath>

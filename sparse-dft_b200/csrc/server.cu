@@ -67,7 +67,11 @@ std::size_t solve_footprint(std::size_t npw, const int* hkl, std::size_t project
   const double r = std::min<double>(roots, n);
   const double cx = 16.0;  // complex128
   double bytes = 0;
-  // Operator: V(r) in FP64 and FP32, maps and diagonals, B, both packed B operands (BF16x6).
+  // Packed operands are counted at the BF16x6 layout (SDFT_B200_SPLIT=x6), the wider
+  // of the two: 24 bytes an entry as left operand and 48 as right one, where the
+  // default takes 8 and 16. That slack is more than the tile autotuner's scratch
+  // product, which is not counted.
+  // Operator: V(r) in FP64 and FP32, maps and diagonals, B, both packed B operands.
   bytes += 12.0 * grid + 40.0 * n + cx * p * n + 2.0 * 24.0 * p * n;
   // Davidson: basis and images, Ritz block and residuals, correction blocks,
   // projected pencil, Rayleigh-Ritz and eigensolver matrices, Gram blocks.
@@ -76,7 +80,7 @@ std::size_t solve_footprint(std::size_t npw, const int* hkl, std::size_t project
   // Largest apply (a full basis refresh): FP64 and FP32 grid slabs, PAW
   // projections, packed tensor-core operands and split-K partials.
   bytes += (cx + 8.0) * grid * cap + 3.0 * cx * p * cap + 24.0 * n * cap + 48.0 * n * kmax + 8.0 * cap * kmax * 64.0;
-  // Mixed search: BF16x6 copies of V^H, HV and SV as right factors, V, HV, SV as left factors.
+  // Mixed search: copies of V^H, HV and SV as right factors, V, HV, SV as left factors (64 n cap by default).
   bytes += 192.0 * n * cap;
   bytes = bytes * 1.1 + 64.0 * 1024 * 1024;  // allocator rounding and handles
   if (!std::isfinite(bytes) || bytes > 1e18) throw Overflow("solve footprint overflow");

@@ -14,11 +14,14 @@
 // Measured (one B200) against radix stages in shared memory, FP64: 97 columns on
 // 81^3 (41 rows) planes in 412 -> 226 us, pencils 729 -> 378 us, planes out 691
 // -> 239 us; 128 bands on 72^3 density planes (rows and columns) 534 -> 206 us,
-// pencils 1005 -> 330 us. The pencils move 834 MB there (2.2 TB/s): issue and
-// shared memory bound them, not HBM. In FP32 the register-resident line kernels
-// of local_hamiltonian.cu stay ahead where they exist (70 points, 160 columns:
-// pencils 235 us there, 295 us here; planes 119 and 137 us, 137 and 161 us here);
-// lengths without them take these (100 points, 32 columns: 1185 -> 563 us a pair).
+// pencils 1005 -> 330 us. The latency of 16 warps an SM (12 in the density's
+// pencils) binds all four: of one capture each at 32 columns, issue slots 33-41 %,
+// FP64 pipe 21-34 %, shared memory 16-34 %, DRAM 11-21 %, and an issued
+// instruction waits 1-3 cycles each on barriers, its operands and loads. In FP32
+// the register-resident line kernels of local_hamiltonian.cu stay ahead where they
+// exist (70 points, 160 columns: pencils 188 us there, 295 us here; planes 119 and
+// 137 us, 137 and 161 us here); lengths without them take these (100 points, 32
+// columns: 1185 -> 563 us a pair).
 #include <type_traits>
 
 #include "split_fft.cuh"

@@ -55,9 +55,11 @@ __device__ __forceinline__ void mma(double (&c)[2], double a, double b) {
 
 // C tile of TM rows x 8 NT columns = alpha op(A) B (+ C), op = adjoint or none.
 // Four real products per complex one, in K order, accumulated in registers;
-// stages of KC entries stream through shared memory by cp.async. Bound by the
-// FP64 matrix pipe: a warp issues 4 NT instructions per K step of 4 for NT + 1
-// shared-memory reads. The CTAs of a cluster (blockIdx.z) take consecutive
+// stages of KC entries stream through shared memory by cp.async. A warp issues
+// 4 NT matrix instructions per K step of 4 for NT + 1 shared-memory reads. At the
+// sizes it takes, latency binds it: 160 x 20 x 1000 and 160^3 keep the matrix pipe
+// 27 and 23 % active with 72 and 120 CTAs in flight, waiting on the stages'
+// barriers, the accumulator chain and the first loads. The CTAs of a cluster (blockIdx.z) take consecutive
 // shares of K and add their tiles through distributed shared memory in rank
 // order, so a small product spread over K needs no second kernel (cuBLAS's
 // shared-K products add one, and a small one leaves most SMs idle: 160 x 20 x
