@@ -104,8 +104,8 @@ def spaced(n, rng):
 
 @pytest.mark.parametrize("n", [2, 3, 16, 17, 64, 65, 127, 128, 129, 255, 256, 257, 258, 400])
 def test_tridiagonalisation_orders(context, n):
-    """Orders around the cluster kernel's tiles (128, 256: rows and columns of the tile that are
-    partly or just filled) and its hand-over from the grid kernel (257 and up)."""
+    """The call's reduction at the orders where the solves' one changes kernels
+    (test_reduction_inside_solves)."""
     rng = np.random.Generator(np.random.PCG64(100 + n))
     h, s = pencil(n, rng, spectrum=spaced(n, rng))
     check(context, h, s, 0)
@@ -113,8 +113,7 @@ def test_tridiagonalisation_orders(context, n):
 
 @pytest.mark.parametrize("n", [511, 512, 513, 769, 1025])
 def test_grid_reduction_orders(context, n):
-    """Orders around the grid kernel's 256 rows per thread slot, where a column's padding is one row, none or
-    255 rows, and odd column counts per CTA."""
+    """Orders around the kernels' 256 rows per thread slot, and odd column counts per CTA."""
     rng = np.random.Generator(np.random.PCG64(300 + n))
     h, s = pencil(n, rng, spectrum=spaced(n, rng))
     check(context, h, s, n // 3)
@@ -156,3 +155,49 @@ def test_vectors_of_near_pairs_are_the_recorded_ones(context, n):
     weights = vectors.real ** 2 + vectors.imag ** 2
     assert np.array_equal(values, recorded[f"values_{n}"])
     assert np.linalg.norm(weights - recorded[f"weights_{n}"]) < 1e-13 * np.linalg.norm(recorded[f"weights_{n}"])
+
+
+@pytest.fixture(scope="module")
+def free_electrons(context):
+    """An operator without potential or projectors, H = T and S = 1 exactly, its levels in Ha, and plane waves whose
+    levels are at least 0.01 Ha apart."""
+    import dataclasses
+
+    from sdft_b200 import synthetic
+    from sdft_b200.operator import PlaneWaveOperator
+    x = synthetic.tiny(ecut_ha=30.0, kpoint=(0.1371, 0.2719, 0.4133), roots=4)
+    x = dataclasses.replace(x, v_values=x.v_values * 0.0, d=x.d * 0.0, q=x.q * 0.0, regularization=0.0)
+    levels = x.kinetic_ev / x.hartree_to_ev
+    apart = []
+    for g in np.argsort(levels):
+        if not apart or levels[g] >= levels[apart[-1]] + 0.01:
+            apart.append(g)
+    op = PlaneWaveOperator(context, x)
+    yield op, levels, np.array(apart)
+    op.close()
+
+
+@pytest.mark.parametrize("n,coupled", [(2, 2), (3, 3), (16, 16), (17, 17), (64, 64), (65, 65), (127, 127), (128, 128),
+                                       (129, 129), (255, 255), (256, 256), (257, 257), (258, 258), (400, 400),
+                                       (511, 511), (512, 512), (513, 513), (769, 769), (1025, 1025), (5, 3), (130, 65),
+                                       (300, 150)])
+def test_reduction_inside_solves(free_electrons, n, coupled):
+    """The reduction that solves use, at chosen orders through the RMM trial's first rotation: a block that spans n
+    plane waves, the last `coupled` of them mixed by a random unitary matrix (the others are decoupled: trivial
+    reflectors and exact zeros), has their levels as Ritz values. Orders around the cluster kernel's tiles (128, 256),
+    its hand-over from the grid kernel (257 and up) and the grid kernel's 256 rows per thread slot. Bars as in check():
+    vectors eps ||T|| / gap = 7e-13 apart at 30 and 0.01 Ha."""
+    op, levels, apart = free_electrons
+    rng = np.random.Generator(np.random.PCG64(500 + n + coupled))
+    rows = rng.permutation(apart)[:n]
+    mix = np.eye(n, dtype=complex)
+    mix[n - coupled:, n - coupled:] = random_unitary(coupled, rng)
+    block = np.zeros((n, op.npw), dtype=complex)
+    block[:, rows] = mix.T
+    got = op.rmm_trial(n, block, 2, 2e-9)
+    assert got["trial_manifold"] and got["iterations"] == 1
+    values, vectors = got["eigenvalues"], got["eigenvectors"].T
+    scale = levels[rows].max()
+    assert np.max(np.abs(values - np.sort(levels[rows]))) < 1e-11 * scale
+    assert np.max(np.linalg.norm((levels[:, None] - values) * vectors, axis=0)) < 1e-11 * scale
+    assert np.max(np.abs(vectors.conj().T @ vectors - np.eye(n))) < 1e-11
