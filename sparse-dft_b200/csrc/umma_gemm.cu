@@ -86,6 +86,13 @@ __device__ bool mbar_wait(std::uint64_t* bar, std::uint32_t parity) {
     }
   }
 }
+// Wait of the wind-down after an error, for work already in flight: the same
+// limit, whatever the error word says.
+__device__ void mbar_drain(std::uint64_t* bar, std::uint32_t parity) {
+  const unsigned long long start = globaltimer();
+  while (!mbar_try_wait(bar, parity) && globaltimer() - start <= kWaitLimitNs) {
+  }
+}
 __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, int c0, int c1, std::uint64_t* bar) {
   asm volatile(
       "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
@@ -165,7 +172,8 @@ __global__ void __launch_bounds__(kThreads, 1)
   std::uint64_t* empty = full + S;
   std::uint64_t* acc_full = empty + S;
   std::uint64_t* acc_empty = acc_full + 2;
-  std::uint32_t* tmem_holder = reinterpret_cast<std::uint32_t*>(acc_empty + 2);
+  std::uint64_t* drained = acc_empty + 2;
+  std::uint32_t* tmem_holder = reinterpret_cast<std::uint32_t*>(drained + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
@@ -177,6 +185,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       mbar_init(&acc_full[b], 1);
       mbar_init(&acc_empty[b], kEpilogueWarps);
     }
+    mbar_init(drained, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
@@ -306,9 +315,15 @@ __global__ void __launch_bounds__(kThreads, 1)
     }
   }
   __syncwarp();
-  // Wind-down: drain TMA copies still in flight on the error path, free TMEM.
-  if (warp == 0 && lane == 0 && *reinterpret_cast<volatile unsigned int*>(&g_umma_error) != 0u) {
-    for (int i = max(0, issued - S); i < issued; ++i) mbar_wait(&full[i % S], (i / S) & 1);
+  // Wind-down: on the error path wait for the TMA copies and the products still in
+  // flight (without an error the last epilogue has), then free TMEM.
+  if (lane == 0 && warp < 2 && *reinterpret_cast<volatile unsigned int*>(&g_umma_error) != 0u) {
+    if (warp == 0) {
+      for (int i = max(0, issued - S); i < issued; ++i) mbar_drain(&full[i % S], (i / S) & 1);
+    } else {
+      umma_commit(drained);
+      mbar_drain(drained, 0);
+    }
   }
   __syncwarp();
   tc_fence_before();
