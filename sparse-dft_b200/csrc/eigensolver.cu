@@ -704,8 +704,13 @@ __global__ void __cluster_dims__(kClusterCtas, 1, 1) __launch_bounds__(kClusterT
       }
     }
   }
-  // No CTA leaves while another may still read or write its shared memory.
+  // No CTA leaves while another may still read or write its shared memory. After
+  // an exchange that ran out of time, stores that no CTA waited for may still be on
+  // their way: 20 us lets them land.
   cluster_barrier();
+  if (tid == 0 && *reinterpret_cast<volatile unsigned int*>(t.error) != 0u)
+    for (const unsigned long long start = global_ns(); global_ns() - start < 20000;) {
+    }
 }
 
 struct ColumnArgs {
